@@ -156,6 +156,9 @@ int b2a_sdpa_forward(const b2a_sdpa_desc* desc, const void* q, const void* k, co
     const size_t es = elem_size(r.d.dtype);
     if (!aligned(q, es) || !aligned(k, es) || !aligned(v, es) || !aligned(o, es)) return B2A_ERR_ALIGN;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    // a few query rows (token generation): no 128-row tile to fill, the keys and values are the work
+    if (sdpa_decode16_supported(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, o))
+        return sdpa_decode16_launch(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, masked ? mask : nullptr, o, status, s);
     if (sdpa_tc_supported(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, o) && (!masked || sdpa_tc_mask_supported(r.d, mask)))
         return sdpa_tc_launch(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, o, status, s, nullptr, masked ? mask : nullptr);
     return sdpa_generic_launch(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, mask, o, status, s);
@@ -263,6 +266,12 @@ int b2a_paged_attention(const b2a_paged_desc* desc, const void* query, const voi
         if (beside && cudaEventRecord(join, s) != cudaSuccess) return B2A_ERR_CUDA;
         return paged_decode_launch(d, plan, query, k_cache, v_cache, t, out, workspace, status, s, nullptr,
                                    beside ? join : nullptr);
+    }
+    if (paged_decode16_supported(d)) {
+        // a 16-bit pool: one-token sequences on the decode kernel, the others (if the step has any) on the general one
+        const int rc2 = paged_decode16_launch(d, query, k_cache, v_cache, t, out, status, s);
+        if (rc2 != B2A_OK || d.max_q_len == 1) return rc2;
+        return paged_generic_launch(d, query, k_cache, v_cache, t, out, status, s, 2);
     }
     return paged_generic_launch(d, query, k_cache, v_cache, t, out, status, s);
 }

@@ -37,6 +37,7 @@ struct GenericParams {
     int paged;     // 0 = contiguous, 1 = paged
     int kv_dtype;  // paged only
     int sliding_window;
+    int min_q_len;  // paged: sequences with fewer new tokens are another kernel's
     PagedTables t;
     const uint8_t* k_cache;
     const uint8_t* v_cache;
@@ -81,6 +82,7 @@ __global__ void __launch_bounds__(kThreads) attn_generic_kernel(const GenericPar
         seq = blockIdx.z;
         const int sb = p.t.subsequence_begins[seq], se = p.t.subsequence_begins[seq + 1];
         const int qlen = se - sb;
+        if (qlen >= 0 && qlen < p.min_q_len) return;
         row0 = blockIdx.x * kBM;
         if (row0 >= qlen) return;
         nrows = min(kBM, qlen - row0);
@@ -327,7 +329,7 @@ int sdpa_generic_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const in
 }
 
 int paged_generic_launch(const b2a_paged_desc& d, const void* query, const void* k_cache, const void* v_cache,
-                         const PagedTables& t, void* out, int32_t* status, cudaStream_t stream) {
+                         const PagedTables& t, void* out, int32_t* status, cudaStream_t stream, int min_q_len) {
     if (d.D > kMaxD || d.Dv > kMaxD) return B2A_ERR_UNSUPPORTED;
     GenericParams p{};
     p.Hq = d.Hq; p.Hkv = d.Hkv; p.D = d.D; p.Dv = d.Dv;
@@ -336,6 +338,7 @@ int paged_generic_launch(const b2a_paged_desc& d, const void* query, const void*
     p.paged = 1;
     p.kv_dtype = d.kv_dtype;
     p.sliding_window = d.sliding_window;
+    p.min_q_len = min_q_len;
     p.t = t;
     p.k_cache = static_cast<const uint8_t*>(k_cache);
     p.v_cache = static_cast<const uint8_t*>(v_cache);

@@ -85,4 +85,25 @@ inline cudaError_t launch_overlapped(void (*kernel)(KernelArgs...), dim3 grid, d
     return cudaLaunchKernelEx(&cfg, kernel, KernelArgs(args)...);
 }
 
+// The same with thread-block clusters of `cluster_x` CTAs along the grid's x dimension.
+template <typename... KernelArgs, typename... Args>
+inline cudaError_t launch_overlapped_cluster(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, int cluster_x, size_t smem,
+                                             cudaStream_t stream, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = static_cast<unsigned>(cluster_x);
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, kernel, KernelArgs(args)...);
+}
+
 }  // namespace b2a

@@ -11,8 +11,20 @@ namespace b2a {
 int sdpa_generic_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t (&ks)[4],
                         const int64_t (&vs)[4], const int64_t (&os)[4], const void* q, const void* k, const void* v,
                         const void* mask, void* o, int32_t* status, cudaStream_t stream);
+// min_q_len: sequences with fewer new tokens are left to another kernel
 int paged_generic_launch(const b2a_paged_desc& d, const void* query, const void* k_cache, const void* v_cache,
-                         const PagedTables& t, void* out, int32_t* status, cudaStream_t stream);
+                         const PagedTables& t, void* out, int32_t* status, cudaStream_t stream, int min_q_len = 1);
+
+// attn_decode16.cu — at most sixteen query rows per KV head over 16-bit keys and values (D = Dv = 64 or 128): a few query
+// rows on dense tensors, any mask; the one-token sequences of a paged step on a pool of the queries' own type
+bool sdpa_decode16_supported(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t (&ks)[4], const int64_t (&vs)[4],
+                             const int64_t (&os)[4], const void* q, const void* k, const void* v, const void* o);
+int sdpa_decode16_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t (&ks)[4], const int64_t (&vs)[4],
+                         const int64_t (&os)[4], const void* q, const void* k, const void* v, const void* mask, void* o,
+                         int32_t* status, cudaStream_t stream);
+bool paged_decode16_supported(const b2a_paged_desc& d);
+int paged_decode16_launch(const b2a_paged_desc& d, const void* query, const void* k_cache, const void* v_cache,
+                          const PagedTables& t, void* out, int32_t* status, cudaStream_t stream);
 
 // paged_kv_store.cu
 struct RopeTables {  // rotary embedding of the key rows: f32 tables [positions][rotary_dim / 2] in device memory

@@ -161,6 +161,10 @@ int b2a_sdpa_forward(const b2a_sdpa_desc* desc, const void* q, const void* k, co
         return sdpa_decode16_launch(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, masked ? mask : nullptr, o, status, s);
     if (sdpa_tc_supported(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, o) && (!masked || sdpa_tc_mask_supported(r.d, mask)))
         return sdpa_tc_launch(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, o, status, s, nullptr, masked ? mask : nullptr);
+    // head size 64, and masks that cannot be read in 16-byte pieces.  From the smallest problems on: a launch of one item
+    // takes about as long as one 32-key step of the general kernel
+    if (sdpa_tc_split_supported(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, o))
+        return sdpa_tc_launch(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, o, status, s, nullptr, masked ? mask : nullptr, true);
     return sdpa_generic_launch(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, mask, o, status, s);
 }
 

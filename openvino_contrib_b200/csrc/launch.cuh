@@ -122,7 +122,11 @@ struct TcPeerOut {
 bool sdpa_tc_mask_supported(const b2a_sdpa_desc& d, const void* mask);
 int sdpa_tc_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t (&ks)[4], const int64_t (&vs)[4],
                    const int64_t (&os)[4], const void* q, const void* k, const void* v, void* o, int32_t* status,
-                   cudaStream_t stream, const TcPeerOut* peers = nullptr, const void* mask = nullptr);
+                   cudaStream_t stream, const TcPeerOut* peers = nullptr, const void* mask = nullptr, bool split_p = false);
+// split_p: the form whose probabilities keep float32-like precision; head size 64 or 128 (128: with a mask), any mask
+bool sdpa_tc_split_supported(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t (&ks)[4],
+                             const int64_t (&vs)[4], const int64_t (&os)[4], const void* q, const void* k, const void* v,
+                             const void* o);
 int sdpa_peer_wait_launch(const int32_t* local_flags, int world, int32_t step, long long wait_ns, int32_t* status,
                           cudaStream_t stream);
 

@@ -1,5 +1,6 @@
 // Fused attention for prefill on the 5th-generation tensor core: S = Q K^T and O = P V as tcgen05.mma with
-// accumulators in tensor memory, online softmax in registers.  f16 / bf16, D = Dv = 128, grouped-query heads.
+// accumulators in tensor memory, online softmax in registers.  f16 / bf16, grouped-query heads, D = Dv = 128 (dense
+// tensors also 64).
 // Three front ends share one kernel body (template parameter kMode):
 //   0 dense  (ScaledDotProductAttention): Q, K, V are [B, H, S, 128] tensors, causal or unmasked; K/V tiles are
 //     staged by TMA;
@@ -60,12 +61,11 @@ constexpr int kBM = 128;             // query rows per tile = TMEM lanes
 constexpr int kBN = 128;             // keys per step
 constexpr int kHeadDim = 128;
 constexpr int kPanel = 128 * 128;    // bytes of one [128 rows x 64 elements] swizzled panel
-constexpr int kTile = 2 * kPanel;    // a [128 x 128] 16-bit tile
 constexpr int kThreadsDense = 384;   // 3 warpgroups: softmax A, softmax B, {producer, MMA issuer, 2 idle warps}
 constexpr int kThreadsPaged = 512;   // plus the de-quantising producer warpgroup
 constexpr int kNumBars = 23;
 constexpr int kStageOut = 8 * 4096;  // epilogue staging: one [32 rows x 64 elements] slab per softmax warp
-constexpr int kSmemBytes = 6 * kTile + kStageOut + 1024 /* alignment slack */ + 256 /* barriers, TMEM slot, abort flag */;
+constexpr int smem_bytes(int tile) { return 6 * tile + kStageOut + 1024 /* alignment slack */ + 256 /* barriers, TMEM slot, abort flag */; }
 constexpr float kLazyThreshold = 8.0f;  // log2 units
 constexpr int kCacheChunk = 16 * (kHeadDim + 4);  // bytes of one (block, KV head) chunk of the u8 pool
 
@@ -76,10 +76,11 @@ struct TcParams {
     int causal;
     int window;  // paged modes: a query at position p sees keys p - window + 1 .. p (0: all of them)
     float scale_log2;
-    // dense mode with an attention mask (kMask 1: u8, non-zero keeps; 2: additive, the tensors' 16-bit type):
-    // logical [B, Hq, Sq, Skv] with element strides mask_strides[0..2] (0 on broadcast dimensions), innermost 1
+    // dense mode with an attention mask (u8, non-zero keeps; or additive, the tensors' 16-bit type): logical
+    // [B, Hq, Sq, Skv] with element strides mask_strides (0 on broadcast dimensions)
     const uint8_t* mask;
-    int64_t mask_strides[3];
+    int mask_kind;
+    int64_t mask_strides[4];
     int32_t* status;
     // paged mode
     const uint8_t* k_cache;
@@ -266,6 +267,27 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
         return *reinterpret_cast<const uint32_t*>(&v);
     }
 }
+template <bool kBf16>
+__device__ __forceinline__ void unpack2(uint32_t w, float& lo, float& hi) {
+    if constexpr (kBf16) {
+        lo = __uint_as_float(w << 16);
+        hi = __uint_as_float(w & 0xffff0000u);
+    } else {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
+        lo = f.x;
+        hi = f.y;
+    }
+}
+// One value of an additive mask, in log2 units.  Finite values end at kMaskFloor (the lowest bf16 times log2(e) would
+// overflow): a row whose keys all carry the type's lowest value stays uniform over them, as in attn_generic_kernel.
+constexpr float kMaskFloor = -1.0e30f;
+template <bool kBf16>
+__device__ __forceinline__ float mask_log2(const uint8_t* row, int64_t at) {
+    const uint16_t bits = reinterpret_cast<const uint16_t*>(row)[at];
+    const float f = kBf16 ? __uint_as_float(static_cast<uint32_t>(bits) << 16) : __half2float(__ushort_as_half(bits));
+    const float v = f * kLog2e;
+    return v < kMaskFloor && f != -INFINITY ? kMaskFloor : v;
+}
 // time-bounded wait that ignores the abort flag: used only to drain work already in flight
 __device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
     const long long t0 = clock64();
@@ -356,11 +378,23 @@ __global__ void __launch_bounds__(128) paged_gather_kernel(const PagedTables t, 
 
 // kMode: 0 dense tensors; 1 paged, K/V de-quantised by producer warps inside the kernel; 2 paged, K/V de-quantised
 // beforehand into per-sequence row ranges of an f16 scratch (paged_gather_kernel) and staged by TMA like dense ones
-template <bool kBf16, int kMode, int kMask = 0>
+// kMask: 0 no mask; 1 boolean and 2 additive, every row read by its thread in 16-byte pieces (unit stride, aligned);
+//   3 boolean and 4 additive, the same for all rows (row stride 0: a padding mask), read once per warp, any key stride
+//   and alignment; 5 either kind with any strides, element by element.
+// kDim: head size, 64 or 128.
+// kSplitP: P enters the second product as the sum of two 16-bit values - hi = round(p), lo = round(p - hi), kept in the two
+//   halves of S's columns - so that these calls lose nothing against the float32 probabilities of attn_generic_kernel.  It
+//   costs half as many second products again (the tensor pipe idles behind the exponentials anyway) and about five
+//   instructions per pair of probabilities.  Bound: the special-function unit, 128 exponentials per row and step; the
+//   f16 encoder batch of 8 x 16 heads x 512 tokens, head size 64, boolean padding mask: 1167 us in attn_generic_kernel,
+//   28.7 us here (5.1 us of memory traffic at the copy rate).
+template <bool kBf16, int kMode, int kMask = 0, int kDim = kHeadDim, bool kSplitP = false>
 __global__ void __launch_bounds__(kMode == 1 ? kThreadsPaged : kThreadsDense, 1)
 attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, const TcParams p,
                const __grid_constant__ TcPeers peers) {
+    static_assert(kDim == kHeadDim || kMode == 0, "the paged modes are built for a head size of 128");
+    constexpr int kTile = 128 * kDim * 2;  // bytes of a [128 x kDim] 16-bit tile: kDim / 64 panels
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;  // 128-byte swizzle atoms want 1024-byte aligned tiles
@@ -685,7 +719,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                     mbar_expect_tx(BAR(Q_FULL + X), kTile);
                     const int row = tok_base + (X ? it.row0B : it.row0A), head = X ? it.headB : it.headA;
                     tma_load_4d_hint(sQ + X * kTile, &tmQ, BAR(Q_FULL + X), 0, row, head, it.b, once_policy);
-                    tma_load_4d_hint(sQ + X * kTile + kPanel, &tmQ, BAR(Q_FULL + X), 64, row, head, it.b, once_policy);
+                    if constexpr (kDim > 64)
+                        tma_load_4d_hint(sQ + X * kTile + kPanel, &tmQ, BAR(Q_FULL + X), 64, row, head, it.b, once_policy);
                     ++qn[X];
                 };
                 load_q(0);
@@ -698,12 +733,14 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                         if (n > 0 && !mbar_wait(BAR(K_EMPTY + st), (n - 1) & 1, abort_flag)) { ok = false; break; }
                         mbar_expect_tx(BAR(K_FULL + st), kTile);
                         tma_load_4d(sK + st * kTile, &tmK, BAR(K_FULL + st), 0, kv_row0 + j * kBN, it.hk, it.b);
-                        tma_load_4d(sK + st * kTile + kPanel, &tmK, BAR(K_FULL + st), 64, kv_row0 + j * kBN, it.hk, it.b);
+                        if constexpr (kDim > 64)
+                            tma_load_4d(sK + st * kTile + kPanel, &tmK, BAR(K_FULL + st), 64, kv_row0 + j * kBN, it.hk, it.b);
                         ++issued_k;
                         if (n > 0 && !mbar_wait(BAR(V_EMPTY + st), (n - 1) & 1, abort_flag)) { ok = false; break; }
                         mbar_expect_tx(BAR(V_FULL + st), kTile);
                         tma_load_4d(sV + st * kTile, &tmV, BAR(V_FULL + st), 0, kv_row0 + j * kBN, it.hk, it.b);
-                        tma_load_4d(sV + st * kTile + kPanel, &tmV, BAR(V_FULL + st), 64, kv_row0 + j * kBN, it.hk, it.b);
+                        if constexpr (kDim > 64)
+                            tma_load_4d(sV + st * kTile + kPanel, &tmV, BAR(V_FULL + st), 64, kv_row0 + j * kBN, it.hk, it.b);
                         ++issued_v;
                     }
                 }
@@ -721,18 +758,19 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             // operand formats (A and B of one MMA must agree): dense mode as given; paged mode f16 throughout - the
             // de-quantised values keep 11 significant bits and bf16 queries are converted in shared memory first
             constexpr uint32_t idesc_qk = instr_desc_f16(kKvBf16, false, kBM, kBN);
-            constexpr uint32_t idesc_pv = instr_desc_f16(kKvBf16, true, kBM, kHeadDim);
+            constexpr uint32_t idesc_pv = instr_desc_f16(kKvBf16, true, kBM, kDim);
             // descriptors are assembled at the point of issue from (tile address >> 4) plus compile-time parts
             constexpr uint32_t kLoK = desc_lo_sw128(16), kHiK = desc_hi_sw128(1024);        // K-major: Q and K tiles
             constexpr uint32_t kLoV = desc_lo_sw128(kPanel), kHiV = desc_hi_sw128(1024);    // MN-major: V tiles
             const uint32_t q16 = (sQ >> 4) & 0x3FFFu, k16 = (sK >> 4) & 0x3FFFu, v16 = (sV >> 4) & 0x3FFFu;
-            auto issue_qk = [&](int X, int st) {  // S_X = Q_X K^T : 8 steps of 16 along D
+            auto issue_qk = [&](int X, int st) {  // S_X = Q_X K^T : steps of 16 along D
                 const uint32_t d = tmem + static_cast<uint32_t>(X * 128);
                 const uint32_t qa = q16 + static_cast<uint32_t>(X * (kTile >> 4)), ka = k16 + static_cast<uint32_t>(st * (kTile >> 4));
 #define B2A_QK(ks) \
     mma_ss_c<((((ks) / 4) * kPanel + ((ks) & 3) * 32) / 16), ((((ks) / 4) * kPanel + ((ks) & 3) * 32) / 16), kLoK, kLoK, kHiK, kHiK, \
              idesc_qk>(d, qa, ka, (ks) > 0 ? 1u : 0u)
-                B2A_QK(0); B2A_QK(1); B2A_QK(2); B2A_QK(3); B2A_QK(4); B2A_QK(5); B2A_QK(6); B2A_QK(7);
+                B2A_QK(0); B2A_QK(1); B2A_QK(2); B2A_QK(3);
+                if constexpr (kDim > 64) { B2A_QK(4); B2A_QK(5); B2A_QK(6); B2A_QK(7); }
 #undef B2A_QK
             };
             // O_X += P_X V : 8 steps of 16 along the keys, issued in two halves as the halves of P arrive
@@ -743,6 +781,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 #define B2A_PV(ks, accv) mma_ts_c<(ks) * 8, ((ks) * 2048) / 16, kLoV, kHiV, idesc_pv>(d, pa, va, accv)
                 B2A_PV(0, acc ? 1u : 0u); B2A_PV(1, 1u); B2A_PV(2, 1u); B2A_PV(3, 1u);
 #undef B2A_PV
+                if constexpr (kSplitP) {  // the low halves of the same probabilities, 64 columns on
+#define B2A_PVLO(ks) mma_ts_c<64 + (ks) * 8, ((ks) * 2048) / 16, kLoV, kHiV, idesc_pv>(d, pa, va, 1u)
+                    B2A_PVLO(0); B2A_PVLO(1); B2A_PVLO(2); B2A_PVLO(3);
+#undef B2A_PVLO
+                }
             };
             bool ok = true;
             constexpr int kQReady = (kPaged && kBf16) ? Q_CONV : Q_FULL;
@@ -841,9 +884,44 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             const int tile0 = kPaged ? item.kv_tile0 : 0;
             const int window = kPaged ? p.window : 0;
             const int low_limit = window > 0 ? row_pos0 + kBM - window : -(1 << 30);  // mask while key0 < low_limit
-            const float c = kMask == 2 ? 1.0f : p.scale_log2;  // (additive masks: the block below has scaled the scores)
+            // (additive masks: the blocks below have scaled the scores)
+            const float c = kMask == 2 || kMask == 4 || (kMask == 5 && p.mask_kind == B2A_MASK_ADD) ? 1.0f : p.scale_log2;
             float m_used = -1.0e30f, l = 0.f;
+            // rows past the end of the tensor read the last row's mask: their results are dropped
+            const uint8_t* mrow = nullptr;
+            if constexpr (kMask != 0)
+                mrow = p.mask + (item.b * p.mask_strides[0] + (X ? item.headB : item.headA) * p.mask_strides[1] +
+                                 min(row_pos0 + r, nrows_total - 1) * p.mask_strides[2]) *
+                                    (kMask == 1 || kMask == 3 || (kMask == 5 && p.mask_kind == B2A_MASK_BOOL) ? 1 : 2);
+            // kMask 4: this warp's 128 mask values of a step, as floats, at the start of its staging slab
+            float* mslab = reinterpret_cast<float*>(gbase + 6 * kTile + warp * 4096);
+            if constexpr (kMask == 4) {
+                if (lane == 0) tma_store_wait_read();  // the previous item's store has read the slab
+                __syncwarp();
+            }
             for (int j = 0; j < nkv; ++j) {
+                uint32_t mword[4];  // kMask 3: bit i of word q keeps key 32 q + i of the step
+                if constexpr (kMask == 3) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int key = j * kBN + 32 * q + lane;
+                        mword[q] = key < kv_limit ? mrow[key * p.mask_strides[3]] : 0u;
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) mword[q] = __ballot_sync(0xffffffffu, mword[q] != 0u);
+                }
+                if constexpr (kMask == 4) {
+                    float mv[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int key = j * kBN + 32 * q + lane;
+                        mv[q] = key < kv_limit ? mask_log2<kBf16>(mrow, key * p.mask_strides[3]) : -INFINITY;
+                    }
+                    __syncwarp();  // the last step's values have been read
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) mslab[32 * q + lane] = mv[q];
+                    __syncwarp();
+                }
                 // every lane takes the same decision, so the warp-collective TMEM instructions stay converged
                 ok = __all_sync(0xffffffffu, mbar_wait(BAR(S_FULL + X), (sxb + j) & 1, abort_flag));
                 if (!ok) break;
@@ -853,13 +931,47 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 for (int q = 0; q < 4; ++q) tmem_ld32(tS + 32 * q, s[q]);
                 tmem_wait_ld();
                 const int key0 = (tile0 + j) * kBN;
-                if constexpr (kMask != 0) {
-                    // this row's 128 mask values of the step, 32 keys at a time (rows past the end of the tensor read
-                    // the last row: their results are dropped; keys past the end are removed below)
-                    const int mrow = min(row_pos0 + r, nrows_total - 1);
-                    const uint8_t* mbase = p.mask + (static_cast<int64_t>(item.b) * p.mask_strides[0] +
-                                                     static_cast<int64_t>(X ? item.headB : item.headA) * p.mask_strides[1] +
-                                                     static_cast<int64_t>(mrow) * p.mask_strides[2] + key0) * (kMask == 1 ? 1 : 2);
+                if constexpr (kMask == 3) {
+                    if ((mword[0] & mword[1] & mword[2] & mword[3]) != 0xffffffffu) {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+#pragma unroll
+                            for (int i = 0; i < 32; ++i)
+                                if (((mword[q] >> i) & 1u) == 0u) s[q][i] = 0xff800000u;  // -inf
+                    }
+                }
+                if constexpr (kMask == 4) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+#pragma unroll
+                        for (int i = 0; i < 32; i += 4) {
+                            const float4 m4 = *reinterpret_cast<const float4*>(mslab + 32 * q + i);
+                            s[q][i] = __float_as_uint(fmaf(__uint_as_float(s[q][i]), p.scale_log2, m4.x));
+                            s[q][i + 1] = __float_as_uint(fmaf(__uint_as_float(s[q][i + 1]), p.scale_log2, m4.y));
+                            s[q][i + 2] = __float_as_uint(fmaf(__uint_as_float(s[q][i + 2]), p.scale_log2, m4.z));
+                            s[q][i + 3] = __float_as_uint(fmaf(__uint_as_float(s[q][i + 3]), p.scale_log2, m4.w));
+                        }
+                }
+                if constexpr (kMask == 5) {
+                    const bool keeps = p.mask_kind == B2A_MASK_BOOL;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) {
+                            const int key = key0 + 32 * q + i;
+                            if (key < kv_limit) {
+                                if (keeps) {
+                                    if (mrow[key * p.mask_strides[3]] == 0) s[q][i] = 0xff800000u;
+                                } else {
+                                    s[q][i] = __float_as_uint(fmaf(__uint_as_float(s[q][i]), p.scale_log2,
+                                                                   mask_log2<kBf16>(mrow, key * p.mask_strides[3])));
+                                }
+                            }
+                        }
+                }
+                if constexpr (kMask == 1 || kMask == 2) {
+                    // this row's 128 mask values of the step, 32 keys at a time (keys past the end are removed below)
+                    const uint8_t* mbase = mrow + key0 * (kMask == 1 ? 1 : 2);
                     const bool whole = key0 + kBN <= kv_limit;  // else only whole 16-byte pieces inside the row are read
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
@@ -882,14 +994,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 #pragma unroll
                                 for (int i = 0; i < 4; ++i) {
                                     float lo, hi;
-                                    if constexpr (kBf16) {
-                                        lo = __uint_as_float(w[i] << 16);
-                                        hi = __uint_as_float(w[i] & 0xffff0000u);
-                                    } else {
-                                        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
-                                        lo = f.x;
-                                        hi = f.y;
-                                    }
+                                    unpack2<kBf16>(w[i], lo, hi);
                                     const int e = 8 * h + 2 * i;
                                     s[q][e] = __float_as_uint(fmaf(__uint_as_float(s[q][e]), c, lo * kLog2e));
                                     s[q][e + 1] = __float_as_uint(fmaf(__uint_as_float(s[q][e + 1]), c, hi * kLog2e));
@@ -898,7 +1003,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                         }
                     }
                 }
-                if (j >= jb || (kPaged && key0 < low_limit)) {
+                if (kMask != 3 && kMask != 4 && (j >= jb || (kPaged && key0 < low_limit))) {
                     const int row_pos = row_pos0 + r;  // last key position this row may see (causal)
                     const int row_low = window > 0 ? row_pos - window + 1 : 0;  // and the first
 #pragma unroll
@@ -935,7 +1040,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    uint32_t pk[16];
+                    uint32_t pk[16], pk_lo[16];
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
                         const uint64_t x2 = f2_fma(f2_pack(__uint_as_float(s[q][2 * i]), __uint_as_float(s[q][2 * i + 1])), c2, nm2);
@@ -944,8 +1049,14 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                         const float p0 = ex2f(x0), p1 = ex2f(x1);
                         sum2[i & 3] = f2_add(sum2[i & 3], f2_pack(p0, p1));
                         pk[i] = pack2<kKvBf16>(p0, p1);
+                        if constexpr (kSplitP) {
+                            float h0, h1;
+                            unpack2<kKvBf16>(pk[i], h0, h1);
+                            pk_lo[i] = pack2<kKvBf16>(p0 - h0, p1 - h1);
+                        }
                     }
                     tmem_st16(tS + 16 * q, pk);  // P over the first 64 columns of S, behind what was already read
+                    if constexpr (kSplitP) tmem_st16(tS + 64 + 16 * q, pk_lo);  // (all of S is in registers by now)
                     // first 64 keys of P are in TMEM: PV can start on them, unless O still has to be rescaled
                     if (q == 1 && !(need_any && j > 0)) {
                         tmem_wait_st();
@@ -964,7 +1075,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                     if (!ok) break;
                     tc_fence_after();
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
+                    for (int q = 0; q < kDim / 32; ++q) {
                         uint32_t o[32];
                         tmem_ld32(tO + 32 * q, o);
                         tmem_wait_ld();
@@ -1016,11 +1127,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                         }
                     }
                 } else {
-                    // two passes of 64 columns through this warp's [32 rows x 128 bytes] staging slab
+                    // passes of 64 columns through this warp's [32 rows x 128 bytes] staging slab
                     const uint32_t slab = sOut + static_cast<uint32_t>(warp) * 4096u;
                     uint8_t* prow = gbase + 6 * kTile + warp * 4096 + (r & 31) * 128;
 #pragma unroll
-                    for (int half = 0; half < 2; ++half) {
+                    for (int half = 0; half < kDim / 64; ++half) {
                         if (lane == 0) tma_store_wait_read();  // the slab's previous store has read it
                         __syncwarp();
 #pragma unroll
@@ -1128,12 +1239,13 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// [B, H, S, 128] view with element strides st[0..3] (st[3] == 1) as a 4-D map, box = [64 x box_rows x 1 x 1],
+// [B, H, S, head_dim] view with element strides st[0..3] (st[3] == 1) as a 4-D map, box = [64 x box_rows x 1 x 1],
 // 128-byte swizzle
-bool make_map(CUtensorMap* map, const void* ptr, bool bf16, int B, int H, int S, const int64_t (&st)[4], int box_rows) {
+bool make_map(CUtensorMap* map, const void* ptr, bool bf16, int B, int H, int S, const int64_t (&st)[4], int box_rows,
+              int head_dim = kHeadDim) {
     EncodeTiledFn enc = encode_fn();
     if (enc == nullptr) return false;
-    const cuuint64_t dims[4] = {static_cast<cuuint64_t>(kHeadDim), static_cast<cuuint64_t>(S),
+    const cuuint64_t dims[4] = {static_cast<cuuint64_t>(head_dim), static_cast<cuuint64_t>(S),
                                 static_cast<cuuint64_t>(H), static_cast<cuuint64_t>(B)};
     // a stride of an extent-1 dimension is never used for addressing but is still validated: give it a legal value
     auto bytes = [](int64_t elems, int extent) { return static_cast<cuuint64_t>(extent == 1 || elems <= 0 ? 256 : elems * 2); };
@@ -1146,6 +1258,18 @@ bool make_map(CUtensorMap* map, const void* ptr, bool bf16, int B, int H, int S,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+template <int kMask, int kDim, bool kSplitP>
+int launch_dense(bool bf16, dim3 grid, cudaStream_t stream, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
+                 const CUtensorMap& mo, const TcParams& p, const TcPeers& peers) {
+    constexpr int smem = smem_bytes(128 * kDim * 2);
+    static bool configured[2][64] = {};
+    auto kern = bf16 ? attn_tc_kernel<true, 0, kMask, kDim, kSplitP> : attn_tc_kernel<false, 0, kMask, kDim, kSplitP>;
+    const int rc = configure_once(kern, configured[bf16], smem);
+    if (rc != B2A_OK) return rc;
+    kern<<<grid, kThreadsDense, smem, stream>>>(mq, mk, mv, mo, p, peers);
+    return cudaGetLastError() == cudaSuccess ? B2A_OK : B2A_ERR_CUDA;
+}
+
 bool strides_ok(const int64_t (&st)[4], int B, int H, int S) {
     if (st[3] != 1) return false;
     const int ext[3] = {B, H, S};
@@ -1155,11 +1279,11 @@ bool strides_ok(const int64_t (&st)[4], int B, int H, int S) {
 }
 
 template <typename Kern>
-int configure_once(Kern kern, bool (&done)[64]) {
+int configure_once(Kern kern, bool (&done)[64], int smem) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return B2A_ERR_CUDA;
     if (dev < 0 || dev >= 64 || !done[dev]) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess)
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
             return B2A_ERR_CUDA;
         if (dev >= 0 && dev < 64) done[dev] = true;
     }
@@ -1168,10 +1292,9 @@ int configure_once(Kern kern, bool (&done)[64]) {
 
 }  // namespace
 
-bool sdpa_tc_supported(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t (&ks)[4], const int64_t (&vs)[4],
-                       const int64_t (&os)[4], const void* q, const void* k, const void* v, const void* o) {
+static bool tc_tensors_ok(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t (&ks)[4], const int64_t (&vs)[4],
+                          const int64_t (&os)[4], const void* q, const void* k, const void* v, const void* o) {
     if (d.dtype != B2A_F16 && d.dtype != B2A_BF16) return false;
-    if (d.D != kHeadDim || d.Dv != kHeadDim) return false;
     if (static_cast<long long>(d.B) * d.Hkv > 65535) return false;
     auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     if (!al(q) || !al(k) || !al(v) || !al(o)) return false;
@@ -1179,6 +1302,16 @@ bool sdpa_tc_supported(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int
         !strides_ok(os, d.B, d.Hq, d.Sq))
         return false;
     return encode_fn() != nullptr;
+}
+
+bool sdpa_tc_supported(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t (&ks)[4], const int64_t (&vs)[4],
+                       const int64_t (&os)[4], const void* q, const void* k, const void* v, const void* o) {
+    return d.D == kHeadDim && d.Dv == kHeadDim && tc_tensors_ok(d, qs, ks, vs, os, q, k, v, o);
+}
+
+bool sdpa_tc_split_supported(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t (&ks)[4], const int64_t (&vs)[4],
+                             const int64_t (&os)[4], const void* q, const void* k, const void* v, const void* o) {
+    return (d.D == 64 || d.D == kHeadDim) && d.D == d.Dv && tc_tensors_ok(d, qs, ks, vs, os, q, k, v, o);
 }
 
 bool sdpa_tc_mask_supported(const b2a_sdpa_desc& d, const void* mask) {
@@ -1196,15 +1329,15 @@ bool sdpa_tc_mask_supported(const b2a_sdpa_desc& d, const void* mask) {
 
 int sdpa_tc_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t (&ks)[4], const int64_t (&vs)[4],
                    const int64_t (&os)[4], const void* q, const void* k, const void* v, void* o, int32_t* status,
-                   cudaStream_t stream, const TcPeerOut* peer_out, const void* mask) {
+                   cudaStream_t stream, const TcPeerOut* peer_out, const void* mask, bool split_p) {
     const bool bf16 = d.dtype == B2A_BF16;
     CUtensorMap mq, mk, mv, mo;
-    if (!make_map(&mq, q, bf16, d.B, d.Hq, d.Sq, qs, 128) || !make_map(&mk, k, bf16, d.B, d.Hkv, d.Skv, ks, 128) ||
-        !make_map(&mv, v, bf16, d.B, d.Hkv, d.Skv, vs, 128))
+    if (!make_map(&mq, q, bf16, d.B, d.Hq, d.Sq, qs, 128, d.D) || !make_map(&mk, k, bf16, d.B, d.Hkv, d.Skv, ks, 128, d.D) ||
+        !make_map(&mv, v, bf16, d.B, d.Hkv, d.Skv, vs, 128, d.D))
         return B2A_ERR_CUDA;
     TcPeers peers{};
     if (peer_out == nullptr) {
-        if (!make_map(&mo, o, bf16, d.B, d.Hq, d.Sq, os, 32)) return B2A_ERR_CUDA;
+        if (!make_map(&mo, o, bf16, d.B, d.Hq, d.Sq, os, 32, d.D)) return B2A_ERR_CUDA;
     } else {
         mo = mq;  // not read
         const int64_t fs[4] = {static_cast<int64_t>(peer_out->hq_total) * d.Sq * kHeadDim,
@@ -1236,16 +1369,28 @@ int sdpa_tc_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t
     const int mask_kind = (mask != nullptr && !d.causal) ? d.mask_kind : B2A_MASK_NONE;
     if (mask_kind != B2A_MASK_NONE) {
         p.mask = static_cast<const uint8_t*>(mask);
-        for (int i = 0; i < 3; ++i) p.mask_strides[i] = d.mask_strides[i];
+        p.mask_kind = mask_kind;
+        for (int i = 0; i < 4; ++i) p.mask_strides[i] = d.mask_strides[i];
     }
-    static bool configured[3][2][64] = {};
-    auto kern = mask_kind == B2A_MASK_BOOL  ? (bf16 ? attn_tc_kernel<true, 0, 1> : attn_tc_kernel<false, 0, 1>)
-                : mask_kind == B2A_MASK_ADD ? (bf16 ? attn_tc_kernel<true, 0, 2> : attn_tc_kernel<false, 0, 2>)
-                                            : (bf16 ? attn_tc_kernel<true, 0, 0> : attn_tc_kernel<false, 0, 0>);
-    const int rc = configure_once(kern, configured[mask_kind][bf16]);
-    if (rc != B2A_OK) return rc;
-    kern<<<grid, kThreadsDense, kSmemBytes, stream>>>(mq, mk, mv, mo, p, peers);
-    return cudaGetLastError() == cudaSuccess ? B2A_OK : B2A_ERR_CUDA;
+    if (split_p) {
+        // a mask that is one row for all queries is read once per warp; anything else row by row
+        const int form = mask_kind == B2A_MASK_NONE                    ? 0
+                         : d.mask_strides[2] != 0 && d.Sq > 1          ? 5
+                         : mask_kind == B2A_MASK_BOOL                  ? 3
+                                                                       : 4;
+        if (d.D == 64) {
+            if (form == 0) return launch_dense<0, 64, true>(bf16, grid, stream, mq, mk, mv, mo, p, peers);
+            if (form == 3) return launch_dense<3, 64, true>(bf16, grid, stream, mq, mk, mv, mo, p, peers);
+            if (form == 4) return launch_dense<4, 64, true>(bf16, grid, stream, mq, mk, mv, mo, p, peers);
+            return launch_dense<5, 64, true>(bf16, grid, stream, mq, mk, mv, mo, p, peers);
+        }
+        if (form == 3) return launch_dense<3, kHeadDim, true>(bf16, grid, stream, mq, mk, mv, mo, p, peers);
+        if (form == 4) return launch_dense<4, kHeadDim, true>(bf16, grid, stream, mq, mk, mv, mo, p, peers);
+        if (form == 5) return launch_dense<5, kHeadDim, true>(bf16, grid, stream, mq, mk, mv, mo, p, peers);
+    }
+    if (mask_kind == B2A_MASK_BOOL) return launch_dense<1, kHeadDim, false>(bf16, grid, stream, mq, mk, mv, mo, p, peers);
+    if (mask_kind == B2A_MASK_ADD) return launch_dense<2, kHeadDim, false>(bf16, grid, stream, mq, mk, mv, mo, p, peers);
+    return launch_dense<0, kHeadDim, false>(bf16, grid, stream, mq, mk, mv, mo, p, peers);
 }
 
 int sdpa_peer_wait_launch(const int32_t* local_flags, int world, int32_t step, long long wait_ns, int32_t* status,
@@ -1359,19 +1504,20 @@ int paged_tc_launch(const b2a_paged_desc& d, const void* query, const void* k_ca
     p.kv_base = kv_base;
     dim3 grid(capacity, d.Hkv, 1);
     TcPeers peers{};
+    constexpr int kSmemPaged = smem_bytes(128 * kHeadDim * 2);
     if (gathered) {
         grid = dim3(static_cast<unsigned>(attention_ctas));
         static bool configured[2][64] = {};
         auto kern = bf16 ? attn_tc_kernel<true, 2> : attn_tc_kernel<false, 2>;
-        const int rc = configure_once(kern, configured[bf16]);
+        const int rc = configure_once(kern, configured[bf16], kSmemPaged);
         if (rc != B2A_OK) return rc;
-        kern<<<grid, kThreadsDense, kSmemBytes, stream>>>(mq, mk, mv, mq, p, peers);
+        kern<<<grid, kThreadsDense, kSmemPaged, stream>>>(mq, mk, mv, mq, p, peers);
     } else {
         static bool configured[2][64] = {};
         auto kern = bf16 ? attn_tc_kernel<true, 1> : attn_tc_kernel<false, 1>;
-        const int rc = configure_once(kern, configured[bf16]);
+        const int rc = configure_once(kern, configured[bf16], kSmemPaged);
         if (rc != B2A_OK) return rc;
-        kern<<<grid, kThreadsPaged, kSmemBytes, stream>>>(mq, mq, mq, mq, p, peers);  // only the Q map is read
+        kern<<<grid, kThreadsPaged, kSmemPaged, stream>>>(mq, mq, mq, mq, p, peers);  // only the Q map is read
     }
     return cudaGetLastError() == cudaSuccess ? B2A_OK : B2A_ERR_CUDA;
 }

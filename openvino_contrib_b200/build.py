@@ -24,7 +24,7 @@ NVCC_FLAGS = [
     "--expt-relaxed-constexpr",
 ]
 
-CU_SOURCES = ["csrc/api.cu", "csrc/attn_generic.cu", "csrc/attn_decode16.cu", "csrc/paged_kv_store.cu", "csrc/paged_decode.cu",
+CU_SOURCES = ["csrc/api.cu", "csrc/attn_generic.cu", "csrc/attn_decode16.cu", "csrc/attn_f32.cu", "csrc/paged_kv_store.cu", "csrc/paged_decode.cu",
               "csrc/sdpa_tcgen05.cu", "csrc/shard_group.cu", "csrc/paged_kv_state.cu", "csrc/paged_scores.cu"]
 # host side in the library: the block manager, the operator classes (registered with the operation registry when the
 # library is loaded) and the host-tensor pipeline built on them

@@ -165,6 +165,8 @@ int b2a_sdpa_forward(const b2a_sdpa_desc* desc, const void* q, const void* k, co
     // takes about as long as one 32-key step of the general kernel
     if (sdpa_tc_split_supported(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, o))
         return sdpa_tc_launch(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, o, status, s, nullptr, masked ? mask : nullptr, true);
+    if (sdpa_f32_supported(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, o))
+        return sdpa_f32_launch(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, masked ? mask : nullptr, o, s);
     return sdpa_generic_launch(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, mask, o, status, s);
 }
 

@@ -1,6 +1,6 @@
 // General attention kernel: any head size up to 256, any mask, any stride, f32 / f16 / bf16, contiguous or paged
-// K/V.  It is the path for the shapes the specialised kernels (tcgen05 prefill, split-K decode) do not take:
-// f32 tensors, explicit masks, odd head sizes, multi-token rows over a paged cache.
+// K/V.  It is the path for the shapes the specialised kernels (tcgen05 prefill, few-row and split-K decode, float32) do
+// not take: odd head sizes and alignments, float32 queries and multi-token rows over a 16-bit paged cache.
 //
 // One CTA of 256 threads owns 32 query rows of one query head and walks the keys 32 at a time with an online
 // (running max / running sum) softmax, all arithmetic in float32:

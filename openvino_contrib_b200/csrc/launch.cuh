@@ -15,6 +15,13 @@ int sdpa_generic_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const in
 int paged_generic_launch(const b2a_paged_desc& d, const void* query, const void* k_cache, const void* v_cache,
                          const PagedTables& t, void* out, int32_t* status, cudaStream_t stream, int min_q_len = 1);
 
+// attn_f32.cu — float32 tensors, D = Dv up to 128 in whole 16-byte pieces, 16-byte aligned rows, any mask
+bool sdpa_f32_supported(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t (&ks)[4], const int64_t (&vs)[4],
+                        const int64_t (&os)[4], const void* q, const void* k, const void* v, const void* o);
+int sdpa_f32_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t (&ks)[4], const int64_t (&vs)[4],
+                    const int64_t (&os)[4], const void* q, const void* k, const void* v, const void* mask, void* o,
+                    cudaStream_t stream);
+
 // attn_decode16.cu — at most sixteen query rows per KV head over 16-bit keys and values (D = Dv = 64 or 128): a few query
 // rows on dense tensors, any mask; the one-token sequences of a paged step on a pool of the queries' own type
 bool sdpa_decode16_supported(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t (&ks)[4], const int64_t (&vs)[4],

@@ -22,6 +22,7 @@ namespace b2a {
 namespace {
 
 constexpr int kWarpsPerCta = 8;
+constexpr int kFewPasses = 148 * 32;  // warps that the GPU holds at once, at the kernel's registers
 
 struct StoreParams {
     const void* key;
@@ -171,11 +172,16 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) paged_kv_store_kernel(const
     }
 }
 
-// The common geometry (u8 cache, D = Dv = 128, 16-bit rows) with one warp per TOKEN: the walk through the step tables
-// is paid once for the token's 2*Hkv rows, and a row is handled by EIGHT lanes (16 values each: two 16-byte loads,
-// one 16-byte store of codes), so one pass of the warp quantises four rows - the per-row work (min/max reduction,
-// now three shuffle steps, the two scalar divisions, addressing) is issued once for four rows.  Same arithmetic as
-// above, operation for operation, except that x / s for the row's values uses one reciprocal (see below).
+// The common geometry (u8 cache, D = Dv = 128, 16-bit rows): a row is handled by EIGHT lanes (16 values each: two
+// 16-byte loads, one 16-byte store of codes), so one pass of a warp quantises four rows - the per-row work (min/max
+// reduction, now three shuffle steps, the two scalar divisions, addressing) is issued once for four rows.  Same
+// arithmetic as above, operation for operation, except that x / s for the row's values uses one reciprocal (see below).
+// A large step gives a warp all 2*Hkv rows of a token, so that the walk through the step's tables is paid once for
+// them, and reads the next four rows while it quantises these; bound there by instruction issue.  A small step (fewer
+// than kFewPasses passes in all: they fit the GPU at once) is a chain of latencies instead, so it gives a warp one pass, and
+// the table entries are requested in one go on the guess that the token is its sequence's only one.
+// Measured cold, 8 KV heads (before: a warp per token, conversions per value): 2 and 64 f16 tokens 11 -> 4.5 us, 8312 bf16
+// tokens 25.6 -> 17.8 us.
 template <typename T>
 __device__ __forceinline__ float bits_to_f32(uint32_t h16);
 template <>
@@ -191,23 +197,55 @@ __device__ __forceinline__ float bits_to_f32<__nv_bfloat16>(uint32_t h16) {
 // sits at the same place in the registers of the lane four lanes away; rotated values are arbitrary float32
 // numbers, for which the reciprocal shortcut below is not proved, so those rows take the division itself.
 template <typename T, bool kRope>
-__global__ void __launch_bounds__(kWarpsPerCta * 32) paged_kv_store_rows128_kernel(const StoreParams p) {
+__global__ void __launch_bounds__(kWarpsPerCta * 32, kRope ? 2 : 4) paged_kv_store_rows128_kernel(const StoreParams p, const int passes_per_warp) {
     constexpr int D = 128;
     const int lane = threadIdx.x & 31, l8 = lane & 7, rg = lane >> 3;
-    const int tok = static_cast<int>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5);
+    const int rows = 2 * p.Hkv;  // row r: head r >> 1, key (0) or value (1)
+    const int passes = (rows + 3) / 4, warps_per_token = (passes + passes_per_warp - 1) / passes_per_warp;
+    const long long item = static_cast<long long>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5);
+    const int tok = static_cast<int>(item / warps_per_token);
+    const int first = static_cast<int>(item - static_cast<long long>(tok) * warps_per_token) * passes_per_warp * 4;
+    const int last = min(rows, first + passes_per_warp * 4);
     grid_dependency_wait();  // the new key/value rows (and the pool's previous readers) belong to earlier kernels
     grid_launch_dependents();
     if (tok >= p.t.num_tokens) return;
-    const int seq = find_sequence(p.t, tok, lane);
-    if (seq < 0) return;  // not scheduled
-    const int pos = p.t.past_lens[seq] + (tok - p.t.subsequence_begins[seq]);
+    uint4 next0 = make_uint4(0u, 0u, 0u, 0u), next1 = next0;
+    auto fetch = [&](int r) {  // this lane's 16 values of row r
+        if (r < last) {
+            const uint4* src = reinterpret_cast<const uint4*>(
+                reinterpret_cast<const T*>((r & 1) ? p.value : p.key) + (static_cast<size_t>(tok) * p.Hkv + (r >> 1)) * D);
+            next0 = src[2 * l8];
+            next1 = src[2 * l8 + 1];
+        }
+    };
+    fetch(first + rg);
+    // the token's sequence: itself in a step of one-token sequences, else by search; the entries of the guess are
+    // requested together with the two that confirm it
+    int seq = -1, past = 0, begin = 0, bib0 = 0, bib1 = 0;
+    if (tok < p.t.num_seqs) {
+        const int b0 = p.t.subsequence_begins[0], bn = p.t.subsequence_begins[p.t.num_seqs];
+        const int mine = p.t.subsequence_begins[tok], after = p.t.subsequence_begins[tok + 1];
+        past = p.t.past_lens[tok];
+        bib0 = p.t.block_indices_begins[tok];
+        bib1 = p.t.block_indices_begins[tok + 1];
+        begin = mine;
+        if (mine <= tok && tok < after && b0 <= tok && tok < bn) seq = tok;
+    }
+    if (seq < 0) {
+        seq = find_sequence(p.t, tok, lane);
+        if (seq < 0) return;  // not scheduled
+        past = p.t.past_lens[seq];
+        begin = p.t.subsequence_begins[seq];
+        bib0 = p.t.block_indices_begins[seq];
+        bib1 = p.t.block_indices_begins[seq + 1];
+    }
+    const int pos = past + (tok - begin);
     const int bs = p.t.block_size;
-    const int nblk_seq = p.t.block_indices_begins[seq + 1] - p.t.block_indices_begins[seq];
-    if (pos < 0 || pos / bs >= nblk_seq) {
+    if (pos < 0 || pos / bs >= bib1 - bib0) {
         if (lane == 0) report(p.status, B2A_DEV_BAD_LEN);
         return;
     }
-    const int blk = p.t.block_indices[p.t.block_indices_begins[seq] + pos / bs];
+    const int blk = p.t.block_indices[bib0 + pos / bs];
     if (blk < 0 || blk >= p.t.num_blocks_total) {
         if (lane == 0) report(p.status, B2A_DEV_BAD_BLOCK);
         return;
@@ -218,18 +256,11 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) paged_kv_store_rows128_kern
         return;
     }
     const size_t chunk_bytes = u8_chunk_bytes(bs, D);
-    const int rows = 2 * p.Hkv;  // row r: head r >> 1, key (0) or value (1)
-    for (int r0 = 0; r0 < rows; r0 += 4) {
+    for (int r0 = first; r0 < last; r0 += 4) {
         const int r = r0 + rg;
-        const bool live = r < rows;  // whole 8-lane groups are live or not: the shuffles below stay inside a group
-        uint4 raw0 = make_uint4(0u, 0u, 0u, 0u), raw1 = raw0;
-        if (live) {
-            const uint4* src = reinterpret_cast<const uint4*>(
-                reinterpret_cast<const T*>((r & 1) ? p.value : p.key) + (static_cast<size_t>(tok) * p.Hkv + (r >> 1)) * D);
-            raw0 = src[2 * l8];
-            raw1 = src[2 * l8 + 1];
-        }
-        const uint32_t w[8] = {raw0.x, raw0.y, raw0.z, raw0.w, raw1.x, raw1.y, raw1.z, raw1.w};
+        const bool live = r < last;  // whole 8-lane groups are live or not: the shuffles below stay inside a group
+        const uint32_t w[8] = {next0.x, next0.y, next0.z, next0.w, next1.x, next1.y, next1.z, next1.w};
+        fetch(r + 4);
         float xv[16];
         float mn = INFINITY, mx = -INFINITY;
 #pragma unroll
@@ -266,21 +297,32 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) paged_kv_store_rows128_kern
         const float zf = __half2float(z16);
         // x / s for the row's values with ONE reciprocal: q0 = x * r, then one Newton step in fused arithmetic.
         // For a scale that is an f16 value and x an f16 or bf16 value this equals the correctly rounded quotient in
-        // every case except |x| below 2^-116, which take the division itself (checked exhaustively on the CPU by
-        // oracle/div_by_scale_check.c).
+        // every case except |x| below 2^-116 (checked exhaustively on the CPU by oracle/div_by_scale_check.c) - and
+        // such a quotient, below 2^-92 whichever way it is rounded (s is at least 2^-24), is lost in the sum with zp,
+        // zero or at least 2^-24: the code is the same.  A row with an infinity (or without a number) has s = 1:
+        // x / s is x, where the Newton step would make a NaN of it.
+        // rint and clamp commute (the bounds are integers), and adding 2^23 to a value in 0..255 rounds it to an
+        // integer, ties to even, in the low byte: no conversion instruction, whose rate is a quarter of the adder's.
+        const bool finite = mn > -INFINITY && mx < INFINITY && mn <= mx;
         const float rs = __frcp_rn(sf);
-        uint32_t packed[4] = {0u, 0u, 0u, 0u};
+        uint32_t packed[4];
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-            float q;
-            if (rotated || fabsf(xv[e]) < 1e-30f) {
-                q = __fdiv_rn(xv[e], sf);
-            } else {
-                const float q0 = __fmul_rn(xv[e], rs);
-                q = fabsf(q0) < INFINITY ? __fmaf_rn(__fmaf_rn(-sf, q0, xv[e]), rs, q0) : q0;
+        for (int i = 0; i < 4; ++i) {
+            uint32_t code[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float x = xv[4 * i + u];
+                float q;
+                if (kRope && rotated) {
+                    q = __fdiv_rn(x, sf);
+                } else {
+                    const float q0 = __fmul_rn(x, rs);
+                    const float q1 = __fmaf_rn(__fmaf_rn(-sf, q0, x), rs, q0);
+                    q = finite ? q1 : x;
+                }
+                code[u] = __float_as_uint(__fadd_rn(fminf(fmaxf(__fadd_rn(q, zf), 0.f), 255.f), 8388608.f));
             }
-            const float t = rintf(__fadd_rn(q, zf));
-            packed[e >> 2] |= static_cast<uint32_t>(fminf(fmaxf(t, 0.f), 255.f)) << (8 * (e & 3));
+            packed[i] = __byte_perm(__byte_perm(code[0], code[1], 0x0040), __byte_perm(code[2], code[3], 0x0040), 0x5410);
         }
         if (live) {
             uint8_t* chunk = ((r & 1) ? p.v_cache : p.k_cache) + (static_cast<size_t>(blk) * p.Hkv + (r >> 1)) * chunk_bytes;
@@ -311,15 +353,18 @@ int paged_kv_store_launch(const b2a_paged_desc& d, const void* key, const void* 
     auto al8 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
     if (d.kv_dtype == B2A_U8 && d.D == 128 && d.Dv == 128 && (d.q_dtype == B2A_F16 || d.q_dtype == B2A_BF16) &&
         al8(key) && al8(value) && (p.rotary_dim == 0 || rope_all)) {
-        const unsigned grid_t = static_cast<unsigned>((d.num_tokens + kWarpsPerCta - 1) / kWarpsPerCta);
+        const int passes = (2 * d.Hkv + 3) / 4;
+        const int per_warp = static_cast<long long>(d.num_tokens) * passes <= kFewPasses ? 1 : passes;
+        const long long warps = static_cast<long long>(d.num_tokens) * ((passes + per_warp - 1) / per_warp);
+        const unsigned grid_t = static_cast<unsigned>((warps + kWarpsPerCta - 1) / kWarpsPerCta);
         const dim3 block(kWarpsPerCta * 32);
         cudaError_t e;
         if (d.q_dtype == B2A_F16)
-            e = rope_all ? launch_overlapped(paged_kv_store_rows128_kernel<__half, true>, dim3(grid_t), block, 0, stream, p)
-                         : launch_overlapped(paged_kv_store_rows128_kernel<__half, false>, dim3(grid_t), block, 0, stream, p);
+            e = rope_all ? launch_overlapped(paged_kv_store_rows128_kernel<__half, true>, dim3(grid_t), block, 0, stream, p, per_warp)
+                         : launch_overlapped(paged_kv_store_rows128_kernel<__half, false>, dim3(grid_t), block, 0, stream, p, per_warp);
         else
-            e = rope_all ? launch_overlapped(paged_kv_store_rows128_kernel<__nv_bfloat16, true>, dim3(grid_t), block, 0, stream, p)
-                         : launch_overlapped(paged_kv_store_rows128_kernel<__nv_bfloat16, false>, dim3(grid_t), block, 0, stream, p);
+            e = rope_all ? launch_overlapped(paged_kv_store_rows128_kernel<__nv_bfloat16, true>, dim3(grid_t), block, 0, stream, p, per_warp)
+                         : launch_overlapped(paged_kv_store_rows128_kernel<__nv_bfloat16, false>, dim3(grid_t), block, 0, stream, p, per_warp);
         return e == cudaSuccess ? B2A_OK : B2A_ERR_CUDA;
     }
     const long long total = 2LL * d.num_tokens * d.Hkv;

@@ -217,6 +217,17 @@ int b2a_paged_last_token_scores(const b2a_paged_desc* desc, const void* query, c
                                 int64_t scores_capacity, int32_t* score_begins, void* workspace, size_t workspace_bytes,
                                 int32_t* status, b2a_stream_t stream);
 
+/* b2a_paged_attention and b2a_paged_last_token_scores of one step in which every sequence has exactly one new token, in
+ * the launches of the first alone: the decode kernel leaves the scores it computes anyway.  `table_blocks`: entries of
+ * block_indices; the workspace grows by 64 * Hq bytes for each.  Outputs as of the two calls (a sequence with several
+ * new tokens reports B2A_DEV_BAD_LEN).  B2A_ERR_UNSUPPORTED where either call's geometry is not met. */
+int b2a_paged_attention_scores_workspace_bytes(const b2a_paged_desc* desc, int sm_count, int64_t table_blocks, size_t* out_bytes);
+int b2a_paged_attention_scores(const b2a_paged_desc* desc, const void* query, const void* k_cache, const void* v_cache,
+                               const int32_t* past_lens, const int32_t* subsequence_begins, const int32_t* block_indices,
+                               const int32_t* block_indices_begins, int64_t table_blocks, void* out, float* scores,
+                               int64_t scores_capacity, int32_t* score_begins, void* workspace, size_t workspace_bytes,
+                               int32_t* status, b2a_stream_t stream);
+
 /* ---------------------------------------------------------------------------------------------
  * Head-sharded attention over the GPUs of one node (one rank per GPU).
  *

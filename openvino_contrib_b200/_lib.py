@@ -54,6 +54,9 @@ SIGNATURES = {
     "b2a_paged_attention_noalloc": (C.c_int, [C.POINTER(PagedDesc), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
                                               C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "b2a_paged_scores_workspace_bytes": (C.c_int, [C.POINTER(PagedDesc), C.c_int, C.POINTER(C.c_size_t)]),
+    "b2a_paged_attention_scores_workspace_bytes": (C.c_int, [C.POINTER(PagedDesc), C.c_int, C.c_int64, C.POINTER(C.c_size_t)]),
+    "b2a_paged_attention_scores": (C.c_int, [C.POINTER(PagedDesc)] + [C.c_void_p] * 7 + [C.c_int64, C.c_void_p, C.c_void_p, C.c_int64,
+                                             C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p, C.c_void_p]),
     "b2a_paged_last_token_scores": (C.c_int, [C.POINTER(PagedDesc), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
                                               C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p,
                                               C.c_size_t, C.c_void_p, C.c_void_p]),

@@ -304,6 +304,55 @@ int b2a_paged_attention_noalloc(const b2a_paged_desc* desc, const void* query, c
         reinterpret_cast<cudaStream_t>(stream));
 }
 
+// layout: [split-K partials, rounded up to 256 bytes][scaled scores of every key of the table's blocks]
+static int decode_scores_layout(const b2a_paged_desc& d, int sm_count, int64_t table_blocks, size_t& raw_at, size_t& total) {
+    if (!paged_decode_supported(d) || !paged_scores_supported(d)) return B2A_ERR_UNSUPPORTED;
+    if (d.max_context_len <= 0 || table_blocks < 0 || table_blocks > INT32_MAX) return B2A_ERR_DIM;
+    raw_at = (paged_decode_plan(d, sm_count).workspace_bytes + 255) & ~static_cast<size_t>(255);
+    total = raw_at + static_cast<size_t>(table_blocks) * d.block_size * d.Hq * sizeof(float);
+    return B2A_OK;
+}
+
+int b2a_paged_attention_scores_workspace_bytes(const b2a_paged_desc* desc, int sm_count, int64_t table_blocks, size_t* out_bytes) {
+    if (out_bytes == nullptr) return B2A_ERR_NULL;
+    b2a_paged_desc d;
+    const int rc = resolve_paged_desc(desc, d);
+    if (rc != B2A_OK) return rc;
+    if (sm_count <= 0) sm_count = device_sm_count();
+    if (sm_count <= 0) sm_count = 148;
+    size_t raw_at = 0;
+    return decode_scores_layout(d, sm_count, table_blocks, raw_at, *out_bytes);
+}
+
+int b2a_paged_attention_scores(const b2a_paged_desc* desc, const void* query, const void* k_cache, const void* v_cache,
+                               const int32_t* past_lens, const int32_t* subsequence_begins, const int32_t* block_indices,
+                               const int32_t* block_indices_begins, int64_t table_blocks, void* out, float* scores,
+                               int64_t scores_capacity, int32_t* score_begins, void* workspace, size_t workspace_bytes,
+                               int32_t* status, b2a_stream_t stream) {
+    b2a_paged_desc d;
+    const int rc = resolve_paged_desc(desc, d);
+    if (rc != B2A_OK) return rc;
+    if (d.num_tokens == 0 || d.num_seqs == 0) return B2A_OK;
+    if (query == nullptr || k_cache == nullptr || v_cache == nullptr || out == nullptr || past_lens == nullptr ||
+        subsequence_begins == nullptr || block_indices == nullptr || block_indices_begins == nullptr || scores == nullptr ||
+        score_begins == nullptr)
+        return B2A_ERR_NULL;
+    if (scores_capacity < 0) return B2A_ERR_DIM;
+    if (!aligned(k_cache, 16) || !aligned(v_cache, 16) || !aligned(query, 16) || !aligned(out, 16)) return B2A_ERR_ALIGN;
+    const int sms = device_sm_count();
+    if (sms <= 0) return B2A_ERR_CUDA;
+    size_t raw_at = 0, need = 0;
+    const int rc2 = decode_scores_layout(d, sms, table_blocks, raw_at, need);
+    if (rc2 != B2A_OK) return rc2;
+    if (workspace == nullptr || workspace_bytes < need) return B2A_ERR_WORKSPACE;
+    if (!aligned(workspace, 16)) return B2A_ERR_ALIGN;
+    const DecodeScores sc{reinterpret_cast<float*>(static_cast<char*>(workspace) + raw_at), static_cast<int>(table_blocks), scores,
+                          scores_capacity, score_begins};
+    return paged_decode_launch(d, paged_decode_plan(d, sms), query, k_cache, v_cache,
+                               tables_of(d, past_lens, subsequence_begins, block_indices, block_indices_begins), out, workspace,
+                               status, reinterpret_cast<cudaStream_t>(stream), nullptr, nullptr, &sc);
+}
+
 int b2a_paged_scores_workspace_bytes(const b2a_paged_desc* desc, int sm_count, size_t* out_bytes) {
     if (out_bytes == nullptr) return B2A_ERR_NULL;
     b2a_paged_desc d;

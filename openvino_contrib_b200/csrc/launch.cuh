@@ -87,8 +87,17 @@ DecodePlan paged_decode_plan(const b2a_paged_desc& d, int sm_count);
 // the ordinary way behind a wait on the event, so it - and whatever follows it on the stream - comes after both.
 int paged_decode_launch(const b2a_paged_desc& d, const DecodePlan& plan, const void* query, const void* k_cache,
                         const void* v_cache, const PagedTables& t, void* out, void* workspace, int32_t* status,
-                        cudaStream_t stream, const PeerPush* push = nullptr, cudaEvent_t beside_predecessor = nullptr);
+                        cudaStream_t stream, const PeerPush* push = nullptr, cudaEvent_t beside_predecessor = nullptr,
+                        const struct DecodeScores* scores = nullptr);
 
+// Score output of a pure decode step, from the scores the decode kernel computes anyway (at most eight query heads per KV head)
+struct DecodeScores {
+    float* raw;         // scratch [raw_blocks][Hkv][16][G]
+    int raw_blocks;     // entries of the step's block table
+    float* scores;
+    long long capacity;
+    int32_t* begins;    // [num_seqs + 1]
+};
 // Same launch with the split-K partials in the library's built-in device array instead of a caller workspace.
 int paged_decode_launch_builtin_scratch(const b2a_paged_desc& d, const DecodePlan& plan, const void* query,
                                         const void* k_cache, const void* v_cache, const PagedTables& t, void* out,

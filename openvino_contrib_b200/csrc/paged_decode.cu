@@ -61,6 +61,13 @@ struct DecodeParams {
     int beside_predecessor;      // see paged_decode_launch: no wait for the kernel before this one
     int cache_rows_settled;      // b2a_paged_desc: the kernel before this one writes no cache row but the new tokens'
     cudaEvent_t predecessor_done;  // host side only: completes with that kernel
+    // score output (kMode 3): the scaled scores of every cached key, base-2 units, [block of the table][Hkv][16 keys][G]
+    float* raw_scores;
+    int raw_blocks;          // blocks that array holds
+    float* scores;           // the caller's flat scores, its capacity and offsets
+    long long scores_capacity;
+    int32_t* score_begins;
+    int max_blocks;          // blocks of the longest admitted context
     PeerPush push;     // world == 0 unless the heads are sharded over several GPUs
 };
 
@@ -156,7 +163,9 @@ enum ChunkState {
 // met; so are the first cache blocks of a CTA that does not hold its sequence's last block.  Everything an earlier
 // kernel of the step produces - the query rows, the cache rows of the new tokens, the workspace, the status word, the
 // exchange's counters - is touched only after the wait.
-template <typename T, int NT, bool kRowIsSeq, int kWarps>
+//
+// With kScores the scaled scores also go to memory (raw_scores), for the kernel that turns them into probabilities.
+template <typename T, int NT, bool kRowIsSeq, int kWarps, bool kScores = false>
 __device__ __forceinline__ ChunkState decode_chunk(const DecodeParams& p, uint8_t* smem, int& nsplit, int& tok_out,
                                                    const bool wait_for_predecessor) {
     const int hk = blockIdx.x, seq = blockIdx.y, split = blockIdx.z;
@@ -350,6 +359,20 @@ __device__ __forceinline__ ChunkState decode_chunk(const DecodeParams& p, uint8_
             const float s1 = ok0 ? (sc[nt][1] - zk0 * qsum_b[nt]) * sk0 : -INFINITY;
             const float s2 = ok1 ? (sc[nt][2] - zk1 * qsum_a[nt]) * sk1 : -INFINITY;
             const float s3 = ok1 ? (sc[nt][3] - zk1 * qsum_b[nt]) * sk1 : -INFINITY;
+            if constexpr (kScores) {  // (one group of eight heads: NT == 1)
+                if (bib0 + lb < p.raw_blocks) {
+                    float* raw = p.raw_scores + ((static_cast<size_t>(bib0 + lb) * p.Hkv + hk) * kBS + gid) * p.G;
+                    if ((p.G & 1) == 0) {
+                        if (2 * tid4 < p.G) {
+                            *reinterpret_cast<float2*>(raw + 2 * tid4) = make_float2(s0, s1);
+                            *reinterpret_cast<float2*>(raw + 8 * p.G + 2 * tid4) = make_float2(s2, s3);
+                        }
+                    } else {
+                        if (2 * tid4 < p.G) raw[2 * tid4] = s0, raw[8 * p.G + 2 * tid4] = s2;
+                        if (2 * tid4 + 1 < p.G) raw[2 * tid4 + 1] = s1, raw[8 * p.G + 2 * tid4 + 1] = s3;
+                    }
+                }
+            }
             float ta = fmaxf(s0, s2), tb = fmaxf(s1, s3);
 #pragma unroll
             for (int o = 4; o <= 16; o <<= 1) {
@@ -640,6 +663,7 @@ __device__ __forceinline__ void receive_row(const PeerPush& push, uint32_t* out,
 }
 
 // kMode 0: the CTA leaves its partial in the workspace and paged_decode_merge_kernel follows (single GPU).
+// kMode 3: the same, and the scaled scores of every key go to memory; paged_decode_merge_scores_kernel follows.
 // kMode 1, 2: the whole step of a head shard in this launch (PeerPush).  After its chunk a CTA takes a ticket of its
 // (sequence, KV head); the CTA that gets the last ticket merges the group's partials and delivers the rows to every
 // rank - mode 1 as low-latency words for the receiving kernel, mode 2 in place: there the rows land in the ranks'
@@ -654,8 +678,8 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) paged_decode_kernel(
     // after its table walk (beside the prefill kernel of a mixed step there is nothing to wait for: that kernel waited
     // for them already and is not waited for itself)
     const bool wait_for_predecessor = !p.beside_predecessor;
-    if constexpr (kMode == 0) {
-        decode_chunk<T, NT, false, kWarps>(p, smem, nsplit, tok, wait_for_predecessor);
+    if constexpr (kMode == 0 || kMode == 3) {
+        decode_chunk<T, NT, false, kWarps, kMode == 3>(p, smem, nsplit, tok, wait_for_predecessor);
     } else {
         constexpr bool kLL = kMode == 1;
         __shared__ int s_role;
@@ -745,8 +769,8 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) paged_decode_kernel(
 // m = max_s m_s.  The (m, l) pairs are read as 8-byte loads and both loops are unrolled so that eight partials are in
 // flight per thread (the loads are independent; only the tiny accumulation is a chain).
 template <typename T>
-__global__ void __launch_bounds__(kD) paged_decode_merge_kernel(const DecodeParams p) {
-    const int h = blockIdx.x, seq = blockIdx.y, d = threadIdx.x;
+__device__ __forceinline__ void merge_head(const DecodeParams& p, const int h, const int seq) {
+    const int d = threadIdx.x;
     // the step's tables are read while the decode kernel drains (see decode_chunk), the partials after the wait
     const int tok = __ldcg(p.t.subsequence_begins + seq);
     const int qlen = __ldcg(p.t.subsequence_begins + seq + 1) - tok;
@@ -798,6 +822,99 @@ __global__ void __launch_bounds__(kD) paged_decode_merge_kernel(const DecodePara
     }
     T* orow = reinterpret_cast<T*>(p.out) + (static_cast<size_t>(tok) * p.Hq + h) * kD;
     orow[d] = from_f32<T>(l > 0.f ? o / l : 0.f);
+}
+template <typename T>
+__global__ void __launch_bounds__(kD) paged_decode_merge_kernel(const DecodeParams p) {
+    merge_head<T>(p, blockIdx.x, blockIdx.y);
+}
+
+// The merge of a step that also wants the attention probabilities of every key, summed over the heads (the operator's
+// score output).  CTAs below Hq merge a head; each of the others takes 512 positions of the sequence: it merges the
+// splits' (max, sum) pairs into lse[h] = max + log2(sum) and writes sum_h 2^(score - lse[h]) from the scores the decode
+// kernel left.  Where the sequence starts in the flat output is the sum of the contexts before it, worked out from the
+// tables while the decode kernel drains.
+// Against two passes of their own over K (paged_scores.cu) this trades 2 x 132 bytes read per key and KV head for 8 G
+// bytes written and read, mostly in L2, and four launches for none: 32 sequences of 512..4096 tokens, 32/8 heads, the
+// whole step 107 -> 46.6 us.
+constexpr int kScorePositions = 512;
+template <typename T>
+__global__ void __launch_bounds__(kD) paged_decode_merge_scores_kernel(const DecodeParams p) {
+    const int seq = blockIdx.y;
+    if (static_cast<int>(blockIdx.x) < p.Hq) {
+        merge_head<T>(p, blockIdx.x, seq);
+        return;
+    }
+    __shared__ float s_lse[128];
+    __shared__ long long s_part[kD / 32];
+    const int tid = threadIdx.x, chunk = static_cast<int>(blockIdx.x) - p.Hq;
+    // entries of sequence s: its context when it has a new token and consistent tables, else none
+    auto entries = [&](int s, bool& bad) {
+        const int t0 = __ldcg(p.t.subsequence_begins + s), t1 = __ldcg(p.t.subsequence_begins + s + 1);
+        const int past = __ldcg(p.t.past_lens + s);
+        const int have = __ldcg(p.t.block_indices_begins + s + 1) - __ldcg(p.t.block_indices_begins + s);
+        const int ctx = past + (t1 - t0), nblk = (ctx + kBS - 1) / kBS;
+        bad = t1 > t0 && (past < 0 || t0 < 0 || t1 > p.t.num_tokens || nblk > have || nblk > p.max_blocks);
+        return t1 > t0 && !bad ? ctx : 0;
+    };
+    bool bad = false, other = false;
+    const int mine = entries(seq, bad);
+    const int tok = __ldcg(p.t.subsequence_begins + seq);
+    const bool one_token = __ldcg(p.t.subsequence_begins + seq + 1) - tok == 1;
+    const int bib0 = __ldcg(p.t.block_indices_begins + seq);
+    long long before = 0;
+    for (int s = tid; s < seq; s += kD) before += entries(s, other);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    if ((tid & 31) == 0) s_part[tid >> 5] = before;
+    __syncthreads();
+    before = s_part[0] + s_part[1] + s_part[2] + s_part[3];
+
+    grid_dependency_wait();
+    grid_launch_dependents();
+    if (chunk == 0 && tid == 0) {
+        p.score_begins[seq] = static_cast<int32_t>(before);
+        if (seq == p.t.num_seqs - 1) p.score_begins[seq + 1] = static_cast<int32_t>(before + mine);
+        // (a sequence of several new tokens has no row here: the caller promised a step of single tokens)
+        if (bad || before + mine > p.scores_capacity || (mine > 0 && !one_token)) report(p.status, B2A_DEV_BAD_LEN);
+    }
+    const int first = chunk * kScorePositions, end = min(mine, first + kScorePositions);
+    if (first >= end || before + mine > p.scores_capacity) return;  // nothing past the caller's buffer is written
+    const int first_pos = p.sliding_window > 0 ? max(0, mine - p.sliding_window) : 0, blk_lo = first_pos / kBS;
+    const int nblk = (mine + kBS - 1) / kBS;
+    const int nsplit = min(p.max_splits, (nblk - blk_lo + p.blocks_per_cta - 1) / p.blocks_per_cta);
+    if (tid < p.Hq) {
+        const float2* ml = reinterpret_cast<const float2*>(p.ws_ml) + (static_cast<size_t>(seq) * p.Hq + tid) * p.max_splits;
+        float mc = kNegBig, l = 0.f;
+#pragma unroll 4
+        for (int i = 0; i < nsplit; ++i) mc = fmaxf(mc, ml[i].x);
+#pragma unroll 4
+        for (int i = 0; i < nsplit; ++i) {
+            const float2 v = ml[i];
+            l += v.y * ex2(v.x - mc);
+        }
+        s_lse[tid] = mc + log2f(l);
+    }
+    __syncthreads();
+    for (int pos = first + tid; pos < end; pos += kD) {
+        float sum = 0.f;
+        const int block = bib0 + pos / kBS;
+        if (pos >= first_pos && one_token && block < p.raw_blocks) {
+            const float* raw = p.raw_scores + (static_cast<size_t>(block) * p.Hkv * kBS + pos % kBS) * p.G;
+            if (p.G == 4) {
+#pragma unroll 4
+                for (int hk = 0; hk < p.Hkv; ++hk) {
+                    const float4 x = *reinterpret_cast<const float4*>(raw + static_cast<size_t>(hk) * kBS * 4);
+                    sum += (ex2(x.x - s_lse[4 * hk]) + ex2(x.y - s_lse[4 * hk + 1])) +
+                           (ex2(x.z - s_lse[4 * hk + 2]) + ex2(x.w - s_lse[4 * hk + 3]));
+                }
+            } else {
+#pragma unroll 2
+                for (int hk = 0; hk < p.Hkv; ++hk)
+                    for (int g = 0; g < p.G; ++g) sum += ex2(raw[static_cast<size_t>(hk) * kBS * p.G + g] - s_lse[hk * p.G + g]);
+            }
+        }
+        p.scores[before + pos] = sum;
+    }
 }
 
 // Receiver of the low-latency exchange as a kernel of its own, one CTA per row, for steps with more rows than the
@@ -857,6 +974,18 @@ int launch_t(const DecodeParams& p, int num_seqs, cudaStream_t stream) {
                    ? B2A_OK
                    : B2A_ERR_CUDA;
     }
+    if (p.raw_scores != nullptr) {
+        if constexpr (NT == 1) {
+            const int rc = launch_kernel<T, NT, 3>(p, num_seqs, stream);
+            if (rc != B2A_OK) return rc;
+            const int chunks = (p.max_blocks * kBS + kScorePositions - 1) / kScorePositions;
+            return launch_overlapped(paged_decode_merge_scores_kernel<T>, dim3(p.Hq + chunks, num_seqs), dim3(kD), 0, stream, p) ==
+                           cudaSuccess
+                       ? B2A_OK
+                       : B2A_ERR_CUDA;
+        }
+        return B2A_ERR_UNSUPPORTED;
+    }
     const int rc = launch_kernel<T, NT, 0>(p, num_seqs, stream);
     if (rc != B2A_OK) return rc;
     if (p.beside_predecessor) {
@@ -913,8 +1042,17 @@ DecodePlan paged_decode_plan(const b2a_paged_desc& d, int sm_count) {
 
 int paged_decode_launch(const b2a_paged_desc& d, const DecodePlan& plan, const void* query, const void* k_cache,
                         const void* v_cache, const PagedTables& t, void* out, void* workspace, int32_t* status,
-                        cudaStream_t stream, const PeerPush* push, cudaEvent_t beside_predecessor) {
+                        cudaStream_t stream, const PeerPush* push, cudaEvent_t beside_predecessor,
+                        const DecodeScores* scores) {
     DecodeParams p{};
+    if (scores != nullptr) {
+        p.raw_scores = scores->raw;
+        p.raw_blocks = scores->raw_blocks;
+        p.scores = scores->scores;
+        p.scores_capacity = scores->capacity;
+        p.score_begins = scores->begins;
+        p.max_blocks = (d.max_context_len + kBS - 1) / kBS;
+    }
     if (push != nullptr) p.push = *push;
     // the rows are received by CTAs of the decode kernel itself while there are no more rows than SMs
     if (push != nullptr && p.push.ll) p.push.receive_in_kernel = d.num_seqs <= device_sm_count() ? 1 : 0;

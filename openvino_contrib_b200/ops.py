@@ -357,6 +357,50 @@ def paged_last_token_scores(query: torch.Tensor, cache: PagedKvCache, past_lens,
     return scores, begins
 
 
+# Scratch of paged_attention_scores beyond which a step takes the two-call form, which needs next to none.
+_SCORE_SCRATCH_LIMIT = 1 << 30
+
+
+def paged_attention_scores(query: torch.Tensor, cache: PagedKvCache, past_lens, subsequence_begins, block_indices,
+                           block_indices_begins, hq: int, max_context_len: int, scale: Optional[float] = None,
+                           sliding_window: int = 0, out: Optional[torch.Tensor] = None,
+                           scores: Optional[torch.Tensor] = None, stream=None, status: Optional[torch.Tensor] = None,
+                           cache_rows_settled: bool = False):
+    """``paged_attention`` and ``paged_last_token_scores`` of a step of one-token sequences, from one walk over the
+    cache.  Returns ``(out, scores, score_begins)``, or None where the kernels do not take the step (more than one
+    token per sequence, another geometry, or more scratch than ``_SCORE_SCRATCH_LIMIT``): make the two calls then."""
+    num_tokens, num_seqs = query.shape[0], past_lens.shape[0]
+    if num_tokens != num_seqs or num_seqs == 0:
+        return None
+    d = _paged_desc(query.dtype, cache, hq, num_seqs, num_tokens, max_context_len, 1, scale, sliding_window, 0, 0,
+                    cache_rows_settled)
+    lib = _lib.load()
+    ws = C.c_size_t(0)
+    blocks = block_indices.numel()
+    if lib.b2a_paged_attention_scores_workspace_bytes(C.byref(d), 0, blocks, C.byref(ws)) != 0 or ws.value > _SCORE_SCRATCH_LIMIT:
+        return None
+    _require_cuda(query, cache.k, cache.v, past_lens, subsequence_begins, block_indices, block_indices_begins, out, scores)
+    if not query.is_contiguous() or query.shape[1] != hq * cache.d:
+        raise ValueError("query must be dense [tokens, Hq*D]")
+    if out is None:
+        out = torch.empty((num_tokens, hq * cache.dv), dtype=query.dtype, device=query.device)
+    if scores is None:
+        scores = torch.empty(num_seqs * max_context_len, dtype=torch.float32, device=query.device)
+    if scores.dtype != torch.float32 or not scores.is_contiguous():
+        raise TypeError("scores must be a contiguous float32 tensor")
+    begins = torch.empty(num_seqs + 1, dtype=torch.int32, device=query.device)
+    workspace = torch.empty(max(16, ws.value), dtype=torch.uint8, device=query.device)
+    check(lib.b2a_paged_attention_scores(C.byref(d), query.data_ptr(), cache.k.data_ptr(), cache.v.data_ptr(),
+                                         _i32(past_lens).data_ptr(), _i32(subsequence_begins).data_ptr(),
+                                         _i32(block_indices).data_ptr(), _i32(block_indices_begins).data_ptr(), blocks,
+                                         out.data_ptr(), scores.data_ptr(), scores.numel(), begins.data_ptr(),
+                                         workspace.data_ptr(), workspace.numel(), _ptr(status), _stream_ptr(stream)),
+          "b2a_paged_attention_scores")
+    if stream is not None:  # the scratch may be handed out again only behind the kernels that use it
+        workspace.record_stream(stream)
+    return out, scores, begins
+
+
 class PagedAttentionOp:
     """Operator-shaped wrapper for ``PagedAttentionExtension`` (the Python twin of the C++ ``PagedAttentionOp``).
 
@@ -442,6 +486,13 @@ class PagedAttentionOp:
         rb, kvt = self.step_hints(num_tokens, num_seqs, prefill_row_blocks, prefill_kv_tokens)
         paged_kv_store(key, value, cache, past_lens, subsequence_begins, block_indices, block_indices_begins,
                        stream=stream, status=status)
+        if len(outputs) > 1 and outputs[1] is not None:
+            done = paged_attention_scores(query, cache, past_lens, subsequence_begins, block_indices, block_indices_begins,
+                                          self.hq, self.max_context_len, self.scale if sc is None else float(sc),
+                                          self.sliding_window, out=outputs[0], scores=outputs[1], stream=stream,
+                                          status=status, cache_rows_settled=True)
+            if done is not None:
+                return done[2]
         paged_attention(query, cache, past_lens, subsequence_begins, block_indices, block_indices_begins,
                         self.hq, self.max_context_len, max_q_len, self.scale if sc is None else float(sc),
                         self.sliding_window, out=outputs[0], workspace=ws, stream=stream,

@@ -87,8 +87,7 @@ struct TcParams {
     const uint8_t* v_cache;
     PagedTables t;
     void* out;        // [tokens, Hq*128]
-    const int* plan;  // work list built by paged_tc_plan_kernel: plan[0] = count, then (sequence, tile pair) entries
-    const int* kv_base;  // gathered K/V: first scratch row of every multi-token sequence
+    const int* plan;  // work list built by paged_tc_plan_kernel: header, then entries of kPlanEntryInts
 };
 
 // Output side of a head-sharded launch (world == 0: single GPU, the tmO map is the output).
@@ -106,6 +105,10 @@ struct TcPeers {
 // count (exact when the caller passes the scheduler's hint) instead of max_q_len x num_seqs, which for a step with
 // a few long prefills and many decode sequences would be almost all empty CTAs.
 constexpr int kPlanHeaderInts = 4;  // [0] items in the list (per KV head), [1] CTAs of the attention kernel that take items
+// An entry carries all that the attention kernel's warps have to know about the item, so that starting one costs them one
+// trip to memory instead of a chain of table lookups: {sequence, first token, new tokens (0: tables inconsistent), past
+// length}, {tile pair, first scratch row of the sequence, 0, 0}.
+constexpr int kPlanEntryInts = 8;
 // A mixed step runs its prefill rows (tensor-bound) and its decode rows (HBM-bound) at the same time: the attention
 // kernel keeps only as many SMs as its share of the step's work needs and the decode kernel, launched as soon as
 // those CTAs are seated, takes the rest (and the others as they come free).  The share is worked out here from the
@@ -162,13 +165,21 @@ __global__ void __launch_bounds__(256) paged_tc_plan_kernel(const PagedTables t,
         atomicAdd(&s_steps, steps);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {  // bucket w starts after all heavier buckets
-        int at = 0;
-        for (int w = kBuckets - 1; w >= 0; --w) {
-            const int n = s_hist[w];
-            s_hist[w] = at;
-            at += n;
+    {  // bucket w starts after all heavier buckets: one bucket per thread, lightest in the last
+        static_assert(kBuckets == 256, "a bucket per thread");
+        __shared__ int s_warp[kBuckets / 32];
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const int n = s_hist[kBuckets - 1 - threadIdx.x];
+        int upto = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += x;
         }
+        if (lane == 31) s_warp[warp] = upto;
+        __syncthreads();
+        for (int w = 0; w < warp; ++w) upto += s_warp[w];
+        s_hist[kBuckets - 1 - threadIdx.x] = upto - n;
     }
     grid_dependency_wait();
     grid_launch_dependents();
@@ -192,11 +203,19 @@ __global__ void __launch_bounds__(256) paged_tc_plan_kernel(const PagedTables t,
         if (qlen < 2) continue;
         const int past = max(0, t.past_lens[s]);
         const int pairs = (((qlen + 127) / 128) * G + 1) / 2;
+        // inconsistent tables (reported): the sequence's items are empty
+        const int tok0 = t.subsequence_begins[s], bib0 = t.block_indices_begins[s];
+        const bool ok = t.past_lens[s] >= 0 && tok0 >= 0 && tok0 + qlen <= t.num_tokens &&
+                        (past + qlen + 15) / 16 <= t.block_indices_begins[s + 1] - bib0;
+        if (!ok) report(status, B2A_DEV_BAD_LEN);
+        const int4 rec0 = make_int4(s, tok0, ok ? qlen : 0, past);
+        const int base = kv_base != nullptr ? kv_base[s] : 0;  // (written by this thread above)
         for (int i = 0; i < pairs; ++i) {
             const int at = atomicAdd(&s_hist[weight(past, qlen, i)], 1);
             if (at < capacity) {
-                plan[kPlanHeaderInts + 2 * at] = s;
-                plan[kPlanHeaderInts + 2 * at + 1] = i;
+                int4* rec = reinterpret_cast<int4*>(plan + kPlanHeaderInts) + 2 * at;
+                rec[0] = rec0;
+                rec[1] = make_int4(i, base, 0, 0);
             }
         }
     }
@@ -425,7 +444,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     struct Item {
         int b, hk, row0A, row0B, headA, headB, nkvA, nkvB, nmax, kv_tile0;
     };
-    int seq = 0, tok_base = 0, nrows_total = 0, pos_base = 0, kv_limit = 0;
+    int seq = 0, tok_base = 0, nrows_total = 0, pos_base = 0, kv_limit = 0, kv_row_base = 0;
     bool causal = true;
     int nrb = 0, tiles = 0, pairs = 0, total_items = 0;
     int active_ctas = static_cast<int>(gridDim.x);  // CTAs that take items
@@ -461,20 +480,19 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             const int e = idx / p.Hkv;
             it.b = 0;
             it.hk = idx - e * p.Hkv;
-            seq = p.plan[kPlanHeaderInts + 2 * e];
-            pair = p.plan[kPlanHeaderInts + 2 * e + 1];
-            tok_base = p.t.subsequence_begins[seq];
-            nrows_total = p.t.subsequence_begins[seq + 1] - tok_base;
-            pos_base = p.t.past_lens[seq];
+            const int4* rec = reinterpret_cast<const int4*>(p.plan + kPlanHeaderInts) + 2 * e;
+            const int4 r0 = rec[0], r1 = rec[1];
+            seq = r0.x;
+            tok_base = r0.y;
+            nrows_total = r0.z;
+            pos_base = r0.w;
+            pair = r1.x;
+            kv_row_base = r1.y;
             kv_limit = pos_base + nrows_total;
             nrb = (nrows_total + kBM - 1) / kBM;
             tiles = nrb * p.G;
             pairs = (tiles + 1) / 2;
-            const int nblk = (kv_limit + 15) / 16;
-            if (nrows_total < 2 || pos_base < 0 || tok_base < 0 || tok_base + nrows_total > p.t.num_tokens ||
-                nblk > p.t.block_indices_begins[seq + 1] - p.t.block_indices_begins[seq] || pair < 0 || pair >= pairs) {
-                // inconsistent tables: an empty item, reported once per item by the producer thread
-                if (threadIdx.x == 8 * 32) report(p.status, B2A_DEV_BAD_LEN);
+            if (nrows_total < 2 || pair >= pairs) {  // inconsistent tables (reported by the plan kernel): an empty item
                 it.hk = 0;
                 it.row0A = it.row0B = it.headA = it.headB = it.nkvA = it.nkvB = it.nmax = it.kv_tile0 = 0;
                 return true;
@@ -681,15 +699,21 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                     ++qn[X];
                     if (ok) {
                         uint4* tile = reinterpret_cast<uint4*>(gbase + X * kTile);
-                        for (int i = tp; i < kTile / 16; i += 64) {
-                            uint4 v = tile[i];
-                            uint32_t* w = reinterpret_cast<uint32_t*>(&v);
+                        // (eight pieces in flight: two warps have nothing else to hide shared memory's latency behind)
+                        for (int i = tp; i < kTile / 16; i += 64 * 8) {
+                            uint4 v[8];
 #pragma unroll
-                            for (int k = 0; k < 4; ++k) {
-                                const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[k]));
-                                w[k] = pack2<false>(fminf(fmaxf(f.x, -65504.f), 65504.f), fminf(fmaxf(f.y, -65504.f), 65504.f));
+                            for (int u = 0; u < 8; ++u) v[u] = tile[i + 64 * u];
+#pragma unroll
+                            for (int u = 0; u < 8; ++u) {
+                                uint32_t* w = reinterpret_cast<uint32_t*>(&v[u]);
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) {
+                                    const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[k]));
+                                    w[k] = pack2<false>(fminf(fmaxf(f.x, -65504.f), 65504.f), fminf(fmaxf(f.y, -65504.f), 65504.f));
+                                }
+                                tile[i + 64 * u] = v[u];
                             }
-                            tile[i] = v;
                         }
                         fence_proxy_async_smem();
                         mbar_arrive(BAR(Q_CONV + X));
@@ -727,7 +751,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 if (ok) load_q(1);
                 if constexpr (!kDequant) {
                     // gathered mode: the sequence's keys start at row kv_row0 of the scratch, which is one [1, Hkv, rows, 128] tensor
-                    const int kv_row0 = kGathered ? p.kv_base[seq] + it.kv_tile0 * kBN : 0;
+                    const int kv_row0 = kGathered ? kv_row_base + it.kv_tile0 * kBN : 0;
                     for (int j = 0; ok && j < it.nmax; ++j, ++g) {
                         const int st = g & 1, n = g >> 1;
                         if (n > 0 && !mbar_wait(BAR(K_EMPTY + st), (n - 1) & 1, abort_flag)) { ok = false; break; }
@@ -1104,17 +1128,20 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 }
                 const int row0 = X ? item.row0B : item.row0A, head = X ? item.headB : item.headA, b = item.b;
                 if constexpr (kPaged) {
-                    // row-wise stores: rows past the sequence's end belong to other sequences and are dropped
-                    const bool valid = row0 + r < nrows_total;
-                    uint4* orow = reinterpret_cast<uint4*>(
-                        reinterpret_cast<uint16_t*>(p.out) +
-                        (static_cast<size_t>(tok_base + row0 + r) * p.Hq + head) * kHeadDim);
+                    // Rows past the sequence's end belong to other sequences and are dropped.  A thread owns a row, so
+                    // storing from the registers would scatter every instruction over 32 lines; the warp's slab turns it
+                    // round: four whole 128-byte pieces of rows per instruction.
+                    uint8_t* slab = gbase + 6 * kTile + warp * 4096;
+                    const int wrow = 32 * (warp & 3), left = nrows_total - row0 - wrow;
+                    uint16_t* orow = reinterpret_cast<uint16_t*>(p.out) +
+                                     (static_cast<size_t>(tok_base + row0 + wrow) * p.Hq + head) * kHeadDim;
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        uint32_t o[32];
-                        tmem_ld32(tO + 32 * q, o);
-                        tmem_wait_ld();
-                        if (valid) {
+                    for (int half = 0; half < 2; ++half) {
+#pragma unroll
+                        for (int qq = 0; qq < 2; ++qq) {
+                            uint32_t o[32];
+                            tmem_ld32(tO + 32 * (2 * half + qq), o);
+                            tmem_wait_ld();
 #pragma unroll
                             for (int ch = 0; ch < 4; ++ch) {
                                 uint4 v;
@@ -1122,9 +1149,18 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                                 v.y = pack2<kBf16>(__uint_as_float(o[8 * ch + 2]) * inv, __uint_as_float(o[8 * ch + 3]) * inv);
                                 v.z = pack2<kBf16>(__uint_as_float(o[8 * ch + 4]) * inv, __uint_as_float(o[8 * ch + 5]) * inv);
                                 v.w = pack2<kBf16>(__uint_as_float(o[8 * ch + 6]) * inv, __uint_as_float(o[8 * ch + 7]) * inv);
-                                orow[q * 4 + ch] = v;
+                                *reinterpret_cast<uint4*>(slab + lane * 128 + (((qq * 4 + ch) ^ (lane & 7)) << 4)) = v;
                             }
                         }
+                        __syncwarp();
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const int row = 4 * i + (lane >> 3), ch = lane & 7;
+                            const uint4 v = *reinterpret_cast<const uint4*>(slab + row * 128 + ((ch ^ (row & 7)) << 4));
+                            if (row < left)
+                                reinterpret_cast<uint4*>(orow + static_cast<size_t>(row) * p.Hq * kHeadDim + 64 * half)[ch] = v;
+                        }
+                        __syncwarp();  // before the slab is written again
                     }
                 } else {
                     // passes of 64 columns through this warp's [32 rows x 128 bytes] staging slab
@@ -1428,7 +1464,7 @@ struct TcWorkspace {
 TcWorkspace tc_workspace(const b2a_paged_desc& d) {
     auto up = [](size_t x, size_t a) { return (x + a - 1) / a * a; };
     TcWorkspace w{};
-    size_t at = up(sizeof(int) * (kPlanHeaderInts + 2 * static_cast<size_t>(paged_tc_capacity(d))), 16);
+    size_t at = up(sizeof(int) * (kPlanHeaderInts + kPlanEntryInts * static_cast<size_t>(paged_tc_capacity(d))), 16);
     if (d.prefill_kv_tokens > 0) {
         w.rows = (d.prefill_kv_tokens + 127) / 128 * 128;
         w.groups = w.rows / 128;
@@ -1501,7 +1537,6 @@ int paged_tc_launch(const b2a_paged_desc& d, const void* query, const void* k_ca
     p.t = t;
     p.out = out;
     p.plan = static_cast<const int*>(plan_ws);
-    p.kv_base = kv_base;
     dim3 grid(capacity, d.Hkv, 1);
     TcPeers peers{};
     constexpr int kSmemPaged = smem_bytes(128 * kHeadDim * 2);

@@ -71,8 +71,27 @@ constexpr int kCacheChunk = 16 * (kHeadDim + 4);  // bytes of one (block, KV hea
 
 enum Bar { Q_FULL = 0, K_FULL = 2, K_EMPTY = 4, V_FULL = 6, V_EMPTY = 8, S_FULL = 10, P_READY = 12, O_DONE = 14, DRAIN = 16, P_HALF = 17, Q_CONV = 19, Q_EMPTY = 21 };
 
+// n / d for 0 <= n < 2^31 by one multiplication: mul = ceil(2^(31 + shift) / d) with shift = ceil(log2 d) errs by less than
+// n / 2^(31 + shift) < 1 / d (Granlund and Montgomery's division by an invariant).  A role works out its place from the
+// item's number at every item, and the run-time divisions took 1500 cycles of the issuing thread's.
+struct FastDiv {
+    uint32_t mul, shift, d;
+};
+FastDiv fast_div(int d) {
+    FastDiv f{0, 0, static_cast<uint32_t>(d)};
+    while ((1u << f.shift) < f.d) ++f.shift;
+    if (f.d > 1) f.mul = static_cast<uint32_t>(((1ull << (31 + f.shift)) + f.d - 1) / f.d);
+    return f;
+}
+__device__ __forceinline__ int div_by(int n, const FastDiv& f) {
+    return f.d == 1 ? n : static_cast<int>((static_cast<uint64_t>(static_cast<uint32_t>(n)) * f.mul) >> (31 + f.shift));
+}
+
 struct TcParams {
     int B, Hq, Hkv, G, Sq, Skv;
+    FastDiv div_g, div_hkv, div_streams;  // by G, Hkv, B * Hkv
+    int64_t out_strides[3];  // dense output: batch, head, row, in elements
+    int out_wide;            // every output row starts on a 32-byte boundary
     int causal;
     int window;  // paged modes: a query at position p sees keys p - window + 1 .. p (0: all of them)
     float scale_log2;
@@ -90,7 +109,7 @@ struct TcParams {
     const int* plan;  // work list built by paged_tc_plan_kernel: header, then entries of kPlanEntryInts
 };
 
-// Output side of a head-sharded launch (world == 0: single GPU, the tmO map is the output).
+// Output side of a head-sharded launch (world == 0: single GPU, TcParams::out is the output).
 struct TcPeers {
     CUtensorMap out_map[kMaxShardWorld];  // [rank]: that rank's [B, Hq_total, Sq, 128] output buffer
     int32_t* flags[kMaxShardWorld];
@@ -286,6 +305,19 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
         return *reinterpret_cast<const uint32_t*>(&v);
     }
 }
+// 64 bytes of an output row, in 32-byte stores where the row starts on such a boundary (else 16)
+__device__ __forceinline__ void store_64_bytes(uint16_t* dst, const uint32_t (&w)[16], bool wide) {
+    if (wide) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + 16 * h), "r"(w[8 * h]), "r"(w[8 * h + 1]),
+                         "r"(w[8 * h + 2]), "r"(w[8 * h + 3]), "r"(w[8 * h + 4]), "r"(w[8 * h + 5]), "r"(w[8 * h + 6]), "r"(w[8 * h + 7])
+                         : "memory");
+    } else {
+#pragma unroll
+        for (int h = 0; h < 4; ++h) reinterpret_cast<uint4*>(dst)[h] = make_uint4(w[4 * h], w[4 * h + 1], w[4 * h + 2], w[4 * h + 3]);
+    }
+}
 template <bool kBf16>
 __device__ __forceinline__ void unpack2(uint32_t w, float& lo, float& hi) {
     if constexpr (kBf16) {
@@ -410,8 +442,7 @@ __global__ void __launch_bounds__(128) paged_gather_kernel(const PagedTables t, 
 template <bool kBf16, int kMode, int kMask = 0, int kDim = kHeadDim, bool kSplitP = false>
 __global__ void __launch_bounds__(kMode == 1 ? kThreadsPaged : kThreadsDense, 1)
 attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-               const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, const TcParams p,
-               const __grid_constant__ TcPeers peers) {
+               const __grid_constant__ CUtensorMap tmV, const TcParams p, const __grid_constant__ TcPeers peers) {
     static_assert(kDim == kHeadDim || kMode == 0, "the paged modes are built for a head size of 128");
     constexpr int kTile = 128 * kDim * 2;  // bytes of a [128 x kDim] 16-bit tile: kDim / 64 panels
     extern __shared__ uint8_t smem_raw[];
@@ -428,9 +459,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     constexpr bool kKvBf16 = kPaged ? false : kBf16;  // element format of the K/V tiles and of P
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // A kernel launched programmatically dependent on this one (the decode kernel of a mixed step) may take the SMs
-    // this grid leaves free as soon as every CTA is seated.
-    grid_launch_dependents();
+    if constexpr (kDequant) {  // the grid is only a bound on the number of items: CTAs without one set nothing up
+        grid_dependency_wait();
+        if (static_cast<int>(blockIdx.x * gridDim.y + blockIdx.y) >= p.plan[0] * p.Hkv) return;
+    }
 
     // ---- work items.  An item is a pair of tiles of one KV head.  Rows are numbered inside the sequence (paged) or
     // the tensor (dense); `pos_base` is the key position the first row of the problem may see up to, `kv_limit` the
@@ -448,23 +480,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     bool causal = true;
     int nrb = 0, tiles = 0, pairs = 0, total_items = 0;
     int active_ctas = static_cast<int>(gridDim.x);  // CTAs that take items
-    if constexpr (kPaged) {
-        total_items = p.plan[0] * p.Hkv;  // the grid is only a bound on the number of items
-        if (kDequant && static_cast<int>(blockIdx.x * gridDim.y + blockIdx.y) >= total_items) return;
-        if constexpr (kGathered) {
-            // the plan kernel decides how many CTAs the prefill rows keep; the others give their SM to the decode rows
-            active_ctas = min(max(p.plan[1], 1), static_cast<int>(gridDim.x));
-            if (static_cast<int>(blockIdx.x) >= active_ctas) return;
-        }
-    } else {
-        nrows_total = p.Sq;
-        kv_limit = p.Skv;
-        causal = p.causal != 0;
-        nrb = (nrows_total + kBM - 1) / kBM;
-        tiles = nrb * p.G;
-        pairs = (tiles + 1) / 2;
-        total_items = pairs * p.B * p.Hkv;  // the launcher keeps this below 2^31
-    }
     auto get_item = [&](int k, Item& it) -> bool {  // the k-th item of this CTA
         int pair;
         if constexpr (kPaged) {
@@ -477,7 +492,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 idx = k * ctas + ((k & 1) ? ctas - 1 - me : me);
             }
             if (idx >= total_items) return false;
-            const int e = idx / p.Hkv;
+            const int e = div_by(idx, p.div_hkv);
             it.b = 0;
             it.hk = idx - e * p.Hkv;
             const int4* rec = reinterpret_cast<const int4*>(p.plan + kPlanHeaderInts) + 2 * e;
@@ -517,15 +532,15 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             // heaviest row blocks of ALL (batch, KV head) streams first (measured faster than walking one stream
             // after the other, although that keeps fewer K/V streams in flight)
             const int bh = p.B * p.Hkv;
-            pair = pairs - 1 - idx / bh;
-            const int y = idx % bh;
-            it.b = y / p.Hkv;
-            it.hk = y % p.Hkv;
+            const int round = div_by(idx, p.div_streams), y = idx - round * bh;
+            pair = pairs - 1 - round;
+            it.b = div_by(y, p.div_hkv);
+            it.hk = y - it.b * p.Hkv;
         }
         // a tile's rows, its head, the end of its keys (in tiles) and the first key tile any of its rows still sees
         auto tile_of = [&](int t, int& row0, int& head, int& nkv, int& first) {
             const bool present = t < tiles;
-            const int rb = present ? t / p.G : 0, g = present ? t % p.G : 0;
+            const int rb = present ? div_by(t, p.div_g) : 0, g = present ? t - rb * p.G : 0;
             row0 = rb * kBM;
             head = it.hk * p.G + g;
             const int kv_end = causal ? min(kv_limit, pos_base + row0 + kBM) : kv_limit;
@@ -574,6 +589,28 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+
+    // Launched programmatically dependent: what is above overlaps the kernel before this one, everything that touches
+    // memory comes after it.  Then a kernel that depends on this one (the decode kernel of a mixed step) may take the SMs
+    // that this grid leaves free.
+    grid_dependency_wait();
+    grid_launch_dependents();
+    if constexpr (kPaged) {
+        total_items = p.plan[0] * p.Hkv;  // the grid is only a bound on the number of items
+        if constexpr (kGathered) {
+            // the plan kernel decides how many CTAs the prefill rows keep; the others give their SM to the decode rows
+            active_ctas = min(max(p.plan[1], 1), static_cast<int>(gridDim.x));
+            if (static_cast<int>(blockIdx.x) >= active_ctas) total_items = 0;
+        }
+    } else {
+        nrows_total = p.Sq;
+        kv_limit = p.Skv;
+        causal = p.causal != 0;
+        nrb = (nrows_total + kBM - 1) / kBM;
+        tiles = nrb * p.G;
+        pairs = (tiles + 1) / 2;
+        total_items = pairs * p.B * p.Hkv;  // the launcher keeps this below 2^31
+    }
 
     // Registers follow the work: the service warpgroup keeps 56 per thread, the softmax groups take what is left
     // (dense: 2*128*224 + 128*56 = 384*168; paged: 2*128*168 + 128*56 + 128*112 <= 512*128).
@@ -1028,16 +1065,27 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                     }
                 }
                 if (kMask != 3 && kMask != 4 && (j >= jb || (kPaged && key0 < low_limit))) {
+                    // the row keeps the tile's keys [low, lim): one comparison with a constant per key, and only in the
+                    // groups of 32 that some row of the warp does not keep whole (the diagonal crosses one of four)
                     const int row_pos = row_pos0 + r;  // last key position this row may see (causal)
-                    const int row_low = window > 0 ? row_pos - window + 1 : 0;  // and the first
+                    const int lim = (causal ? min(kv_limit, row_pos + 1) : kv_limit) - key0;
 #pragma unroll
                     for (int q = 0; q < 4; ++q)
+                        if (__any_sync(0xffffffffu, lim < 32 * q + 32)) {
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            const int key = key0 + q * 32 + i;
-                            const bool keep = key < kv_limit && (!causal || key <= row_pos) && (!kPaged || key >= row_low);
-                            if (!keep) s[q][i] = 0xff800000u;  // -inf
+                            for (int i = 0; i < 32; ++i)
+                                if (32 * q + i >= lim) s[q][i] = 0xff800000u;  // -inf
                         }
+                    if (kPaged && key0 < low_limit) {
+                        const int low = row_pos - window + 1 - key0;
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            if (__any_sync(0xffffffffu, low > 32 * q)) {
+#pragma unroll
+                                for (int i = 0; i < 32; ++i)
+                                    if (32 * q + i < low) s[q][i] = 0xff800000u;
+                            }
+                    }
                 }
                 // row maximum: four independent chains of 3-input max (a single chain of 128 would be latency-bound)
                 float mq[4];
@@ -1127,40 +1175,24 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                     get_item(k_again, item);
                 }
                 const int row0 = X ? item.row0B : item.row0A, head = X ? item.headB : item.headA, b = item.b;
-                if constexpr (kPaged) {
-                    // Rows past the sequence's end belong to other sequences and are dropped.  A thread owns a row, so
-                    // storing from the registers would scatter every instruction over 32 lines; the warp's slab turns it
-                    // round: four whole 128-byte pieces of rows per instruction.
-                    uint8_t* slab = gbase + 6 * kTile + warp * 4096;
-                    const int wrow = 32 * (warp & 3), left = nrows_total - row0 - wrow;
-                    uint16_t* orow = reinterpret_cast<uint16_t*>(p.out) +
-                                     (static_cast<size_t>(tok_base + row0 + wrow) * p.Hq + head) * kHeadDim;
+                if (kPaged || peers.world == 0) {
+                    // A thread's row straight from its registers, whole 32-byte sectors: nothing to wait for, and the
+                    // warp goes on to the next item while the stores drain.  (Through the slab and TMA stores, the second
+                    // half waited for the first to be read, behind the next item's loads in the TMA unit's queue: 5000
+                    // cycles an item, longer than a key step.)  Rows past the end belong to nobody, or to another sequence.
+                    uint16_t* orow = static_cast<uint16_t*>(p.out);
+                    if constexpr (kPaged) orow += (static_cast<int64_t>(tok_base + row0 + r) * p.Hq + head) * kDim;
+                    else orow += b * p.out_strides[0] + head * p.out_strides[1] + (row0 + r) * p.out_strides[2];
+                    const bool valid = row0 + r < nrows_total;
 #pragma unroll
-                    for (int half = 0; half < 2; ++half) {
+                    for (int q = 0; q < kDim / 32; ++q) {
+                        uint32_t o[32], w[16];
+                        tmem_ld32(tO + 32 * q, o);
+                        tmem_wait_ld();
 #pragma unroll
-                        for (int qq = 0; qq < 2; ++qq) {
-                            uint32_t o[32];
-                            tmem_ld32(tO + 32 * (2 * half + qq), o);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int ch = 0; ch < 4; ++ch) {
-                                uint4 v;
-                                v.x = pack2<kBf16>(__uint_as_float(o[8 * ch + 0]) * inv, __uint_as_float(o[8 * ch + 1]) * inv);
-                                v.y = pack2<kBf16>(__uint_as_float(o[8 * ch + 2]) * inv, __uint_as_float(o[8 * ch + 3]) * inv);
-                                v.z = pack2<kBf16>(__uint_as_float(o[8 * ch + 4]) * inv, __uint_as_float(o[8 * ch + 5]) * inv);
-                                v.w = pack2<kBf16>(__uint_as_float(o[8 * ch + 6]) * inv, __uint_as_float(o[8 * ch + 7]) * inv);
-                                *reinterpret_cast<uint4*>(slab + lane * 128 + (((qq * 4 + ch) ^ (lane & 7)) << 4)) = v;
-                            }
-                        }
-                        __syncwarp();
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            const int row = 4 * i + (lane >> 3), ch = lane & 7;
-                            const uint4 v = *reinterpret_cast<const uint4*>(slab + row * 128 + ((ch ^ (row & 7)) << 4));
-                            if (row < left)
-                                reinterpret_cast<uint4*>(orow + static_cast<size_t>(row) * p.Hq * kHeadDim + 64 * half)[ch] = v;
-                        }
-                        __syncwarp();  // before the slab is written again
+                        for (int i = 0; i < 16; ++i)
+                            w[i] = pack2<kBf16>(__uint_as_float(o[2 * i]) * inv, __uint_as_float(o[2 * i + 1]) * inv);
+                        if (valid) store_64_bytes(orow + 32 * q, w, p.out_wide != 0);
                     }
                 } else {
                     // passes of 64 columns through this warp's [32 rows x 128 bytes] staging slab
@@ -1190,10 +1222,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                         fence_proxy_async_smem();
                         __syncwarp();
                         if (lane == 0) {
-                            if (peers.world == 0) {
-                                tma_store_4d_hint(&tmO, slab, 64 * half, row0 + 32 * (warp & 3), head, b, l2_evict_first_policy());
-                            } else {
-                                // the same slab into every rank's buffer, the next rank first so that the ranks do
+                            {
+                                // the slab into every rank's buffer, the next rank first so that the ranks do
                                 // not all write to the same peer at the same time; local copy last
                                 for (int i = 1; i <= peers.world; ++i) {
                                     const int dst = (peers.rank + i) % peers.world;
@@ -1296,14 +1326,13 @@ bool make_map(CUtensorMap* map, const void* ptr, bool bf16, int B, int H, int S,
 
 template <int kMask, int kDim, bool kSplitP>
 int launch_dense(bool bf16, dim3 grid, cudaStream_t stream, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
-                 const CUtensorMap& mo, const TcParams& p, const TcPeers& peers) {
+                 const TcParams& p, const TcPeers& peers) {
     constexpr int smem = smem_bytes(128 * kDim * 2);
     static bool configured[2][64] = {};
     auto kern = bf16 ? attn_tc_kernel<true, 0, kMask, kDim, kSplitP> : attn_tc_kernel<false, 0, kMask, kDim, kSplitP>;
     const int rc = configure_once(kern, configured[bf16], smem);
     if (rc != B2A_OK) return rc;
-    kern<<<grid, kThreadsDense, smem, stream>>>(mq, mk, mv, mo, p, peers);
-    return cudaGetLastError() == cudaSuccess ? B2A_OK : B2A_ERR_CUDA;
+    return launch_overlapped(kern, grid, dim3(kThreadsDense), smem, stream, mq, mk, mv, p, peers) == cudaSuccess ? B2A_OK : B2A_ERR_CUDA;
 }
 
 bool strides_ok(const int64_t (&st)[4], int B, int H, int S) {
@@ -1367,15 +1396,12 @@ int sdpa_tc_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t
                    const int64_t (&os)[4], const void* q, const void* k, const void* v, void* o, int32_t* status,
                    cudaStream_t stream, const TcPeerOut* peer_out, const void* mask, bool split_p) {
     const bool bf16 = d.dtype == B2A_BF16;
-    CUtensorMap mq, mk, mv, mo;
+    CUtensorMap mq, mk, mv;
     if (!make_map(&mq, q, bf16, d.B, d.Hq, d.Sq, qs, 128, d.D) || !make_map(&mk, k, bf16, d.B, d.Hkv, d.Skv, ks, 128, d.D) ||
         !make_map(&mv, v, bf16, d.B, d.Hkv, d.Skv, vs, 128, d.D))
         return B2A_ERR_CUDA;
     TcPeers peers{};
-    if (peer_out == nullptr) {
-        if (!make_map(&mo, o, bf16, d.B, d.Hq, d.Sq, os, 32, d.D)) return B2A_ERR_CUDA;
-    } else {
-        mo = mq;  // not read
+    if (peer_out != nullptr) {
         const int64_t fs[4] = {static_cast<int64_t>(peer_out->hq_total) * d.Sq * kHeadDim,
                                static_cast<int64_t>(d.Sq) * kHeadDim, kHeadDim, 1};
         for (int r = 0; r < peer_out->world; ++r) {
@@ -1392,6 +1418,16 @@ int sdpa_tc_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t
     }
     TcParams p{};
     p.B = d.B; p.Hq = d.Hq; p.Hkv = d.Hkv; p.G = d.Hq / d.Hkv; p.Sq = d.Sq; p.Skv = d.Skv;
+    p.div_g = fast_div(p.G);
+    p.div_hkv = fast_div(p.Hkv);
+    p.div_streams = fast_div(p.B * p.Hkv);
+    p.out = o;
+    const int extents[3] = {d.B, d.Hq, d.Sq};
+    p.out_wide = (reinterpret_cast<uintptr_t>(o) & 31) == 0;
+    for (int i = 0; i < 3; ++i) {
+        p.out_strides[i] = os[i];
+        if (extents[i] > 1 && os[i] % 16 != 0) p.out_wide = 0;
+    }
     p.causal = d.causal;
     p.scale_log2 = d.scale * kLog2e;
     p.status = status;
@@ -1415,18 +1451,18 @@ int sdpa_tc_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t
                          : mask_kind == B2A_MASK_BOOL                  ? 3
                                                                        : 4;
         if (d.D == 64) {
-            if (form == 0) return launch_dense<0, 64, true>(bf16, grid, stream, mq, mk, mv, mo, p, peers);
-            if (form == 3) return launch_dense<3, 64, true>(bf16, grid, stream, mq, mk, mv, mo, p, peers);
-            if (form == 4) return launch_dense<4, 64, true>(bf16, grid, stream, mq, mk, mv, mo, p, peers);
-            return launch_dense<5, 64, true>(bf16, grid, stream, mq, mk, mv, mo, p, peers);
+            if (form == 0) return launch_dense<0, 64, true>(bf16, grid, stream, mq, mk, mv, p, peers);
+            if (form == 3) return launch_dense<3, 64, true>(bf16, grid, stream, mq, mk, mv, p, peers);
+            if (form == 4) return launch_dense<4, 64, true>(bf16, grid, stream, mq, mk, mv, p, peers);
+            return launch_dense<5, 64, true>(bf16, grid, stream, mq, mk, mv, p, peers);
         }
-        if (form == 3) return launch_dense<3, kHeadDim, true>(bf16, grid, stream, mq, mk, mv, mo, p, peers);
-        if (form == 4) return launch_dense<4, kHeadDim, true>(bf16, grid, stream, mq, mk, mv, mo, p, peers);
-        if (form == 5) return launch_dense<5, kHeadDim, true>(bf16, grid, stream, mq, mk, mv, mo, p, peers);
+        if (form == 3) return launch_dense<3, kHeadDim, true>(bf16, grid, stream, mq, mk, mv, p, peers);
+        if (form == 4) return launch_dense<4, kHeadDim, true>(bf16, grid, stream, mq, mk, mv, p, peers);
+        if (form == 5) return launch_dense<5, kHeadDim, true>(bf16, grid, stream, mq, mk, mv, p, peers);
     }
-    if (mask_kind == B2A_MASK_BOOL) return launch_dense<1, kHeadDim, false>(bf16, grid, stream, mq, mk, mv, mo, p, peers);
-    if (mask_kind == B2A_MASK_ADD) return launch_dense<2, kHeadDim, false>(bf16, grid, stream, mq, mk, mv, mo, p, peers);
-    return launch_dense<0, kHeadDim, false>(bf16, grid, stream, mq, mk, mv, mo, p, peers);
+    if (mask_kind == B2A_MASK_BOOL) return launch_dense<1, kHeadDim, false>(bf16, grid, stream, mq, mk, mv, p, peers);
+    if (mask_kind == B2A_MASK_ADD) return launch_dense<2, kHeadDim, false>(bf16, grid, stream, mq, mk, mv, p, peers);
+    return launch_dense<0, kHeadDim, false>(bf16, grid, stream, mq, mk, mv, p, peers);
 }
 
 int sdpa_peer_wait_launch(const int32_t* local_flags, int world, int32_t step, long long wait_ns, int32_t* status,
@@ -1528,6 +1564,9 @@ int paged_tc_launch(const b2a_paged_desc& d, const void* query, const void* k_ca
     }
     TcParams p{};
     p.B = 1; p.Hq = d.Hq; p.Hkv = d.Hkv; p.G = d.Hq / d.Hkv; p.Sq = 0; p.Skv = 0;
+    p.div_g = fast_div(p.G);
+    p.div_hkv = p.div_streams = fast_div(p.Hkv);
+    p.out_wide = (reinterpret_cast<uintptr_t>(out) & 31) == 0;
     p.causal = 1;
     p.window = d.sliding_window;
     p.scale_log2 = d.scale * kLog2e;
@@ -1546,15 +1585,16 @@ int paged_tc_launch(const b2a_paged_desc& d, const void* query, const void* k_ca
         auto kern = bf16 ? attn_tc_kernel<true, 2> : attn_tc_kernel<false, 2>;
         const int rc = configure_once(kern, configured[bf16], kSmemPaged);
         if (rc != B2A_OK) return rc;
-        kern<<<grid, kThreadsDense, kSmemPaged, stream>>>(mq, mk, mv, mq, p, peers);
+        if (launch_overlapped(kern, grid, dim3(kThreadsDense), kSmemPaged, stream, mq, mk, mv, p, peers) != cudaSuccess) return B2A_ERR_CUDA;
     } else {
         static bool configured[2][64] = {};
         auto kern = bf16 ? attn_tc_kernel<true, 1> : attn_tc_kernel<false, 1>;
         const int rc = configure_once(kern, configured[bf16], kSmemPaged);
         if (rc != B2A_OK) return rc;
-        kern<<<grid, kThreadsPaged, kSmemPaged, stream>>>(mq, mq, mq, mq, p, peers);  // only the Q map is read
+        // (only the Q map is read)
+        if (launch_overlapped(kern, grid, dim3(kThreadsPaged), kSmemPaged, stream, mq, mq, mq, p, peers) != cudaSuccess) return B2A_ERR_CUDA;
     }
-    return cudaGetLastError() == cudaSuccess ? B2A_OK : B2A_ERR_CUDA;
+    return B2A_OK;
 }
 
 }  // namespace b2a

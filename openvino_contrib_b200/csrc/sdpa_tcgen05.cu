@@ -318,6 +318,12 @@ __device__ __forceinline__ void store_64_bytes(uint16_t* dst, const uint32_t (&w
         for (int h = 0; h < 4; ++h) reinterpret_cast<uint4*>(dst)[h] = make_uint4(w[4 * h], w[4 * h + 1], w[4 * h + 2], w[4 * h + 3]);
     }
 }
+// two values rounded to f16, magnitudes beyond its range to the largest finite one
+__device__ __forceinline__ uint32_t pack_f16_finite(float lo, float hi) {
+    uint32_t d;
+    asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+    return d;
+}
 template <bool kBf16>
 __device__ __forceinline__ void unpack2(uint32_t w, float& lo, float& hi) {
     if constexpr (kBf16) {
@@ -644,7 +650,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 #pragma unroll
                                 for (int k = 0; k < 4; ++k) {
                                     const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[k]));
-                                    w[k] = pack2<false>(fminf(fmaxf(f.x, -65504.f), 65504.f), fminf(fmaxf(f.y, -65504.f), 65504.f));
+                                    w[k] = pack_f16_finite(f.x, f.y);
                                 }
                                 tile[i] = v;
                             }
@@ -747,7 +753,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 #pragma unroll
                                 for (int k = 0; k < 4; ++k) {
                                     const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[k]));
-                                    w[k] = pack2<false>(fminf(fmaxf(f.x, -65504.f), 65504.f), fminf(fmaxf(f.y, -65504.f), 65504.f));
+                                    w[k] = pack_f16_finite(f.x, f.y);
                                 }
                                 tile[i + 64 * u] = v[u];
                             }
@@ -784,8 +790,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                         tma_load_4d_hint(sQ + X * kTile + kPanel, &tmQ, BAR(Q_FULL + X), 64, row, head, it.b, once_policy);
                     ++qn[X];
                 };
-                load_q(0);
-                if (ok) load_q(1);
+                if constexpr (kDequant) {
+                    load_q(0);
+                    if (ok) load_q(1);
+                }
                 if constexpr (!kDequant) {
                     // gathered mode: the sequence's keys start at row kv_row0 of the scratch, which is one [1, Hkv, rows, 128] tensor
                     const int kv_row0 = kGathered ? kv_row_base + it.kv_tile0 * kBN : 0;
@@ -797,6 +805,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                         if constexpr (kDim > 64)
                             tma_load_4d(sK + st * kTile + kPanel, &tmK, BAR(K_FULL + st), 64, kv_row0 + j * kBN, it.hk, it.b);
                         ++issued_k;
+                        if (j == 0) {  // (the first K tile has room before the previous item's last QK^T gives up the Q tiles)
+                            load_q(0);
+                            if (ok) load_q(1);
+                            if (!ok) break;
+                        }
                         if (n > 0 && !mbar_wait(BAR(V_EMPTY + st), (n - 1) & 1, abort_flag)) { ok = false; break; }
                         mbar_expect_tx(BAR(V_FULL + st), kTile);
                         tma_load_4d(sV + st * kTile, &tmV, BAR(V_FULL + st), 0, kv_row0 + j * kBN, it.hk, it.b);
@@ -856,17 +869,19 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             for (int k = 0; ok && get_item(k, it); ++k) {
                 const int nkvA = it.nkvA, nkvB = it.nkvB, nmax = it.nmax;
                 if (nmax == 0) continue;  // an item that was refused (inconsistent tables)
-                if (nkvA > 0) ok = ok && mbar_wait(BAR(kQReady + 0), qn[0] & 1, abort_flag);
-                if (nkvB > 0) ok = ok && mbar_wait(BAR(kQReady + 1), qn[1] & 1, abort_flag);
                 ok = ok && mbar_wait(BAR(K_FULL + (g0 & 1)), (g0 >> 1) & 1, abort_flag);
+                if (nkvA > 0) ok = ok && mbar_wait(BAR(kQReady + 0), qn[0] & 1, abort_flag);
                 if (!ok) break;
                 tc_fence_after();
-                if (nkvA > 0) {
+                if (nkvA > 0) {  // (tile A starts as soon as its own operands are there)
                     issue_qk(0, g0 & 1);
                     mma_commit(BAR(S_FULL + 0));
                     if (nkvA == 1) mma_commit(BAR(Q_EMPTY + 0));  // last use of this Q tile: the producer may refill it
                 }
                 if (nkvB > 0) {
+                    ok = mbar_wait(BAR(kQReady + 1), qn[1] & 1, abort_flag);
+                    if (!ok) break;
+                    tc_fence_after();
                     issue_qk(1, g0 & 1);
                     mma_commit(BAR(S_FULL + 1));
                     if (nkvB == 1) mma_commit(BAR(Q_EMPTY + 1));

@@ -29,7 +29,10 @@ def _dtype_code(t: torch.dtype) -> int:
 
 
 def _stream_ptr(stream: Optional[torch.cuda.Stream]) -> int:
-    return (stream or torch.cuda.current_stream()).cuda_stream
+    if stream is not None:
+        return stream.cuda_stream
+    # the handle torch.cuda.current_stream() would wrap, without building the wrapper (4 us a call)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _require_cuda(*ts: torch.Tensor) -> None:
@@ -88,17 +91,9 @@ def sdpa(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, attn_mask: Optional[
     if o4.stride(-1) != 1:
         raise ValueError("the output needs a unit innermost stride")
 
-    d = SdpaDesc()
-    d.dtype = _dtype_code(q.dtype)
-    d.B, d.Hq, d.Hkv, d.Sq, d.Skv, d.D, d.Dv = B, Hq, Hkv, Sq, Skv, D, Dv
-    d.causal = int(bool(causal))
-    d.scale = 0.0 if scale is None else float(scale)
-    d.q_strides[:] = q4.stride()
-    d.k_strides[:] = k4.stride()
-    d.v_strides[:] = v4.stride()
-    d.o_strides[:] = o4.stride()
+    d = SdpaDesc(_dtype_code(q.dtype), B, Hq, Hkv, Sq, Skv, D, Dv, int(bool(causal)), 0.0 if scale is None else float(scale),
+                 q4.stride(), k4.stride(), v4.stride(), o4.stride(), _lib.MASK_NONE)
     mask_t = None
-    d.mask_kind = _lib.MASK_NONE
     if attn_mask is not None and not causal:
         m = attn_mask
         if m.dtype == torch.bool:
@@ -114,13 +109,9 @@ def sdpa(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, attn_mask: Optional[
         m = m.expand(B, Hq, Sq, Skv)  # broadcast dimensions get stride 0
         d.mask_strides[:] = m.stride()
         mask_t = m
-    lib = _lib.load()
-    ws = C.c_size_t(0)
-    check(lib.b2a_sdpa_workspace_bytes(C.byref(d), sm_count(), C.byref(ws)), "b2a_sdpa_workspace_bytes")
-    wbuf = torch.empty(ws.value, dtype=torch.uint8, device=q.device) if ws.value else None
-    check(lib.b2a_sdpa_forward(C.byref(d), q4.data_ptr(), k4.data_ptr(), v4.data_ptr(), _ptr(mask_t),
-                               o4.data_ptr(), _ptr(wbuf), ws.value, _ptr(status), _stream_ptr(stream)),
-          "b2a_sdpa_forward")
+    # (no workspace: b2a_sdpa_workspace_bytes is 0 for every kernel)
+    check(_lib.load().b2a_sdpa_forward(C.byref(d), q4.data_ptr(), k4.data_ptr(), v4.data_ptr(), _ptr(mask_t),
+                                       o4.data_ptr(), None, 0, _ptr(status), _stream_ptr(stream)), "b2a_sdpa_forward")
     return out
 
 
@@ -241,18 +232,9 @@ class PagedKvCache:
 def _paged_desc(q_dtype, cache: PagedKvCache, hq: int, num_seqs: int, num_tokens: int, max_context_len: int,
                 max_q_len: int, scale: Optional[float], sliding_window: int, prefill_row_blocks: int = 0,
                 prefill_kv_tokens: int = 0, cache_rows_settled: bool = False) -> PagedDesc:
-    d = PagedDesc()
-    d.q_dtype = _dtype_code(q_dtype)
-    d.kv_dtype = _dtype_code(cache.kv_dtype)
-    d.Hq, d.Hkv, d.D, d.Dv, d.block_size = hq, cache.hkv, cache.d, cache.dv, cache.block_size
-    d.num_seqs, d.num_tokens, d.num_blocks_total = num_seqs, num_tokens, cache.num_blocks
-    d.max_context_len, d.max_q_len = max_context_len, max_q_len
-    d.scale = 0.0 if scale is None else float(scale)
-    d.sliding_window = int(sliding_window)
-    d.prefill_row_blocks = int(prefill_row_blocks)
-    d.prefill_kv_tokens = int(prefill_kv_tokens)
-    d.cache_rows_settled = 1 if cache_rows_settled else 0
-    return d
+    return PagedDesc(_dtype_code(q_dtype), _dtype_code(cache.kv_dtype), hq, cache.hkv, cache.d, cache.dv, cache.block_size,
+                     num_seqs, num_tokens, cache.num_blocks, max_context_len, max_q_len, 0.0 if scale is None else float(scale),
+                     int(sliding_window), int(prefill_row_blocks), int(prefill_kv_tokens), 1 if cache_rows_settled else 0)
 
 
 def _i32(t: torch.Tensor) -> torch.Tensor:
@@ -484,25 +466,40 @@ class PagedAttentionOp:
         if ws is None or ws.numel() * ws.element_size() < self._workspace_bytes:
             raise B2AError(5, "PagedAttentionOp: pass the work buffer GetWorkBufferRequest() asked for")
         rb, kvt = self.step_hints(num_tokens, num_seqs, prefill_row_blocks, prefill_kv_tokens)
-        paged_kv_store(key, value, cache, past_lens, subsequence_begins, block_indices, block_indices_begins,
-                       stream=stream, status=status)
+        # What paged_kv_store and paged_attention check, once for both, and one descriptor: a small step is bound by this
+        # code, not by its kernels (two sequences: 28 us of host time before, 10 us of kernels).
+        _require_cuda(query, key, value, k_cache, v_cache, past_lens, subsequence_begins, block_indices, block_indices_begins,
+                      outputs[0])
+        if key.dtype != value.dtype or not key.is_contiguous() or not value.is_contiguous():
+            raise ValueError("key and value must be dense and share one element type")
+        width, key_tokens = self.hkv * self.d, key.shape[0]
+        if key.shape[1] != width or value.shape[1] != width or value.shape[0] != key_tokens:
+            raise ValueError("key/value row width does not match the cache geometry")
+        if not query.is_contiguous() or query.shape[1] != self.hq * self.d:
+            raise ValueError("query must be dense [tokens, Hq*D]")
+        lib, scale_value = _lib.load(), self.scale if sc is None else float(sc)
+        d = _paged_desc(key.dtype, cache, self.hq, num_seqs, key_tokens, self.max_context_len, max_q_len, scale_value,
+                        self.sliding_window, rb, kvt, True)  # (settled: the kernel before the attention is this step's store)
+        caches = (k_cache.data_ptr(), v_cache.data_ptr())
+        tables = (_i32(past_lens).data_ptr(), _i32(subsequence_begins).data_ptr(), _i32(block_indices).data_ptr(),
+                  _i32(block_indices_begins).data_ptr())
+        status_ptr, stream_ptr = _ptr(status), _stream_ptr(stream)
+        check(lib.b2a_paged_kv_store(C.byref(d), key.data_ptr(), value.data_ptr(), *caches, *tables, status_ptr, stream_ptr),
+              "b2a_paged_kv_store")
         if len(outputs) > 1 and outputs[1] is not None:
             done = paged_attention_scores(query, cache, past_lens, subsequence_begins, block_indices, block_indices_begins,
-                                          self.hq, self.max_context_len, self.scale if sc is None else float(sc),
+                                          self.hq, self.max_context_len, scale_value,
                                           self.sliding_window, out=outputs[0], scores=outputs[1], stream=stream,
                                           status=status, cache_rows_settled=True)
             if done is not None:
                 return done[2]
-        paged_attention(query, cache, past_lens, subsequence_begins, block_indices, block_indices_begins,
-                        self.hq, self.max_context_len, max_q_len, self.scale if sc is None else float(sc),
-                        self.sliding_window, out=outputs[0], workspace=ws, stream=stream,
-                        status=status, prefill_row_blocks=rb, prefill_kv_tokens=kvt,
-                        cache_rows_settled=True)  # the kernel before it is this step's store
+        d.q_dtype, d.num_tokens = _dtype_code(query.dtype), num_tokens
+        check(lib.b2a_paged_attention(C.byref(d), query.data_ptr(), *caches, *tables, outputs[0].data_ptr(), ws.data_ptr(),
+                                      ws.numel() * ws.element_size(), status_ptr, stream_ptr), "b2a_paged_attention")
         if len(outputs) > 1 and outputs[1] is not None:
             _, begins = paged_last_token_scores(query, cache, past_lens, subsequence_begins, block_indices,
-                                                block_indices_begins, self.hq, self.max_context_len,
-                                                self.scale if sc is None else float(sc), self.sliding_window,
-                                                scores=outputs[1], stream=stream, status=status)
+                                                block_indices_begins, self.hq, self.max_context_len, scale_value,
+                                                self.sliding_window, scores=outputs[1], stream=stream, status=status)
             return begins
         return None
 

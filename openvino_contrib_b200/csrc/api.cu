@@ -188,7 +188,7 @@ int b2a_paged_workspace_bytes(const b2a_paged_desc* desc, int sm_count, size_t* 
     // layout: [split-K partials of the decode kernel, rounded up to 16 bytes][work list of the prefill kernel]
     size_t bytes = 0;
     if (paged_decode_geometry_ok(d)) {
-        bytes = (paged_decode_plan(d, sm_count).workspace_bytes + 15) & ~static_cast<size_t>(15);
+        bytes = (paged_decode_plan(d, sm_count, d.max_q_len >= 2).workspace_bytes + 15) & ~static_cast<size_t>(15);
         if (d.max_q_len >= 2) bytes += paged_tc_plan_bytes(d);
     }
     *out_bytes = bytes;
@@ -258,7 +258,7 @@ int b2a_paged_attention(const b2a_paged_desc* desc, const void* query, const voi
         // mixed step: multi-token sequences on the tensor-core kernel, one-token sequences on the decode kernel
         const int sms = device_sm_count();
         if (sms <= 0) return B2A_ERR_CUDA;
-        const DecodePlan plan = paged_decode_plan(d, sms);
+        const DecodePlan plan = paged_decode_plan(d, sms, true);
         const size_t list_at = (plan.workspace_bytes + 15) & ~static_cast<size_t>(15);
         if (workspace == nullptr || workspace_bytes < list_at + paged_tc_plan_bytes(d)) return B2A_ERR_WORKSPACE;
         if (!aligned(workspace, 16)) return B2A_ERR_ALIGN;
@@ -308,7 +308,7 @@ int b2a_paged_attention_noalloc(const b2a_paged_desc* desc, const void* query, c
 static int decode_scores_layout(const b2a_paged_desc& d, int sm_count, int64_t table_blocks, size_t& raw_at, size_t& total) {
     if (!paged_decode_supported(d) || !paged_scores_supported(d)) return B2A_ERR_UNSUPPORTED;
     if (d.max_context_len <= 0 || table_blocks < 0 || table_blocks > INT32_MAX) return B2A_ERR_DIM;
-    raw_at = (paged_decode_plan(d, sm_count).workspace_bytes + 255) & ~static_cast<size_t>(255);
+    raw_at = (paged_decode_plan(d, sm_count, true).workspace_bytes + 255) & ~static_cast<size_t>(255);
     total = raw_at + static_cast<size_t>(table_blocks) * d.block_size * d.Hq * sizeof(float);
     return B2A_OK;
 }
@@ -348,7 +348,7 @@ int b2a_paged_attention_scores(const b2a_paged_desc* desc, const void* query, co
     if (!aligned(workspace, 16)) return B2A_ERR_ALIGN;
     const DecodeScores sc{reinterpret_cast<float*>(static_cast<char*>(workspace) + raw_at), static_cast<int>(table_blocks), scores,
                           scores_capacity, score_begins};
-    return paged_decode_launch(d, paged_decode_plan(d, sms), query, k_cache, v_cache,
+    return paged_decode_launch(d, paged_decode_plan(d, sms, true), query, k_cache, v_cache,
                                tables_of(d, past_lens, subsequence_begins, block_indices, block_indices_begins), out, workspace,
                                status, reinterpret_cast<cudaStream_t>(stream), nullptr, nullptr, &sc);
 }

@@ -79,7 +79,7 @@ struct DecodePlan {
 };
 bool paged_decode_supported(const b2a_paged_desc& d);   // a pure decode step
 bool paged_decode_geometry_ok(const b2a_paged_desc& d); // the kernel's shape limits, whatever the step's mix
-DecodePlan paged_decode_plan(const b2a_paged_desc& d, int sm_count);
+DecodePlan paged_decode_plan(const b2a_paged_desc& d, int sm_count, bool short_chunks = false);
 // beside_predecessor != nullptr: the kernel before this launch on the stream is the prefill kernel of the same mixed
 // step, which has already waited for everything the decode rows read (cache, tables, query) and writes nothing they
 // touch; the event was recorded right behind it.  The decode kernel then starts as soon as that kernel's CTAs are

@@ -1012,7 +1012,13 @@ bool paged_decode_supported(const b2a_paged_desc& d) {
     return paged_decode_geometry_ok(d) && d.max_q_len == 1 && d.num_tokens == d.num_seqs;
 }
 
-DecodePlan paged_decode_plan(const b2a_paged_desc& d, int sm_count) {
+// short_chunks: the decode rows of a mixed step, whose CTAs get their SMs one after the other, and a step with scores,
+// whose merge kernel works on the sequences' scores anyway.  A CTA of a full chunk of 128 blocks is half the step there;
+// with 128 / 96 / 64 / 48 / 32 blocks 120 decode sequences beside eight prompts take 229 / 219 / 221 / 223 / 231 us, 32
+// sequences of at most 4096 tokens with scores 55.3 / 53.2 / 49.2 / 51.2 / 53.2 us: 64.  (Pure decode steps gain less with
+// 64 uneven sequences, 122.8 / 118.8 / 116.8 / 116.8 / 120.8, and lose with long even ones: 199.5 -> 204.9 us for
+// 16 x 32768 tokens with 64 blocks.)
+DecodePlan paged_decode_plan(const b2a_paged_desc& d, int sm_count, bool short_chunks) {
     // Long chunks win (a CTA's pipeline start and its merge are paid once per chunk), so a CTA walks up to 128
     // blocks - 32 per warp, the size of a warp's block-id window.  Only when the whole step is smaller than one
     // wave of 4 CTAs per SM are the chunks shortened, so that every SM still has work.
@@ -1030,6 +1036,7 @@ DecodePlan paged_decode_plan(const b2a_paged_desc& d, int sm_count) {
         const long long floor_bpc = ((nblk_max + 15) / 16 + 3) / 4 * 4;
         if (bpc < floor_bpc) bpc = floor_bpc;
     }
+    else if (short_chunks) bpc = 64;
     if (bpc < 16) bpc = 16;
     if (bpc > 128) bpc = 128;
     DecodePlan plan;

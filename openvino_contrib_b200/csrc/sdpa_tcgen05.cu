@@ -133,10 +133,10 @@ constexpr int kPlanEntryInts = 8;
 // those CTAs are seated, takes the rest (and the others as they come free).  The share is worked out here from the
 // tables: item-steps of the work list against cached bytes of the one-token sequences, each divided by what one SM
 // gets through per microsecond (measured on a step of eight 1024-token prefills beside 120 decode sequences: about
-// 3.4 us per item-step of two 128 x 128 tiles over 128 keys at the efficiency of short items; about 52 bytes per
+// 2.8 us per item-step of two 128 x 128 tiles over 128 keys at the efficiency of short items; about 52 bytes per
 // nanosecond of u8 cache per SM while the SMs that decode are a minority - a sweep of the share on that step was
 // flat within 5 % between 0.59 and 0.70 and best at 0.59).
-constexpr float kUsPerItemStep = 3.4f;
+constexpr float kUsPerItemStep = 2.8f;
 constexpr float kDecodeBytesPerNsPerSm = 52.f;
 constexpr float kHbmBytesPerNs = 6500.f;
 // With `owner` given the kernel also lays out the gathered K/V scratch: every multi-token sequence gets a row range

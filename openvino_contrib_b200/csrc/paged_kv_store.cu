@@ -70,6 +70,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) paged_kv_store_kernel(const
     const int lane = threadIdx.x & 31;
     const long long item = static_cast<long long>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5);
     const long long total = 2LL * p.t.num_tokens * p.Hkv;
+    grid_dependency_wait();  // the new key/value rows (and the pool's previous readers) belong to earlier kernels
+    grid_launch_dependents();
     if (item >= total) return;
     const int which = static_cast<int>(item % 2);  // 0 = key, 1 = value
     const int hk = static_cast<int>((item / 2) % p.Hkv);
@@ -369,13 +371,14 @@ int paged_kv_store_launch(const b2a_paged_desc& d, const void* key, const void* 
     }
     const long long total = 2LL * d.num_tokens * d.Hkv;
     const unsigned grid = static_cast<unsigned>((total + kWarpsPerCta - 1) / kWarpsPerCta);
+    void (*kern)(StoreParams) = nullptr;
     switch (d.q_dtype) {
-        case B2A_F32: paged_kv_store_kernel<float><<<grid, kWarpsPerCta * 32, 0, stream>>>(p); break;
-        case B2A_F16: paged_kv_store_kernel<__half><<<grid, kWarpsPerCta * 32, 0, stream>>>(p); break;
-        case B2A_BF16: paged_kv_store_kernel<__nv_bfloat16><<<grid, kWarpsPerCta * 32, 0, stream>>>(p); break;
+        case B2A_F32: kern = paged_kv_store_kernel<float>; break;
+        case B2A_F16: kern = paged_kv_store_kernel<__half>; break;
+        case B2A_BF16: kern = paged_kv_store_kernel<__nv_bfloat16>; break;
         default: return B2A_ERR_DTYPE;
     }
-    return cudaGetLastError() == cudaSuccess ? B2A_OK : B2A_ERR_CUDA;
+    return launch_overlapped(kern, dim3(grid), dim3(kWarpsPerCta * 32), 0, stream, p) == cudaSuccess ? B2A_OK : B2A_ERR_CUDA;
 }
 
 }  // namespace b2a

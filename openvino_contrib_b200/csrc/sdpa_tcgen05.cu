@@ -147,10 +147,14 @@ __global__ void __launch_bounds__(256) paged_tc_plan_kernel(const PagedTables t,
                                                             int* kv_base, int* owner, const int owner_groups,
                                                             const int attention_ctas, const int share_with_decode) {
     // The list is sorted by weight (key steps of the pair's later tile, clamped to 255), heaviest first: a counting
-    // sort in three passes over the sequences - histogram, bucket offsets, scatter.
+    // sort in three passes over the sequences - histogram, bucket offsets, scatter.  Sequences are looked at 256 at a time,
+    // a thread each, and the tile pairs of those with several new tokens are spread over the lanes of a warp.
     constexpr int kBuckets = 256;
     __shared__ int s_hist[kBuckets], s_count, s_groups, s_steps;
+    __shared__ int c_tok[256], c_qlen[256], c_past[256];
+    __shared__ unsigned char c_ok[256];
     __shared__ unsigned long long s_decode_blocks;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // Everything that only reads the step's tables - the histogram of the weights, the counts, the bucket offsets -
     // is done while the kernel in front (the step's store) drains; what this kernel WRITES (list, scratch layout)
     // may still be read by earlier kernels, so the writes come after the wait.  (The tables of a step exist before
@@ -160,34 +164,59 @@ __global__ void __launch_bounds__(256) paged_tc_plan_kernel(const PagedTables t,
         s_count = s_groups = s_steps = 0;
         s_decode_blocks = 0ull;
     }
-    __syncthreads();
     auto weight = [&](int past, int qlen, int pair) {
         const int tiles = ((qlen + 127) / 128) * G;
         const int tile = min(2 * pair + 1, tiles - 1);  // the pair's later tile
         const int keys = min(past + qlen, past + (tile / G) * 128 + 128);
         return min(kBuckets - 1, max(0, (keys + 127) / 128));
     };
-    for (int s = threadIdx.x; s < t.num_seqs; s += blockDim.x) {
-        const int qlen = t.subsequence_begins[s + 1] - t.subsequence_begins[s];
-        if (qlen == 1 && t.past_lens[s] >= 0)
-            atomicAdd(&s_decode_blocks, static_cast<unsigned long long>(t.past_lens[s] / t.block_size + 1));
-        if (qlen < 2) continue;
-        const int past = max(0, t.past_lens[s]);
-        const int pairs = (((qlen + 127) / 128) * G + 1) / 2;
-        atomicAdd(&s_count, pairs);
-        int steps = 0;
-        for (int i = 0; i < pairs; ++i) {
-            const int w = weight(past, qlen, i);
-            atomicAdd(&s_hist[w], 1);
-            steps += w;
+    auto pairs_of = [&](int qlen) { return (((qlen + 127) / 128) * G + 1) / 2; };
+    // this thread's sequence of the 256 from s0; returns the blocks of its context if it is a one-token sequence
+    auto load_chunk = [&](int s0) -> int {
+        const int s = s0 + threadIdx.x;
+        int tok0 = 0, qlen = 0, past = 0, ok = 0;
+        if (s < t.num_seqs) {
+            tok0 = t.subsequence_begins[s];
+            qlen = t.subsequence_begins[s + 1] - tok0;
+            past = t.past_lens[s];
+            const int have = t.block_indices_begins[s + 1] - t.block_indices_begins[s];
+            ok = past >= 0 && tok0 >= 0 && tok0 + qlen <= t.num_tokens && (past + qlen + 15) / 16 <= have;
         }
-        atomicAdd(&s_steps, steps);
+        c_tok[threadIdx.x] = tok0;
+        c_qlen[threadIdx.x] = qlen >= 2 ? qlen : 0;
+        c_past[threadIdx.x] = past;
+        c_ok[threadIdx.x] = static_cast<unsigned char>(ok);
+        return qlen == 1 && past >= 0 ? past / t.block_size + 1 : 0;
+    };
+    int steps = 0;
+    long long decode_blocks = 0;
+    for (int s0 = 0; s0 < t.num_seqs; s0 += 256) {
+        if (s0 > 0) __syncthreads();  // the chunk before has been read
+        decode_blocks += load_chunk(s0);
+        __syncthreads();
+        for (int i = warp; i < min(256, t.num_seqs - s0); i += 8) {
+            const int qlen = c_qlen[i];
+            if (qlen == 0) continue;
+            const int past = max(0, c_past[i]), pairs = pairs_of(qlen);
+            if (lane == 0) atomicAdd(&s_count, pairs);
+            for (int k = lane; k < pairs; k += 32) {
+                const int w = weight(past, qlen, k);
+                atomicAdd(&s_hist[w], 1);
+                steps += w;
+            }
+        }
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        steps += __shfl_xor_sync(0xffffffffu, steps, o);
+        decode_blocks += __shfl_xor_sync(0xffffffffu, decode_blocks, o);
+    }
+    if (lane == 0 && steps > 0) atomicAdd(&s_steps, steps);
+    if (lane == 0 && decode_blocks > 0) atomicAdd(&s_decode_blocks, static_cast<unsigned long long>(decode_blocks));
     __syncthreads();
     {  // bucket w starts after all heavier buckets: one bucket per thread, lightest in the last
         static_assert(kBuckets == 256, "a bucket per thread");
         __shared__ int s_warp[kBuckets / 32];
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         const int n = s_hist[kBuckets - 1 - threadIdx.x];
         int upto = n;
 #pragma unroll
@@ -202,39 +231,40 @@ __global__ void __launch_bounds__(256) paged_tc_plan_kernel(const PagedTables t,
     }
     grid_dependency_wait();
     grid_launch_dependents();
-    if (owner != nullptr) {
+    if (owner != nullptr)
         for (int g = threadIdx.x; g < owner_groups; g += blockDim.x) owner[g] = -1;
-        __syncthreads();
-        for (int s = threadIdx.x; s < t.num_seqs; s += blockDim.x) {
-            const int qlen = t.subsequence_begins[s + 1] - t.subsequence_begins[s];
-            if (qlen < 2) continue;
-            const int past = max(0, t.past_lens[s]);
-            const int groups = t.past_lens[s] < 0 ? 0 : (past + qlen + 127) / 128;
-            const int g0 = atomicAdd(&s_groups, groups);
-            kv_base[s] = g0 * 128;
-            for (int i = 0; i < groups; ++i)
-                if (g0 + i < owner_groups) owner[g0 + i] = s;
-        }
-    }
     __syncthreads();
-    for (int s = threadIdx.x; s < t.num_seqs; s += blockDim.x) {
-        const int qlen = t.subsequence_begins[s + 1] - t.subsequence_begins[s];
-        if (qlen < 2) continue;
-        const int past = max(0, t.past_lens[s]);
-        const int pairs = (((qlen + 127) / 128) * G + 1) / 2;
-        // inconsistent tables (reported): the sequence's items are empty
-        const int tok0 = t.subsequence_begins[s], bib0 = t.block_indices_begins[s];
-        const bool ok = t.past_lens[s] >= 0 && tok0 >= 0 && tok0 + qlen <= t.num_tokens &&
-                        (past + qlen + 15) / 16 <= t.block_indices_begins[s + 1] - bib0;
-        if (!ok) report(status, B2A_DEV_BAD_LEN);
-        const int4 rec0 = make_int4(s, tok0, ok ? qlen : 0, past);
-        const int base = kv_base != nullptr ? kv_base[s] : 0;  // (written by this thread above)
-        for (int i = 0; i < pairs; ++i) {
-            const int at = atomicAdd(&s_hist[weight(past, qlen, i)], 1);
-            if (at < capacity) {
-                int4* rec = reinterpret_cast<int4*>(plan + kPlanHeaderInts) + 2 * at;
-                rec[0] = rec0;
-                rec[1] = make_int4(i, base, 0, 0);
+    for (int s0 = 0; s0 < t.num_seqs; s0 += 256) {
+        if (t.num_seqs > 256) {  // (a single chunk is still there)
+            __syncthreads();
+            load_chunk(s0);
+            __syncthreads();
+        }
+        for (int i = warp; i < min(256, t.num_seqs - s0); i += 8) {
+            const int s = s0 + i, qlen = c_qlen[i];
+            if (qlen == 0) continue;
+            const int past = max(0, c_past[i]), pairs = pairs_of(qlen);
+            int base = 0;
+            if (owner != nullptr) {  // the sequence's rows of the scratch
+                const int groups = c_past[i] < 0 ? 0 : (past + qlen + 127) / 128;
+                if (lane == 0) base = atomicAdd(&s_groups, groups);
+                base = __shfl_sync(0xffffffffu, base, 0);
+                for (int g = lane; g < groups; g += 32)
+                    if (base + g < owner_groups) owner[base + g] = s;
+                base *= 128;
+                if (lane == 0) kv_base[s] = base;
+            }
+            // inconsistent tables (reported): the sequence's items are empty
+            const bool ok = c_ok[i] != 0;
+            if (!ok && lane == 0) report(status, B2A_DEV_BAD_LEN);
+            const int4 rec0 = make_int4(s, c_tok[i], ok ? qlen : 0, past);
+            for (int k = lane; k < pairs; k += 32) {
+                const int at = atomicAdd(&s_hist[weight(past, qlen, k)], 1);
+                if (at < capacity) {
+                    int4* rec = reinterpret_cast<int4*>(plan + kPlanHeaderInts) + 2 * at;
+                    rec[0] = rec0;
+                    rec[1] = make_int4(k, base, 0, 0);
+                }
             }
         }
     }
@@ -386,51 +416,69 @@ __device__ __forceinline__ void dequant_piece_f16(uint4 w, unsigned short scale_
 }
 
 // De-quantise the contexts of the step's multi-token sequences into the f16 scratch [Hkv][rows][128] (K and V each):
-// one CTA per (16 scratch rows, KV head), thread = (token, 16-byte piece) for K and again for V.  Rows past a
-// sequence's context (its range is rounded up to 128 rows) become zeros, so a tile that reaches past the context
+// one CTA per (kGatherRows scratch rows, KV head), thread = (token, 16-byte piece) of K and of V in every block of sixteen.
+// A chain of dependent loads (owner, tables, block ids, cache), so a thread carries several blocks along it at once.  Rows
+// past a sequence's context (its range is rounded up to 128 rows) become zeros, so a tile that reaches past the context
 // holds nothing that could turn 0 * x into NaN.
+constexpr int kGatherRows = 64;
 __global__ void __launch_bounds__(128) paged_gather_kernel(const PagedTables t, const uint8_t* k_cache, const uint8_t* v_cache,
                                                            const int Hkv, const int* kv_base, const int* owner,
                                                            const int scratch_rows, uint16_t* k_out, uint16_t* v_out,
                                                            int32_t* status) {
-    const int row0 = blockIdx.x * 16, hk = blockIdx.y;
+    constexpr int kBlocks = kGatherRows / 16;
+    const int row0 = blockIdx.x * kGatherRows, hk = blockIdx.y;
     grid_dependency_wait();  // the scratch layout (plan kernel) and this step's cache rows (store kernel)
     grid_launch_dependents();
     const int seq = owner[row0 / 128];
     if (seq < 0) return;
     const int tok = threadIdx.x >> 3, c16 = threadIdx.x & 7;
-    const int pos = row0 - kv_base[seq] + tok;  // position inside the sequence
+    const int pos0 = row0 - kv_base[seq] + tok;  // position inside the sequence
     const int qlen = t.subsequence_begins[seq + 1] - t.subsequence_begins[seq];
     const int ctx = t.past_lens[seq] + qlen;
-    uint4 wk = make_uint4(0u, 0u, 0u, 0u), wv = wk;
-    unsigned short sck = 0, zpk = 0, scv = 0, zpv = 0;
-    if (pos < ctx) {
-        const int lb = pos >> 4;
-        int phys = -1;
-        if (lb < t.block_indices_begins[seq + 1] - t.block_indices_begins[seq]) phys = t.block_indices[t.block_indices_begins[seq] + lb];
-        if (phys < 0 || phys >= t.num_blocks_total) {
-            report(status, B2A_DEV_BAD_BLOCK);
-        } else {
-            const size_t chunk = (static_cast<size_t>(phys) * Hkv + hk) * kCacheChunk;
-            const int tb = pos & 15;
-            wk = *reinterpret_cast<const uint4*>(k_cache + chunk + tb * 128 + c16 * 16);
-            wv = *reinterpret_cast<const uint4*>(v_cache + chunk + tb * 128 + c16 * 16);
-            const unsigned short* mk = reinterpret_cast<const unsigned short*>(k_cache + chunk + 2048);
-            const unsigned short* mv = reinterpret_cast<const unsigned short*>(v_cache + chunk + 2048);
-            sck = mk[tb];
-            zpk = mk[16 + tb];
-            scv = mv[tb];
-            zpv = mv[16 + tb];
+    const int bib0 = t.block_indices_begins[seq], have = t.block_indices_begins[seq + 1] - bib0;
+    int phys[kBlocks];
+#pragma unroll
+    for (int i = 0; i < kBlocks; ++i) {
+        const int pos = pos0 + 16 * i, lb = pos >> 4;
+        phys[i] = -1;
+        if (pos < ctx) {
+            if (lb < have) phys[i] = t.block_indices[bib0 + lb];
+            if (phys[i] < 0 || phys[i] >= t.num_blocks_total) {
+                report(status, B2A_DEV_BAD_BLOCK);
+                phys[i] = -1;
+            }
         }
     }
-    const size_t at = (static_cast<size_t>(hk) * scratch_rows + row0 + tok) * kHeadDim + c16 * 16;
-    uint32_t o[8];
-    dequant16_f16(wk, sck, zpk, o);
-    *reinterpret_cast<uint4*>(k_out + at) = make_uint4(o[0], o[1], o[2], o[3]);
-    *reinterpret_cast<uint4*>(k_out + at + 8) = make_uint4(o[4], o[5], o[6], o[7]);
-    dequant16_f16(wv, scv, zpv, o);
-    *reinterpret_cast<uint4*>(v_out + at) = make_uint4(o[0], o[1], o[2], o[3]);
-    *reinterpret_cast<uint4*>(v_out + at + 8) = make_uint4(o[4], o[5], o[6], o[7]);
+    uint4 wk[kBlocks], wv[kBlocks];
+    unsigned short sck[kBlocks], zpk[kBlocks], scv[kBlocks], zpv[kBlocks];
+    const int tb = pos0 & 15;  // (the same in every block)
+#pragma unroll
+    for (int i = 0; i < kBlocks; ++i) {
+        wk[i] = wv[i] = make_uint4(0u, 0u, 0u, 0u);
+        sck[i] = zpk[i] = scv[i] = zpv[i] = 0;
+        if (phys[i] >= 0) {
+            const size_t chunk = (static_cast<size_t>(phys[i]) * Hkv + hk) * kCacheChunk;
+            wk[i] = *reinterpret_cast<const uint4*>(k_cache + chunk + tb * 128 + c16 * 16);
+            wv[i] = *reinterpret_cast<const uint4*>(v_cache + chunk + tb * 128 + c16 * 16);
+            const unsigned short* mk = reinterpret_cast<const unsigned short*>(k_cache + chunk + 2048);
+            const unsigned short* mv = reinterpret_cast<const unsigned short*>(v_cache + chunk + 2048);
+            sck[i] = mk[tb];
+            zpk[i] = mk[16 + tb];
+            scv[i] = mv[tb];
+            zpv[i] = mv[16 + tb];
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kBlocks; ++i) {
+        const size_t at = (static_cast<size_t>(hk) * scratch_rows + row0 + 16 * i + tok) * kHeadDim + c16 * 16;
+        uint32_t o[8];
+        dequant16_f16(wk[i], sck[i], zpk[i], o);
+        *reinterpret_cast<uint4*>(k_out + at) = make_uint4(o[0], o[1], o[2], o[3]);
+        *reinterpret_cast<uint4*>(k_out + at + 8) = make_uint4(o[4], o[5], o[6], o[7]);
+        dequant16_f16(wv[i], scv[i], zpv[i], o);
+        *reinterpret_cast<uint4*>(v_out + at) = make_uint4(o[0], o[1], o[2], o[3]);
+        *reinterpret_cast<uint4*>(v_out + at + 8) = make_uint4(o[4], o[5], o[6], o[7]);
+    }
 }
 
 // kMode: 0 dense tensors; 1 paged, K/V de-quantised by producer warps inside the kernel; 2 paged, K/V de-quantised
@@ -1566,7 +1614,7 @@ int paged_tc_launch(const b2a_paged_desc& d, const void* query, const void* k_ca
     if (gathered) {
         uint16_t* ks = reinterpret_cast<uint16_t*>(ws + w.k_at);
         uint16_t* vs = reinterpret_cast<uint16_t*>(ws + w.v_at);
-        if (launch_overlapped(paged_gather_kernel, dim3(w.rows / 16, d.Hkv), dim3(128), 0, stream, t,
+        if (launch_overlapped(paged_gather_kernel, dim3(w.rows / kGatherRows, d.Hkv), dim3(128), 0, stream, t,
                               static_cast<const uint8_t*>(k_cache), static_cast<const uint8_t*>(v_cache), d.Hkv,
                               static_cast<const int*>(kv_base), static_cast<const int*>(owner), w.rows, ks, vs,
                               status) != cudaSuccess)

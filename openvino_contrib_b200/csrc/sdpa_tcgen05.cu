@@ -49,6 +49,8 @@
 // loops, outstanding copies and MMAs are drained with bounded waits, TMEM is freed and the status word gets
 // B2A_DEV_TIMEOUT.  All barrier phases are derived from running counts (K/V ring position, steps of a tile, Q tiles
 // loaded) so that they carry over from one item to the next.
+#include <algorithm>
+
 #include "launch.cuh"
 #include "tcgen05.cuh"
 
@@ -63,13 +65,14 @@ constexpr int kHeadDim = 128;
 constexpr int kPanel = 128 * 128;    // bytes of one [128 rows x 64 elements] swizzled panel
 constexpr int kThreadsDense = 384;   // 3 warpgroups: softmax A, softmax B, {producer, MMA issuer, 2 idle warps}
 constexpr int kThreadsPaged = 512;   // plus the de-quantising producer warpgroup
-constexpr int kNumBars = 23;
+constexpr int kNumBars = 27;
 constexpr int kStageOut = 8 * 4096;  // epilogue staging: one [32 rows x 64 elements] slab per softmax warp
 constexpr int smem_bytes(int tile) { return 6 * tile + kStageOut + 1024 /* alignment slack */ + 256 /* barriers, TMEM slot, abort flag */; }
 constexpr float kLazyThreshold = 8.0f;  // log2 units
 constexpr int kCacheChunk = 16 * (kHeadDim + 4);  // bytes of one (block, KV head) chunk of the u8 pool
 
-enum Bar { Q_FULL = 0, K_FULL = 2, K_EMPTY = 4, V_FULL = 6, V_EMPTY = 8, S_FULL = 10, P_READY = 12, O_DONE = 14, DRAIN = 16, P_HALF = 17, Q_CONV = 19, Q_EMPTY = 21 };
+enum Bar { Q_FULL = 0, K_FULL = 2, K_EMPTY = 4, V_FULL = 6, V_EMPTY = 8, S_FULL = 10, P_READY = 12, O_DONE = 14, DRAIN = 16, P_HALF = 17, Q_CONV = 19, Q_EMPTY = 21,
+           HALVES = 23 };
 
 // n / d for 0 <= n < 2^31 by one multiplication: mul = ceil(2^(31 + shift) / d) with shift = ceil(log2 d) errs by less than
 // n / 2^(31 + shift) < 1 / d (Granlund and Montgomery's division by an invariant).  A role works out its place from the
@@ -493,11 +496,19 @@ __global__ void __launch_bounds__(128) paged_gather_kernel(const PagedTables t, 
 //   instructions per pair of probabilities.  Bound: the special-function unit, 128 exponentials per row and step; the
 //   f16 encoder batch of 8 x 16 heads x 512 tokens, head size 64, boolean padding mask: 1167 us in attn_generic_kernel,
 //   28.7 us here (5.1 us of memory traffic at the copy rate).
-template <bool kBf16, int kMode, int kMask = 0, int kDim = kHeadDim, bool kSplitP = false>
+// kKeySplit (dense): a small problem - fewer pairs of tiles than SMs - is bound by its longest chain of key steps, one tile's
+//   softmax after the other's.  Then an item is ONE tile whose keys are shared out: "tile A" takes the first half of its key
+//   tiles, "tile B" the second, each with its own maximum, sum and accumulator, which are merged in the epilogue (the two
+//   warps of the same 32 rows exchange maximum and sum through shared memory and read both accumulators: a warp reaches
+//   the tensor-memory lanes of its number modulo four).  One item per CTA; the launcher's rule compares the two chains.
+//   Causal prompts, 32/8 heads, D = 128, graph replay: 512 tokens 12.9 -> 9.4 us, 777 tokens 17.6 -> 15.7 us; 8 heads x 2048
+//   tokens, D = 64, no mask: 36.9 -> 22.2 us.
+template <bool kBf16, int kMode, int kMask = 0, int kDim = kHeadDim, bool kSplitP = false, bool kKeySplit = false>
 __global__ void __launch_bounds__(kMode == 1 ? kThreadsPaged : kThreadsDense, 1)
 attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                const __grid_constant__ CUtensorMap tmV, const TcParams p, const __grid_constant__ TcPeers peers) {
     static_assert(kDim == kHeadDim || kMode == 0, "the paged modes are built for a head size of 128");
+    static_assert(!kKeySplit || kMode == 0, "the keys of a tile are shared out in dense mode only");
     constexpr int kTile = 128 * kDim * 2;  // bytes of a [128 x kDim] 16-bit tile: kDim / 64 panels
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -567,6 +578,21 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 return true;
             }
         } else {
+            if constexpr (kKeySplit) {  // one tile, both halves of its keys; heaviest row blocks first
+                if (k > 0) return false;
+                const int idx = static_cast<int>(blockIdx.x), round = div_by(idx, p.div_streams), y = idx - round * p.B * p.Hkv;
+                const int t = tiles - 1 - round, rb = div_by(t, p.div_g);
+                it.b = div_by(y, p.div_hkv);
+                it.hk = y - it.b * p.Hkv;
+                it.row0A = it.row0B = rb * kBM;
+                it.headA = it.headB = it.hk * p.G + (t - rb * p.G);
+                const int n = ((causal ? min(kv_limit, it.row0A + kBM) : kv_limit) + kBN - 1) / kBN;
+                it.nkvA = (n + 1) / 2;
+                it.nkvB = n / 2;
+                it.kv_tile0 = 0;
+                it.nmax = it.nkvA;
+                return true;
+            }
             const int ctas = static_cast<int>(gridDim.x), me = static_cast<int>(blockIdx.x);
             // With four or more ranks the step is bound by the exchange of the output tiles, which can only start
             // when the first items end: then a CTA walks the SAME items (the deal below is what balances the CTAs)
@@ -628,6 +654,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             if (i == P_READY || i == P_READY + 1 || i == P_HALF || i == P_HALF + 1) count = 128;
             if (i == Q_CONV || i == Q_CONV + 1) count = 128;
             if (i == Q_EMPTY || i == Q_EMPTY + 1) count = 1;
+            if (i >= HALVES) count = 64;  // the two warps of the same rows
             if (kDequant && (i == K_FULL || i == K_FULL + 1 || i == V_FULL || i == V_FULL + 1)) count = 128;
             if (kGathered && (i == Q_CONV || i == Q_CONV + 1)) count = 64;  // converted by warps 10 and 11
             mbar_init(BAR(i), count);
@@ -842,7 +869,23 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                     load_q(0);
                     if (ok) load_q(1);
                 }
-                if constexpr (!kDequant) {
+                if constexpr (kKeySplit) {
+                    // tiles in the order A0 B0 A1 B1 ..: stage 0 of the rings is A's, stage 1 is B's; both use A's queries
+                    for (int n = 0; ok && n < it.nkvA + it.nkvB; ++n) {
+                        const int st = n & 1, j = n >> 1, row = (st ? it.nkvA + j : j) * kBN;
+                        if (j > 0 && !mbar_wait(BAR(K_EMPTY + st), (j - 1) & 1, abort_flag)) { ok = false; break; }
+                        mbar_expect_tx(BAR(K_FULL + st), kTile);
+                        tma_load_4d(sK + st * kTile, &tmK, BAR(K_FULL + st), 0, row, it.hk, it.b);
+                        if constexpr (kDim > 64) tma_load_4d(sK + st * kTile + kPanel, &tmK, BAR(K_FULL + st), 64, row, it.hk, it.b);
+                        ++issued_k;
+                        if (n == 0) load_q(0);
+                        if (j > 0 && !mbar_wait(BAR(V_EMPTY + st), (j - 1) & 1, abort_flag)) { ok = false; break; }
+                        mbar_expect_tx(BAR(V_FULL + st), kTile);
+                        tma_load_4d(sV + st * kTile, &tmV, BAR(V_FULL + st), 0, row, it.hk, it.b);
+                        if constexpr (kDim > 64) tma_load_4d(sV + st * kTile + kPanel, &tmV, BAR(V_FULL + st), 64, row, it.hk, it.b);
+                        ++issued_v;
+                    }
+                } else if constexpr (!kDequant) {
                     // gathered mode: the sequence's keys start at row kv_row0 of the scratch, which is one [1, Hkv, rows, 128] tensor
                     const int kv_row0 = kGathered ? kv_row_base + it.kv_tile0 * kBN : 0;
                     for (int j = 0; ok && j < it.nmax; ++j, ++g) {
@@ -887,7 +930,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             const uint32_t q16 = (sQ >> 4) & 0x3FFFu, k16 = (sK >> 4) & 0x3FFFu, v16 = (sV >> 4) & 0x3FFFu;
             auto issue_qk = [&](int X, int st) {  // S_X = Q_X K^T : steps of 16 along D
                 const uint32_t d = tmem + static_cast<uint32_t>(X * 128);
-                const uint32_t qa = q16 + static_cast<uint32_t>(X * (kTile >> 4)), ka = k16 + static_cast<uint32_t>(st * (kTile >> 4));
+                const uint32_t qa = q16 + static_cast<uint32_t>((kKeySplit ? 0 : X) * (kTile >> 4)), ka = k16 + static_cast<uint32_t>(st * (kTile >> 4));
 #define B2A_QK(ks) \
     mma_ss_c<((((ks) / 4) * kPanel + ((ks) & 3) * 32) / 16), ((((ks) / 4) * kPanel + ((ks) & 3) * 32) / 16), kLoK, kLoK, kHiK, kHiK, \
              idesc_qk>(d, qa, ka, (ks) > 0 ? 1u : 0u)
@@ -917,6 +960,40 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             for (int k = 0; ok && get_item(k, it); ++k) {
                 const int nkvA = it.nkvA, nkvB = it.nkvB, nmax = it.nmax;
                 if (nmax == 0) continue;  // an item that was refused (inconsistent tables)
+                if constexpr (kKeySplit) {
+                    const int n = nkvA + nkvB;
+                    ok = mbar_wait(BAR(Q_FULL), 0, abort_flag);
+                    for (int X = 0; ok && X < min(n, 2); ++X) {
+                        ok = mbar_wait(BAR(K_FULL + X), 0, abort_flag);
+                        if (!ok) break;
+                        tc_fence_after();
+                        issue_qk(X, X);
+                        mma_commit(BAR(S_FULL + X));
+                        mma_commit(BAR(K_EMPTY + X));
+                    }
+                    for (int i = 0; ok && i < n; ++i) {
+                        const int X = i & 1, j = i >> 1;
+                        ok = mbar_wait(BAR(V_FULL + X), j & 1, abort_flag) && mbar_wait(BAR(P_HALF + X), j & 1, abort_flag);
+                        if (!ok) break;
+                        tc_fence_after();
+                        issue_pv(X, X, j > 0, 0);
+                        ok = mbar_wait(BAR(P_READY + X), j & 1, abort_flag);
+                        if (!ok) break;
+                        tc_fence_after();
+                        issue_pv(X, X, true, 1);
+                        mma_commit(BAR(O_DONE + X));
+                        mma_commit(BAR(V_EMPTY + X));
+                        if (i + 2 < n) {
+                            ok = mbar_wait(BAR(K_FULL + X), (j + 1) & 1, abort_flag);
+                            if (!ok) break;
+                            tc_fence_after();
+                            issue_qk(X, X);
+                            mma_commit(BAR(S_FULL + X));
+                            mma_commit(BAR(K_EMPTY + X));
+                        }
+                    }
+                    break;  // one item per CTA
+                }
                 ok = ok && mbar_wait(BAR(K_FULL + (g0 & 1)), (g0 >> 1) & 1, abort_flag);
                 if (nkvA > 0) ok = ok && mbar_wait(BAR(kQReady + 0), qn[0] & 1, abort_flag);
                 if (!ok) break;
@@ -1002,10 +1079,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 const int j_end = kv_limit / kBN;
                 const int dgl = row_pos0 - (kBN - 1);
                 const int j_diag = dgl < 0 ? 0 : dgl / kBN + 1;
-                jb = (causal ? min(j_end, j_diag) : j_end) - (kPaged ? item.kv_tile0 : 0);
+                jb = (causal ? min(j_end, j_diag) : j_end) - (kPaged ? item.kv_tile0 : kKeySplit && X ? item.nkvA : 0);
             }
             // with a sliding window, key tiles that begin below the window of the tile's LAST row need the mask too
-            const int tile0 = kPaged ? item.kv_tile0 : 0;
+            const int tile0 = kPaged ? item.kv_tile0 : kKeySplit && X ? item.nkvA : 0;
             const int window = kPaged ? p.window : 0;
             const int low_limit = window > 0 ? row_pos0 + kBM - window : -(1 << 30);  // mask while key0 < low_limit
             // (additive masks: the blocks below have scaled the scores)
@@ -1028,7 +1105,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 if constexpr (kMask == 3) {
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
-                        const int key = j * kBN + 32 * q + lane;
+                        const int key = (tile0 + j) * kBN + 32 * q + lane;
                         mword[q] = key < kv_limit ? mrow[key * p.mask_strides[3]] : 0u;
                     }
 #pragma unroll
@@ -1038,7 +1115,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                     float mv[4];
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
-                        const int key = j * kBN + 32 * q + lane;
+                        const int key = (tile0 + j) * kBN + 32 * q + lane;
                         mv[q] = key < kv_limit ? mask_log2<kBf16>(mrow, key * p.mask_strides[3]) : -INFINITY;
                     }
                     __syncwarp();  // the last step's values have been read
@@ -1232,13 +1309,60 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 tc_fence_after();
                 const float inv = l > 0.f ? 1.f / l : 0.f;
                 // where the tile goes: worked out again here rather than kept in registers across the key loop
-                if constexpr (!kPaged) {  // (paged items come from tables in global memory: those are kept)
+                if constexpr (!kPaged && !kKeySplit) {  // (paged items come from tables in global memory: those are kept)
                     int k_again = k;
                     asm volatile("" : "+r"(k_again));
                     get_item(k_again, item);
                 }
                 const int row0 = X ? item.row0B : item.row0A, head = X ? item.headB : item.headA, b = item.b;
-                if (kPaged || peers.world == 0) {
+                if constexpr (kKeySplit) {
+                    // (maximum, sum) of this row's other half of the keys, from the warp that has it; a tile of one key
+                    // step has no other half
+                    const bool both = item.nkvB > 0;
+                    float inv_own = inv, inv_other = 0.f;
+                    if (both) {
+                        float2* mine = reinterpret_cast<float2*>(gbase + 6 * kTile + warp * 4096 + 1024);
+                        const float2* theirs = reinterpret_cast<const float2*>(gbase + 6 * kTile + (warp ^ 4) * 4096 + 1024);
+                        mine[lane] = make_float2(m_used, l);
+                        tc_fence_before();
+                        mbar_arrive(BAR(HALVES + (warp & 3)));
+                        ok = __all_sync(0xffffffffu, mbar_wait(BAR(HALVES + (warp & 3)), 0, abort_flag));
+                        if (!ok) break;
+                        tc_fence_after();  // (the other warp has waited for its accumulator: it may be read here too)
+                        const float2 o = theirs[lane];
+                        const float m = fmaxf(m_used, o.x);
+                        const float f_own = ex2f(m_used - m), f_other = ex2f(o.x - m);
+                        const float sum = l * f_own + o.y * f_other;
+                        const float inv_sum = sum > 0.f ? 1.f / sum : 0.f;
+                        inv_own = f_own * inv_sum;
+                        inv_other = f_other * inv_sum;
+                    }
+                    uint16_t* orow = static_cast<uint16_t*>(p.out) + b * p.out_strides[0] + head * p.out_strides[1] +
+                                     (row0 + r) * p.out_strides[2];
+                    const bool valid = row0 + r < nrows_total;
+                    const uint32_t tOther = tmem + lane_base + static_cast<uint32_t>(256 + (X ^ 1) * 128);
+#pragma unroll
+                    for (int q = 0; q < kDim / 32; ++q) {
+                        if (both && (q / (kDim / 64)) != X) continue;  // the other warp's columns
+                        uint32_t o[32], w[16];
+                        tmem_ld32(tO + 32 * q, o);
+                        if (both) {
+                            uint32_t o2[32];
+                            tmem_ld32(tOther + 32 * q, o2);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int i = 0; i < 32; ++i)
+                                o[i] = __float_as_uint(__uint_as_float(o[i]) * inv_own + __uint_as_float(o2[i]) * inv_other);
+                        } else {
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * inv_own);
+                        }
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) w[i] = pack2<kBf16>(__uint_as_float(o[2 * i]), __uint_as_float(o[2 * i + 1]));
+                        if (valid) store_64_bytes(orow + 32 * q, w, p.out_wide != 0);
+                    }
+                } else if (kPaged || peers.world == 0) {
                     // A thread's row straight from its registers, whole 32-byte sectors: nothing to wait for, and the
                     // warp goes on to the next item while the stores drain.  (Through the slab and TMA stores, the second
                     // half waited for the first to be read, behind the next item's loads in the TMA unit's queue: 5000
@@ -1387,12 +1511,12 @@ bool make_map(CUtensorMap* map, const void* ptr, bool bf16, int B, int H, int S,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int kMask, int kDim, bool kSplitP>
+template <int kMask, int kDim, bool kSplitP, bool kKeySplit = false>
 int launch_dense(bool bf16, dim3 grid, cudaStream_t stream, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                  const TcParams& p, const TcPeers& peers) {
     constexpr int smem = smem_bytes(128 * kDim * 2);
     static bool configured[2][64] = {};
-    auto kern = bf16 ? attn_tc_kernel<true, 0, kMask, kDim, kSplitP> : attn_tc_kernel<false, 0, kMask, kDim, kSplitP>;
+    auto kern = bf16 ? attn_tc_kernel<true, 0, kMask, kDim, kSplitP, kKeySplit> : attn_tc_kernel<false, 0, kMask, kDim, kSplitP, kKeySplit>;
     const int rc = configure_once(kern, configured[bf16], smem);
     if (rc != B2A_OK) return rc;
     return launch_overlapped(kern, grid, dim3(kThreadsDense), smem, stream, mq, mk, mv, p, peers) == cudaSuccess ? B2A_OK : B2A_ERR_CUDA;
@@ -1507,12 +1631,33 @@ int sdpa_tc_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t
         p.mask_kind = mask_kind;
         for (int i = 0; i < 4; ++i) p.mask_strides[i] = d.mask_strides[i];
     }
+    // Pairs of tiles, or single tiles with their keys shared out (kKeySplit)?  With fewer pairs than SMs the former takes the
+    // longest pair's key steps, n; the latter the longest half or, if more, the halves' steps over the SMs, plus another
+    // CTA's start (about one and a half steps) when there are more tiles than SMs.
+    bool key_split = false;
+    const long long streams = static_cast<long long>(d.B) * d.Hkv, all_tiles = streams * nrb * p.G;
+    if (peer_out == nullptr && items <= sms) {
+        const int n = ((d.causal ? std::min(d.Skv, nrb * kBM) : d.Skv) + kBN - 1) / kBN;
+        long long halves = 0;
+        for (int rb = 0; rb < nrb; ++rb) {
+            const int keys = d.causal ? std::min(d.Skv, (rb + 1) * kBM) : d.Skv;
+            halves += ((keys + kBN - 1) / kBN + 1) / 2;
+        }
+        const double steps = std::max<double>((n + 1) / 2, static_cast<double>(halves * p.G * streams) / sms);
+        key_split = steps + (all_tiles > sms ? 1.5 : 0.0) < n;
+    }
+    const dim3 tile_grid(static_cast<unsigned>(key_split ? all_tiles : 0));
     if (split_p) {
         // a mask that is one row for all queries is read once per warp; anything else row by row
         const int form = mask_kind == B2A_MASK_NONE                    ? 0
                          : d.mask_strides[2] != 0 && d.Sq > 1          ? 5
                          : mask_kind == B2A_MASK_BOOL                  ? 3
                                                                        : 4;
+        if (d.D == 64 && key_split && form != 5) {
+            if (form == 0) return launch_dense<0, 64, true, true>(bf16, tile_grid, stream, mq, mk, mv, p, peers);
+            if (form == 3) return launch_dense<3, 64, true, true>(bf16, tile_grid, stream, mq, mk, mv, p, peers);
+            return launch_dense<4, 64, true, true>(bf16, tile_grid, stream, mq, mk, mv, p, peers);
+        }
         if (d.D == 64) {
             if (form == 0) return launch_dense<0, 64, true>(bf16, grid, stream, mq, mk, mv, p, peers);
             if (form == 3) return launch_dense<3, 64, true>(bf16, grid, stream, mq, mk, mv, p, peers);
@@ -1525,6 +1670,7 @@ int sdpa_tc_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t
     }
     if (mask_kind == B2A_MASK_BOOL) return launch_dense<1, kHeadDim, false>(bf16, grid, stream, mq, mk, mv, p, peers);
     if (mask_kind == B2A_MASK_ADD) return launch_dense<2, kHeadDim, false>(bf16, grid, stream, mq, mk, mv, p, peers);
+    if (key_split) return launch_dense<0, kHeadDim, false, true>(bf16, tile_grid, stream, mq, mk, mv, p, peers);
     return launch_dense<0, kHeadDim, false>(bf16, grid, stream, mq, mk, mv, p, peers);
 }
 

@@ -1321,8 +1321,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                     const bool both = item.nkvB > 0;
                     float inv_own = inv, inv_other = 0.f;
                     if (both) {
-                        float2* mine = reinterpret_cast<float2*>(gbase + 6 * kTile + warp * 4096 + 1024);
-                        const float2* theirs = reinterpret_cast<const float2*>(gbase + 6 * kTile + (warp ^ 4) * 4096 + 1024);
+                        float2* mine = reinterpret_cast<float2*>(gbase + kTile) + warp * 32;  // (Q tile B's place, not used here)
+                        const float2* theirs = reinterpret_cast<const float2*>(gbase + kTile) + (warp ^ 4) * 32;
                         mine[lane] = make_float2(m_used, l);
                         tc_fence_before();
                         mbar_arrive(BAR(HALVES + (warp & 3)));
@@ -1360,7 +1360,31 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                         }
 #pragma unroll
                         for (int i = 0; i < 16; ++i) w[i] = pack2<kBf16>(__uint_as_float(o[2 * i]), __uint_as_float(o[2 * i + 1]));
-                        if (valid) store_64_bytes(orow + 32 * q, w, p.out_wide != 0);
+                        if (peers.world == 0) {
+                            if (valid) store_64_bytes(orow + 32 * q, w, p.out_wide != 0);
+                            continue;
+                        }
+                        // sharded heads: 64 columns through this warp's slab into every rank's buffer, as below
+                        if ((q & 1) == 0) {
+                            if (lane == 0) tma_store_wait_read();
+                            __syncwarp();
+                        }
+#pragma unroll
+                        for (int ch = 0; ch < 4; ++ch)
+                            *reinterpret_cast<uint4*>(gbase + 6 * kTile + warp * 4096 + lane * 128 + ((((q & 1) * 4 + ch) ^ (lane & 7)) << 4)) =
+                                make_uint4(w[4 * ch], w[4 * ch + 1], w[4 * ch + 2], w[4 * ch + 3]);
+                        if ((q & 1) == 1) {
+                            fence_proxy_async_smem();
+                            __syncwarp();
+                            if (lane == 0) {
+                                for (int i = 1; i <= peers.world; ++i) {
+                                    const int dst = (peers.rank + i) % peers.world;
+                                    tma_store_4d(&peers.out_map[dst], sOut + static_cast<uint32_t>(warp) * 4096u, 32 * (q - 1),
+                                                 row0 + 32 * (warp & 3), peers.head_offset + head, b);
+                                }
+                                tma_store_commit();
+                            }
+                        }
                     }
                 } else if (kPaged || peers.world == 0) {
                     // A thread's row straight from its registers, whole 32-byte sectors: nothing to wait for, and the
@@ -1409,13 +1433,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                         fence_proxy_async_smem();
                         __syncwarp();
                         if (lane == 0) {
-                            {
-                                // the slab into every rank's buffer, the next rank first so that the ranks do
-                                // not all write to the same peer at the same time; local copy last
-                                for (int i = 1; i <= peers.world; ++i) {
-                                    const int dst = (peers.rank + i) % peers.world;
-                                    tma_store_4d(&peers.out_map[dst], slab, 64 * half, row0 + 32 * (warp & 3), peers.head_offset + head, b);
-                                }
+                            // the slab into every rank's buffer, the next rank first so that the ranks do not all write to
+                            // the same peer at the same time; local copy last
+                            for (int i = 1; i <= peers.world; ++i) {
+                                const int dst = (peers.rank + i) % peers.world;
+                                tma_store_4d(&peers.out_map[dst], slab, 64 * half, row0 + 32 * (warp & 3), peers.head_offset + head, b);
                             }
                             tma_store_commit();
                         }
@@ -1636,7 +1658,8 @@ int sdpa_tc_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t
     // CTA's start (about one and a half steps) when there are more tiles than SMs.
     bool key_split = false;
     const long long streams = static_cast<long long>(d.B) * d.Hkv, all_tiles = streams * nrb * p.G;
-    if (peer_out == nullptr && items <= sms) {
+    // (Sharded launches follow the same rule: their output is the unsharded kernel's, bit for bit.)
+    if (items <= sms) {
         const int n = ((d.causal ? std::min(d.Skv, nrb * kBM) : d.Skv) + kBN - 1) / kBN;
         long long halves = 0;
         for (int rb = 0; rb < nrb; ++rb) {

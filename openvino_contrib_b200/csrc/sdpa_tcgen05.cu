@@ -22,10 +22,8 @@
 //   warps 0-3   softmax of tile A: thread = query row = TMEM lane.  Reads S_A (tcgen05.ld), keeps the running max
 //               and sum, writes P_A = exp2(S*c - m) as 16-bit pairs over the first half of S_A's columns
 //               (tcgen05.st) and signals the MMA issuer after the first 64 keys and again after all 128; rescales
-//               O_A in TMEM when the maximum moved; finally normalises O_A and stores it (dense: through a
-//               staging slab per warp - [32 x 64] and one TMA tensor store per slab, to every rank's buffer when the
-//               heads are sharded over two ranks; pieces of 16 full rows and one bulk store per rank from four ranks
-//               on; paged: row-wise stores).
+//               O_A in TMEM when the maximum moved; finally normalises O_A and stores it, a thread its row (heads sharded
+//               over several ranks: through a staging slab per warp, [32 x 64] and one TMA tensor store per slab and rank).
 //   warps 4-7   the same for tile B.
 //   warp  8     TMA producer (one lane): the Q tiles of an item as soon as the previous item's last QK^T has
 //               completed, and (modes 0, 2) K_j and V_j into two-stage rings that run on across items.

@@ -1652,20 +1652,24 @@ int sdpa_tc_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t
         for (int i = 0; i < 4; ++i) p.mask_strides[i] = d.mask_strides[i];
     }
     // Pairs of tiles, or single tiles with their keys shared out (kKeySplit)?  With fewer pairs than SMs the former takes the
-    // longest pair's key steps, n; the latter the longest half or, if more, the halves' steps over the SMs, plus another
-    // CTA's start (about one and a half steps) when there are more tiles than SMs.
+    // longest pair's key steps, n.  The latter takes the longest half per round of CTAs (tiles of equal length) or, if
+    // more, the halves' steps over the SMs (causal), plus a CTA's start (about one and a half steps) for a second round.
+    // It reads K and V twice as fast.  On more than half of the SMs that is more than the pairs ever ask of L2, and copies
+    // running beside it starve: host tensors in pieces of 8 heads x 4096 tokens (256 tiles) took 5.05 ms a step instead of
+    // 4.53, although the kernel itself went from 61 to 37 us.  So such grids share the keys out up to sixteen steps only.
+    // (Sharded launches follow the same rule: their output is the unsharded kernel's, bit for bit.)
     bool key_split = false;
     const long long streams = static_cast<long long>(d.B) * d.Hkv, all_tiles = streams * nrb * p.G;
-    // (Sharded launches follow the same rule: their output is the unsharded kernel's, bit for bit.)
-    if (items <= sms) {
-        const int n = ((d.causal ? std::min(d.Skv, nrb * kBM) : d.Skv) + kBN - 1) / kBN;
-        long long halves = 0;
-        for (int rb = 0; rb < nrb; ++rb) {
-            const int keys = d.causal ? std::min(d.Skv, (rb + 1) * kBM) : d.Skv;
-            halves += ((keys + kBN - 1) / kBN + 1) / 2;
+    const int n = ((d.causal ? std::min(d.Skv, nrb * kBM) : d.Skv) + kBN - 1) / kBN, half = (n + 1) / 2;
+    if (items <= sms && (n <= 16 || 2 * all_tiles <= sms)) {
+        const long long rounds = (all_tiles + sms - 1) / sms;
+        double steps = static_cast<double>(rounds * half);
+        if (d.causal) {
+            long long halves = 0;
+            for (int rb = 0; rb < nrb; ++rb) halves += ((std::min(d.Skv, (rb + 1) * kBM) + kBN - 1) / kBN + 1) / 2;
+            steps = std::max<double>(half, static_cast<double>(halves * p.G * streams) / sms);
         }
-        const double steps = std::max<double>((n + 1) / 2, static_cast<double>(halves * p.G * streams) / sms);
-        key_split = steps + (all_tiles > sms ? 1.5 : 0.0) < n;
+        key_split = steps + (rounds > 1 ? 1.5 : 0.0) < n;
     }
     const dim3 tile_grid(static_cast<unsigned>(key_split ? all_tiles : 0));
     if (split_p) {

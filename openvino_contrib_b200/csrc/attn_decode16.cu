@@ -4,7 +4,7 @@
 //
 // Bound by HBM: every cached token is 2 * D * 2 bytes per KV head, read once for all the query heads that share it.
 // Both contractions run on the warp-level MMA (m16n8k16) with the keys / the value columns as the M side, so a KV
-// head's rows fill the N side and the instruction count follows the bytes (sixteen keys: 8 KB and 40 MMAs at D = 128).
+// head's rows fill the N side and the instruction count follows the bytes (sixteen keys: 8 KB and 24 to 32 MMAs at D = 128).
 //
 // One launch, no workspace: a CLUSTER of up to eight CTAs owns one (sequence, KV head).  The sequence's 16-key tiles
 // are cut evenly over the cluster whatever its length, each of a CTA's four warps walks its share with its own cp.async
@@ -12,12 +12,13 @@
 // across the cluster through distributed shared memory, every CTA finishing its slice of the output columns.
 // (A workspace would have to be asked of callers that never needed one, and a merge kernel costs a launch.)
 //
-// The probabilities keep float32 precision: they enter the second product as the sum of two 16-bit values, which costs
-// eight more MMAs per tile where the tensor pipe idles anyway.
+// The probabilities keep float32's precision and, as far as a row can tell, its range: they enter the second product as two
+// f16 or three bf16 values (Pieces), which costs eight or sixteen more MMAs per tile where the tensor pipe idles anyway.
 //
 // Measured on a B200 (graph replay): bf16, 8 sequences x 3003 keys x 8 KV heads, additive mask (98 MB): 2049 us on
-// attn_generic_kernel before, 20.9 us now (4.7 TB/s; 14.8 us at the copy rate); 32 bf16 sequences of 256..4096 tokens in
-// a pool (293 MB, with the store of the step): 8149 us before, 54.8 us now (5.3 TB/s; 44 us at the copy rate).
+// attn_generic_kernel before, 23.3 us now (4.2 TB/s; 15.1 us at the copy rate); 32 bf16 sequences of 256..4096 tokens in
+// a pool (293 MB, with the store of the step): 8149 us before, 56.5 us now (5.2 TB/s; 44.8 us at the copy rate).  Two bf16
+// pieces, which keep 2^-16 of a probability, took 22.8 and 55.3 us; two tf32 pieces beside V widened to tf32 24.0 and 59.5.
 #include <algorithm>
 #include <atomic>
 
@@ -122,6 +123,43 @@ template <>
 __device__ __forceinline__ float2 unpack_pair<__nv_bfloat16>(uint32_t w) {
     return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
 }
+
+// Two probabilities as packed pieces of T.
+//   f16: p 2^14 = hi + lo 2^-11, eleven bits each, and lo in an accumulator of its own: with one scale for both, the
+//     probabilities of many keys beside one that stands far above them fall below f16's smallest value (32768 equal keys 17.4
+//     below one with a zero value row: 3 % off).  Here 2^-49 of the maximum still counts.
+//   bf16: p = hi + mid + lo, eight bits each.
+// Every piece but the last is cut from a value a little below what is left, so that all are above zero wherever p is (f16:
+// above 2^-37): an infinity in V then stays one in the sum of the products, where a piece of zero or below would make it NaN.
+template <typename T>
+struct Pieces;
+template <>
+struct Pieces<__half> {
+    static constexpr int kCount = 2, kAccs = 2;  // pieces; accumulators (piece e goes to the e-th or the last of them)
+    static constexpr float kSumScale = 16384.f, kLowScale = 1.f / 2048.f;
+    static __device__ __forceinline__ void split(float p0, float p1, uint32_t (&w)[2]) {
+        p0 *= 16384.f;
+        p1 *= 16384.f;
+        asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(w[0]) : "f"(p1 * (1.f - 1.f / 8192.f)), "f"(p0 * (1.f - 1.f / 8192.f)));
+        const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&w[0]));
+        const __half2 l = __floats2half2_rn((p0 - h.x) * 2048.f, (p1 - h.y) * 2048.f);
+        w[1] = *reinterpret_cast<const uint32_t*>(&l);
+    }
+};
+template <>
+struct Pieces<__nv_bfloat16> {
+    static constexpr int kCount = 3, kAccs = 1;
+    static constexpr float kSumScale = 1.f;
+    static __device__ __forceinline__ void split(float p0, float p1, uint32_t (&w)[3]) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            w[e] = __byte_perm(__float_as_uint(p0 * (1.f - 1.f / 1024.f)), __float_as_uint(p1 * (1.f - 1.f / 1024.f)), 0x7632);
+            p0 -= __uint_as_float(w[e] << 16);
+            p1 -= __uint_as_float(w[e] & 0xffff0000u);
+        }
+        w[2] = pack_pair<__nv_bfloat16>(p0, p1);
+    }
+};
 
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
@@ -315,14 +353,17 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attn_decode16_kernel(const Dec
     for (int nt = 0; nt < NT; ++nt) mv[nt][0] = mv[nt][1] = mv[nt][2] = mv[nt][3] = 0.f;
     if (masked && n_w > 0) load_mask(0);
 
-    float acc[NT][D / 16][4];
+    using P = Pieces<T>;
+    float acc[NT][P::kAccs][D / 16][4];
     float m_a[NT], m_b[NT], l_a[NT], l_b[NT];
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
         m_a[nt] = m_b[nt] = kNegBig;
         l_a[nt] = l_b[nt] = 0.f;
 #pragma unroll
-        for (int j = 0; j < D / 16; ++j) acc[nt][j][0] = acc[nt][j][1] = acc[nt][j][2] = acc[nt][j][3] = 0.f;
+        for (int a = 0; a < P::kAccs; ++a)
+#pragma unroll
+            for (int j = 0; j < D / 16; ++j) acc[nt][a][j][0] = acc[nt][a][j][1] = acc[nt][a][j][2] = acc[nt][a][j][3] = 0.f;
     }
 
     const int mat = lane >> 3, mrow8 = lane & 7;  // ldmatrix: matrix and row whose address this lane supplies
@@ -347,7 +388,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attn_decode16_kernel(const Dec
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) mma16816<T>(sc[nt], a, qf[nt][j][0], qf[nt][j][1]);
         }
-        uint32_t ph[NT][2], pl[NT][2];
+        uint32_t pp[NT][P::kCount][2];
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
             float s0 = fmaf(sc[nt][0], p.scale_log2, mv[nt][0]), s1 = fmaf(sc[nt][1], p.scale_log2, mv[nt][1]);
@@ -369,21 +410,24 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attn_decode16_kernel(const Dec
             const float p0 = ex2(s0 - na), p1 = ex2(s1 - nb), p2 = ex2(s2 - na), p3 = ex2(s3 - nb);
             l_a[nt] = l_a[nt] * alpha_a + p0 + p2;
             l_b[nt] = l_b[nt] * alpha_b + p1 + p3;
-            // P = high + low, both in T
-            const uint32_t h0 = pack_pair<T>(p0, p1), h1 = pack_pair<T>(p2, p3);
-            const float2 f0 = unpack_pair<T>(h0), f1 = unpack_pair<T>(h1);
-            ph[nt][0] = movmatrix_trans(h0);
-            ph[nt][1] = movmatrix_trans(h1);
-            pl[nt][0] = movmatrix_trans(pack_pair<T>(p0 - f0.x, p1 - f0.y));
-            pl[nt][1] = movmatrix_trans(pack_pair<T>(p2 - f1.x, p3 - f1.y));
+            uint32_t w0[P::kCount], w1[P::kCount];
+            P::split(p0, p1, w0);
+            P::split(p2, p3, w1);
+#pragma unroll
+            for (int e = 0; e < P::kCount; ++e) {
+                pp[nt][e][0] = movmatrix_trans(w0[e]);
+                pp[nt][e][1] = movmatrix_trans(w1[e]);
+            }
             if (__any_sync(0xffffffffu, alpha_a != 1.f || alpha_b != 1.f)) {
 #pragma unroll
-                for (int j = 0; j < D / 16; ++j) {
-                    acc[nt][j][0] *= alpha_a;
-                    acc[nt][j][1] *= alpha_b;
-                    acc[nt][j][2] *= alpha_a;
-                    acc[nt][j][3] *= alpha_b;
-                }
+                for (int a = 0; a < P::kAccs; ++a)
+#pragma unroll
+                    for (int j = 0; j < D / 16; ++j) {
+                        acc[nt][a][j][0] *= alpha_a;
+                        acc[nt][a][j][1] *= alpha_b;
+                        acc[nt][a][j][2] *= alpha_a;
+                        acc[nt][a][j][3] *= alpha_b;
+                    }
             }
         }
         if (masked && i + 1 < n_w) load_mask(i + 1);
@@ -394,10 +438,9 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attn_decode16_kernel(const Dec
             uint32_t a[4];
             ldmatrix4_trans(sV + row * kRowBytes + ((col ^ (row & 7)) << 4), a);
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt) {
-                mma16816<T>(acc[nt][j], a, ph[nt][0], ph[nt][1]);
-                mma16816<T>(acc[nt][j], a, pl[nt][0], pl[nt][1]);
-            }
+            for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                for (int e = 0; e < P::kCount; ++e) mma16816<T>(acc[nt][e < P::kAccs ? e : P::kAccs - 1][j], a, pp[nt][e][0], pp[nt][e][1]);
         }
         __syncwarp();  // every lane is done with this stage before it is refilled
     }
@@ -417,16 +460,22 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attn_decode16_kernel(const Dec
         const int ra = nt * 8 + 2 * tid4, rb = ra + 1;
 #pragma unroll
         for (int j = 0; j < D / 16; ++j) {  // accumulator rows: d = 16 j + gid, + 8; columns: rows a, b
-            wbuf[ra * D + 16 * j + gid] = acc[nt][j][0];
-            wbuf[rb * D + 16 * j + gid] = acc[nt][j][1];
-            wbuf[ra * D + 16 * j + gid + 8] = acc[nt][j][2];
-            wbuf[rb * D + 16 * j + gid + 8] = acc[nt][j][3];
+            float o[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                o[i] = acc[nt][0][j][i];
+                if constexpr (P::kAccs == 2) o[i] = fmaf(acc[nt][1][j][i], P::kLowScale, o[i]);
+            }
+            wbuf[ra * D + 16 * j + gid] = o[0];
+            wbuf[rb * D + 16 * j + gid] = o[1];
+            wbuf[ra * D + 16 * j + gid + 8] = o[2];
+            wbuf[rb * D + 16 * j + gid + 8] = o[3];
         }
-        if (gid == 0) {
+        if (gid == 0) {  // (f16: O carries the pieces' factor, so the sums do too)
             wbuf[GP * D + ra] = m_a[nt];
             wbuf[GP * D + rb] = m_b[nt];
-            wbuf[GP * D + GP + ra] = l_a[nt];
-            wbuf[GP * D + GP + rb] = l_b[nt];
+            wbuf[GP * D + GP + ra] = l_a[nt] * P::kSumScale;
+            wbuf[GP * D + GP + rb] = l_b[nt] * P::kSumScale;
         }
     }
     __syncthreads();

@@ -114,3 +114,34 @@ def test_sixteen_bit_pool(b2a, dtype, hq, hkv, d, bs):
     out = b2a.paged_attention(q.cuda(), cache, t[0], t[1], torch.from_numpy(bad).cuda(), t[3], hq=hq, max_context_len=4096,
                               max_q_len=33, status=status)
     assert int(status.item()) & 2 and torch.isfinite(out.float()).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("sq,d", [(1, 128), (1, 64), (12, 128)])
+@pytest.mark.parametrize("gap", [10.0, 16.0, 17.4, 20.0])
+def test_many_keys_far_below_one(b2a, dtype, sq, d, gap):
+    # an attention sink: one key with a zero value row stands `gap` above 32768 equal ones, whose values are the result.
+    # Their probabilities lie down to 2^-29 below the maximum, under f16's smallest value times 2^-4.  Bounds: the rounding of
+    # the result (half a unit in the last place, 2^-25 where f16 has no smaller step; twice that is allowed), beside which the
+    # 2^-20 of exponentials and split vanish.
+    n = 32768
+    q, k, v = torch.zeros(1, 2, sq, d), torch.zeros(1, 2, n, d), torch.ones(1, 2, n, d)
+    q[..., 0], k[:, :, 5, 0], v[:, :, 5] = 1.0, gap, 0.0
+    q, k, v = q.to(dtype), k.to(dtype), v.to(dtype)
+    out = b2a.sdpa(q.cuda(), k.cuda(), v.cuda(), scale=1.0)
+    np.testing.assert_allclose(out.float().cpu().numpy(), osdpa.sdpa_ref(q, k, v, scale=1.0), atol=2.0 ** -24,
+                               rtol=2.0 ** -10 if dtype == torch.float16 else 2.0 ** -8)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("sq,d,n", [(1, 128, 100), (4, 64, 333), (12, 128, 3000)])
+def test_an_infinity_in_the_values_stays_one(b2a, dtype, sq, d, n):
+    q, k, v = _rand((1, 2, sq, d), 1, dtype), _rand((1, 2, n, d), 2, dtype), _rand((1, 2, n, d), 3, dtype)
+    v[0, 0, 7, 3], v[0, 1, n - 1, d - 1] = float("inf"), float("-inf")
+    out = b2a.sdpa(q.cuda(), k.cuda(), v.cuda()).float().cpu()
+    assert (out[0, 0, :, 3] == float("inf")).all() and (out[0, 1, :, d - 1] == float("-inf")).all()
+    v[0, 0, 7, 3] = v[0, 1, n - 1, d - 1] = 0.0
+    out[0, 0, :, 3] = out[0, 1, :, d - 1] = 0.0
+    ref = osdpa.sdpa_ref(q, k, v)
+    ref[0, 0, :, 3] = ref[0, 1, :, d - 1] = 0.0
+    _check(out, ref, dtype)

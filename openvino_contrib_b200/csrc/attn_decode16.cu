@@ -13,7 +13,7 @@
 // (A workspace would have to be asked of callers that never needed one, and a merge kernel costs a launch.)
 //
 // The probabilities keep float32's precision and, as far as a row can tell, its range: they enter the second product as two
-// f16 or three bf16 values (Pieces), which costs eight or sixteen more MMAs per tile where the tensor pipe idles anyway.
+// f16 or three bf16 values (ProbPieces), which costs eight or sixteen more MMAs per tile where the tensor pipe idles anyway.
 //
 // Measured on a B200 (graph replay): bf16, 8 sequences x 3003 keys x 8 KV heads, additive mask (98 MB): 2049 us on
 // attn_generic_kernel before, 23.3 us now (4.2 TB/s; 15.1 us at the copy rate); 32 bf16 sequences of 256..4096 tokens in
@@ -124,42 +124,12 @@ __device__ __forceinline__ float2 unpack_pair<__nv_bfloat16>(uint32_t w) {
     return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
 }
 
-// Two probabilities as packed pieces of T.
-//   f16: p 2^14 = hi + lo 2^-11, eleven bits each, and lo in an accumulator of its own: with one scale for both, the
-//     probabilities of many keys beside one that stands far above them fall below f16's smallest value (32768 equal keys 17.4
-//     below one with a zero value row: 3 % off).  Here 2^-49 of the maximum still counts.
-//   bf16: p = hi + mid + lo, eight bits each.
-// Every piece but the last is cut from a value a little below what is left, so that all are above zero wherever p is (f16:
-// above 2^-37): an infinity in V then stays one in the sum of the products, where a piece of zero or below would make it NaN.
+// Factor on the probabilities before they are cut into pieces (ProbPieces), carried by the row sum: f16's pieces reach down to
+// 2^-49 of the row's maximum with it.
 template <typename T>
-struct Pieces;
+constexpr float kPieceScale = 1.f;
 template <>
-struct Pieces<__half> {
-    static constexpr int kCount = 2, kAccs = 2;  // pieces; accumulators (piece e goes to the e-th or the last of them)
-    static constexpr float kSumScale = 16384.f, kLowScale = 1.f / 2048.f;
-    static __device__ __forceinline__ void split(float p0, float p1, uint32_t (&w)[2]) {
-        p0 *= 16384.f;
-        p1 *= 16384.f;
-        asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(w[0]) : "f"(p1 * (1.f - 1.f / 8192.f)), "f"(p0 * (1.f - 1.f / 8192.f)));
-        const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&w[0]));
-        const __half2 l = __floats2half2_rn((p0 - h.x) * 2048.f, (p1 - h.y) * 2048.f);
-        w[1] = *reinterpret_cast<const uint32_t*>(&l);
-    }
-};
-template <>
-struct Pieces<__nv_bfloat16> {
-    static constexpr int kCount = 3, kAccs = 1;
-    static constexpr float kSumScale = 1.f;
-    static __device__ __forceinline__ void split(float p0, float p1, uint32_t (&w)[3]) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            w[e] = __byte_perm(__float_as_uint(p0 * (1.f - 1.f / 1024.f)), __float_as_uint(p1 * (1.f - 1.f / 1024.f)), 0x7632);
-            p0 -= __uint_as_float(w[e] << 16);
-            p1 -= __uint_as_float(w[e] & 0xffff0000u);
-        }
-        w[2] = pack_pair<__nv_bfloat16>(p0, p1);
-    }
-};
+constexpr float kPieceScale<__half> = 16384.f;
 
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
@@ -353,7 +323,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attn_decode16_kernel(const Dec
     for (int nt = 0; nt < NT; ++nt) mv[nt][0] = mv[nt][1] = mv[nt][2] = mv[nt][3] = 0.f;
     if (masked && n_w > 0) load_mask(0);
 
-    using P = Pieces<T>;
+    using P = ProbPieces<T>;
     float acc[NT][P::kAccs][D / 16][4];
     float m_a[NT], m_b[NT], l_a[NT], l_b[NT];
 #pragma unroll
@@ -411,8 +381,8 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attn_decode16_kernel(const Dec
             l_a[nt] = l_a[nt] * alpha_a + p0 + p2;
             l_b[nt] = l_b[nt] * alpha_b + p1 + p3;
             uint32_t w0[P::kCount], w1[P::kCount];
-            P::split(p0, p1, w0);
-            P::split(p2, p3, w1);
+            P::split(p0 * kPieceScale<T>, p1 * kPieceScale<T>, w0);
+            P::split(p2 * kPieceScale<T>, p3 * kPieceScale<T>, w1);
 #pragma unroll
             for (int e = 0; e < P::kCount; ++e) {
                 pp[nt][e][0] = movmatrix_trans(w0[e]);
@@ -474,8 +444,8 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attn_decode16_kernel(const Dec
         if (gid == 0) {  // (f16: O carries the pieces' factor, so the sums do too)
             wbuf[GP * D + ra] = m_a[nt];
             wbuf[GP * D + rb] = m_b[nt];
-            wbuf[GP * D + GP + ra] = l_a[nt] * P::kSumScale;
-            wbuf[GP * D + GP + rb] = l_b[nt] * P::kSumScale;
+            wbuf[GP * D + GP + ra] = l_a[nt] * kPieceScale<T>;
+            wbuf[GP * D + GP + rb] = l_b[nt] * kPieceScale<T>;
         }
     }
     __syncthreads();

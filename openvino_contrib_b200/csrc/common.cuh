@@ -59,6 +59,53 @@ __host__ __device__ __forceinline__ size_t u8_chunk_bytes(int block_size, int d)
 
 constexpr float kLog2e = 1.4426950408889634f;
 
+// Two probabilities as packed pieces of T, for a second product on the tensor core that keeps float32's precision.
+//   f16: p = hi + lo 2^-11, eleven bits each, and lo in an accumulator of its own: with one scale for both, the
+//     probabilities of many keys beside one that stands far above them fall below f16's smallest value (32768 equal keys 17.4
+//     below one with a zero value row: 3 % off).  The caller scales p by a power of two, to 2^15 at most, which its row sum
+//     carries too; what counts then reaches down to 2^-35 of the value one.
+//   bf16: p = hi + mid + lo, eight bits each.
+// Every piece but the last is cut from a value a little below what is left, so that all are above zero wherever p is (f16:
+// above 2^-23): an infinity in V then stays one in the sum of the products, where a piece of zero or below would make it NaN.
+template <typename T>
+struct ProbPieces;
+template <>
+struct ProbPieces<__half> {
+    static constexpr int kCount = 2, kAccs = 2;  // pieces; accumulators (piece e goes to the e-th or the last of them)
+    static constexpr float kLowScale = 1.f / 2048.f;
+    static __device__ __forceinline__ void split(float p0, float p1, uint32_t (&w)[2]) {
+        // (two lanes an instruction; the remainder (p - hi) 2^11 is exact in this order of operations too)
+        uint64_t p, below, rest;
+        float b0, b1;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(p0), "f"(p1));
+        asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(below) : "l"(p), "l"(0x3f7ff8003f7ff800ull));  // 1 - 2^-13
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(b0), "=f"(b1) : "l"(below));
+        asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(w[0]) : "f"(b1), "f"(b0));
+        const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&w[0]));
+        uint64_t hi;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(hi) : "f"(h.x), "f"(h.y));
+        asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(rest) : "l"(p), "l"(0x4500000045000000ull));             // 2^11
+        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(rest) : "l"(hi), "l"(0xc5000000c5000000ull), "l"(rest));
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(b0), "=f"(b1) : "l"(rest));
+        const __half2 l = __floats2half2_rn(b0, b1);
+        w[1] = *reinterpret_cast<const uint32_t*>(&l);
+    }
+};
+template <>
+struct ProbPieces<__nv_bfloat16> {
+    static constexpr int kCount = 3, kAccs = 1;
+    static __device__ __forceinline__ void split(float p0, float p1, uint32_t (&w)[3]) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            w[e] = __byte_perm(__float_as_uint(p0 * (1.f - 1.f / 1024.f)), __float_as_uint(p1 * (1.f - 1.f / 1024.f)), 0x7632);
+            p0 -= __uint_as_float(w[e] << 16);
+            p1 -= __uint_as_float(w[e] & 0xffff0000u);
+        }
+        const __nv_bfloat162 l = __floats2bfloat162_rn(p0, p1);
+        w[2] = *reinterpret_cast<const uint32_t*>(&l);
+    }
+};
+
 // Programmatic dependent launch: a kernel launched with launch_overlapped may be scheduled while the kernel before
 // it on the stream is still running (as soon as that one has executed grid_launch_dependents in every CTA, or has
 // finished), so that its launch latency and set-up hide behind the predecessor's tail.  It must call

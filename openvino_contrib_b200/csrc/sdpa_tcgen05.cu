@@ -488,12 +488,14 @@ __global__ void __launch_bounds__(128) paged_gather_kernel(const PagedTables t, 
 //   3 boolean and 4 additive, the same for all rows (row stride 0: a padding mask), read once per warp, any key stride
 //   and alignment; 5 either kind with any strides, element by element.
 // kDim: head size, 64 or 128.
-// kSplitP: P enters the second product as the sum of two 16-bit values - hi = round(p), lo = round(p - hi), kept in the two
-//   halves of S's columns - so that these calls lose nothing against the float32 probabilities of attn_generic_kernel.  It
-//   costs half as many second products again (the tensor pipe idles behind the exponentials anyway) and about five
-//   instructions per pair of probabilities.  Bound: the special-function unit, 128 exponentials per row and step; the
-//   f16 encoder batch of 8 x 16 heads x 512 tokens, head size 64, boolean padding mask: 1167 us in attn_generic_kernel,
-//   28.7 us here (5.1 us of memory traffic at the copy rate).
+// kSplitP: P enters the second product as several 16-bit values (ProbPieces in common.cuh), so that these calls keep the
+//   precision of attn_generic_kernel's float32 probabilities: 22 bits in f16, 24 in bf16.  Two pieces lie in the two halves of S's
+//   columns; the second product of f16's low one has an accumulator of its own, bf16's third piece columns of its own, both
+//   `kDim` columns behind O_X.  With a head size of 128 that is tile B's place: an item is then ONE tile.  It costs one or two
+//   times as many second products again (the tensor pipe idles behind the exponentials anyway) and six to eight instructions
+//   per pair of probabilities.  Bound: the special-function unit, 128 exponentials per row and step; the f16 encoder batch
+//   of 8 x 16 heads x 512 tokens, head size 64, boolean padding mask: 1167 us in attn_generic_kernel, 27.1 us here (5.1 us
+//   of memory traffic at the copy rate).
 // kKeySplit (dense): a small problem - fewer pairs of tiles than SMs - is bound by its longest chain of key steps, one tile's
 //   softmax after the other's.  Then an item is ONE tile whose keys are shared out: "tile A" takes the first half of its key
 //   tiles, "tile B" the second, each with its own maximum, sum and accumulator, which are merged in the epilogue (the two
@@ -507,6 +509,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                const __grid_constant__ CUtensorMap tmV, const TcParams p, const __grid_constant__ TcPeers peers) {
     static_assert(kDim == kHeadDim || kMode == 0, "the paged modes are built for a head size of 128");
     static_assert(!kKeySplit || kMode == 0, "the keys of a tile are shared out in dense mode only");
+    static_assert(!kSplitP || kMode == 0, "the paged modes hold P in 16 bits");
+    constexpr bool kSingle = kSplitP && kDim == kHeadDim;  // an item is one tile: the pieces of P need tile B's columns
+    static_assert(!(kSingle && kKeySplit), "no columns for the other half of the keys");
     constexpr int kTile = 128 * kDim * 2;  // bytes of a [128 x kDim] 16-bit tile: kDim / 64 panels
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -520,6 +525,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     auto BAR = [&](int i) { return bars + 8u * static_cast<uint32_t>(i); };
     constexpr bool kPaged = kMode != 0, kDequant = kMode == 1, kGathered = kMode == 2;
     constexpr bool kKvBf16 = kPaged ? false : kBf16;  // element format of the K/V tiles and of P
+    using Pieces = ProbPieces<std::conditional_t<kKvBf16, __nv_bfloat16, __half>>;
+    constexpr bool kLowAcc = kSplitP && Pieces::kAccs == 2;      // O = O_X + kLowScale * (what lies kDim columns on)
+    constexpr bool kThirdPiece = kSplitP && Pieces::kCount == 3;  // kDim columns behind O_X
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if constexpr (kDequant) {  // the grid is only a bound on the number of items: CTAs without one set nothing up
@@ -631,8 +639,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             }
         };
         int firstA, firstB;
-        tile_of(2 * pair, it.row0A, it.headA, it.nkvA, firstA);
-        tile_of(2 * pair + 1, it.row0B, it.headB, it.nkvB, firstB);
+        tile_of(kSingle ? pair : 2 * pair, it.row0A, it.headA, it.nkvA, firstA);
+        tile_of(kSingle ? tiles : 2 * pair + 1, it.row0B, it.headB, it.nkvB, firstB);
         it.kv_tile0 = 0;
         if constexpr (kPaged) {
             // the two tiles walk the same key tiles: both start at the earlier of their first ones (a tile that starts
@@ -687,7 +695,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         causal = p.causal != 0;
         nrb = (nrows_total + kBM - 1) / kBM;
         tiles = nrb * p.G;
-        pairs = (tiles + 1) / 2;
+        pairs = kSingle ? tiles : (tiles + 1) / 2;
         total_items = pairs * p.B * p.Hkv;  // the launcher keeps this below 2^31
     }
 
@@ -944,10 +952,17 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 #define B2A_PV(ks, accv) mma_ts_c<(ks) * 8, ((ks) * 2048) / 16, kLoV, kHiV, idesc_pv>(d, pa, va, accv)
                 B2A_PV(0, acc ? 1u : 0u); B2A_PV(1, 1u); B2A_PV(2, 1u); B2A_PV(3, 1u);
 #undef B2A_PV
-                if constexpr (kSplitP) {  // the low halves of the same probabilities, 64 columns on
-#define B2A_PVLO(ks) mma_ts_c<64 + (ks) * 8, ((ks) * 2048) / 16, kLoV, kHiV, idesc_pv>(d, pa, va, 1u)
-                    B2A_PVLO(0); B2A_PVLO(1); B2A_PVLO(2); B2A_PVLO(3);
+                if constexpr (kSplitP) {  // the second pieces of the same probabilities, 64 columns on
+                    const uint32_t dl = kLowAcc ? d + kDim : d;
+#define B2A_PVLO(ks, accv) mma_ts_c<64 + (ks) * 8, ((ks) * 2048) / 16, kLoV, kHiV, idesc_pv>(dl, pa, va, accv)
+                    B2A_PVLO(0, acc || !kLowAcc ? 1u : 0u); B2A_PVLO(1, 1u); B2A_PVLO(2, 1u); B2A_PVLO(3, 1u);
 #undef B2A_PVLO
+                }
+                if constexpr (kThirdPiece) {
+                    const uint32_t pt = d + kDim + static_cast<uint32_t>(half * 32);
+#define B2A_PV3(ks) mma_ts_c<(ks) * 8, ((ks) * 2048) / 16, kLoV, kHiV, idesc_pv>(d, pt, va, 1u)
+                    B2A_PV3(0); B2A_PV3(1); B2A_PV3(2); B2A_PV3(3);
+#undef B2A_PV3
                 }
             };
             bool ok = true;
@@ -1063,6 +1078,17 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
         const uint32_t tS = tmem + lane_base + static_cast<uint32_t>(X * 128);
         const uint32_t tO = tmem + lane_base + static_cast<uint32_t>(256 + X * 128);
+        // 32 columns of an accumulator
+        auto load_o = [&](uint32_t t, int q, uint32_t (&o)[32]) {
+            tmem_ld32(t + 32 * q, o);
+            if constexpr (kLowAcc) {
+                uint32_t low[32];
+                tmem_ld32(t + kDim + 32 * q, low);
+                tmem_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(fmaf(__uint_as_float(low[i]), Pieces::kLowScale, __uint_as_float(o[i])));
+            }
+        };
         int sxb = 0;  // steps of this tile in the CTA's earlier items: every per-step barrier is at phase (sxb + j)
         bool ok = true;
         Item item;
@@ -1094,10 +1120,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                                     (kMask == 1 || kMask == 3 || (kMask == 5 && p.mask_kind == B2A_MASK_BOOL) ? 1 : 2);
             // kMask 4: this warp's 128 mask values of a step, as floats, at the start of its staging slab
             float* mslab = reinterpret_cast<float*>(gbase + 6 * kTile + warp * 4096);
-            if constexpr (kMask == 4) {
-                if (lane == 0) tma_store_wait_read();  // the previous item's store has read the slab
-                __syncwarp();
-            }
             for (int j = 0; j < nkv; ++j) {
                 uint32_t mword[4];  // kMask 3: bit i of word q keeps key 32 q + i of the step
                 if constexpr (kMask == 3) {
@@ -1245,12 +1267,14 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                     m_used = m_new;
                     l *= alpha;
                 }
-                // P = exp2(S*c - m): the scale-and-shift and the row sum run two elements per instruction (f32x2)
-                const uint64_t c2 = f2_pack(c, c), nm2 = f2_pack(-m_used, -m_used);
+                // P = exp2(S*c - m): the scale-and-shift and the row sum run two elements per instruction (f32x2).  (f16 in
+                // pieces: 2^7 P, at most 2^15, so that the pieces reach as far down as they can; the sum carries the factor too)
+                const float shift = kLowAcc ? 7.f - m_used : -m_used;
+                const uint64_t c2 = f2_pack(c, c), nm2 = f2_pack(shift, shift);
                 uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    uint32_t pk[16], pk_lo[16];
+                    uint32_t pk[16], pk_lo[16], pk_third[16];
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
                         const uint64_t x2 = f2_fma(f2_pack(__uint_as_float(s[q][2 * i]), __uint_as_float(s[q][2 * i + 1])), c2, nm2);
@@ -1258,15 +1282,19 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                         f2_unpack(x2, x0, x1);
                         const float p0 = ex2f(x0), p1 = ex2f(x1);
                         sum2[i & 3] = f2_add(sum2[i & 3], f2_pack(p0, p1));
-                        pk[i] = pack2<kKvBf16>(p0, p1);
                         if constexpr (kSplitP) {
-                            float h0, h1;
-                            unpack2<kKvBf16>(pk[i], h0, h1);
-                            pk_lo[i] = pack2<kKvBf16>(p0 - h0, p1 - h1);
+                            uint32_t w[Pieces::kCount];
+                            Pieces::split(p0, p1, w);
+                            pk[i] = w[0];
+                            pk_lo[i] = w[1];
+                            if constexpr (kThirdPiece) pk_third[i] = w[2];
+                        } else {
+                            pk[i] = pack2<kKvBf16>(p0, p1);
                         }
                     }
                     tmem_st16(tS + 16 * q, pk);  // P over the first 64 columns of S, behind what was already read
                     if constexpr (kSplitP) tmem_st16(tS + 64 + 16 * q, pk_lo);  // (all of S is in registers by now)
+                    if constexpr (kThirdPiece) tmem_st16(tO + kDim + 16 * q, pk_third);
                     // first 64 keys of P are in TMEM: PV can start on them, unless O still has to be rescaled
                     if (q == 1 && !(need_any && j > 0)) {
                         tmem_wait_st();
@@ -1285,7 +1313,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                     if (!ok) break;
                     tc_fence_after();
 #pragma unroll
-                    for (int q = 0; q < kDim / 32; ++q) {
+                    for (int q = 0; q < (kLowAcc ? 2 : 1) * kDim / 32; ++q) {
                         uint32_t o[32];
                         tmem_ld32(tO + 32 * q, o);
                         tmem_wait_ld();
@@ -1343,10 +1371,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                     for (int q = 0; q < kDim / 32; ++q) {
                         if (both && (q / (kDim / 64)) != X) continue;  // the other warp's columns
                         uint32_t o[32], w[16];
-                        tmem_ld32(tO + 32 * q, o);
+                        load_o(tO, q, o);
                         if (both) {
                             uint32_t o2[32];
-                            tmem_ld32(tOther + 32 * q, o2);
+                            load_o(tOther, q, o2);
                             tmem_wait_ld();
 #pragma unroll
                             for (int i = 0; i < 32; ++i)
@@ -1396,7 +1424,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 #pragma unroll
                     for (int q = 0; q < kDim / 32; ++q) {
                         uint32_t o[32], w[16];
-                        tmem_ld32(tO + 32 * q, o);
+                        load_o(tO, q, o);
                         tmem_wait_ld();
 #pragma unroll
                         for (int i = 0; i < 16; ++i)
@@ -1639,7 +1667,8 @@ int sdpa_tc_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t
     p.scale_log2 = d.scale * kLog2e;
     p.status = status;
     const int nrb = (d.Sq + kBM - 1) / kBM;
-    const int pairs = (nrb * p.G + 1) / 2;
+    const bool single = split_p && d.D == kHeadDim;  // (kSingle)
+    const int pairs = single ? nrb * p.G : (nrb * p.G + 1) / 2;
     const long long items = static_cast<long long>(pairs) * d.B * d.Hkv;
     if (items >= (1LL << 30)) return B2A_ERR_UNSUPPORTED;
     const int sms = device_sm_count();

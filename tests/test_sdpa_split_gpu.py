@@ -106,3 +106,38 @@ def test_precision_is_that_of_float32_probabilities(b2a):
     # rounding the result errs by at most 2^-11 of each value and, spread evenly over that, by 2^-11 / sqrt(3) times at most
     # 1 / sqrt(2)..1 of it in the 2-norm: below 2^-11.8 in all.  Probabilities in f16 alone would add their own 2^-12.3.
     assert float((out - ref).norm() / ref.norm()) < 2.0 ** -11.8
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("heads,sq,d,mask", [(2, 140, 64, "none"), (160, 140, 64, "none"), (2, 140, 64, "keys"), (2, 140, 64, "rows"),
+                                             (2, 140, 128, "keys"), (2, 140, 128, "rows")])
+@pytest.mark.parametrize("gap", [10.0, 16.0, 17.4, 20.0])
+def test_many_keys_far_below_one(b2a, dtype, heads, sq, d, mask, gap):
+    # an attention sink: one key with a zero value row stands `gap` above thousands of equal ones, whose values are the result.
+    # Their probabilities lie down to 2^-29 below the maximum, under f16's smallest value times 2^-4.  Bounds: the rounding of
+    # the result (half a unit in the last place, 2^-25 where f16 has no smaller step; twice that is allowed), beside which the
+    # 2^-14 of exponentials and split vanish.  (160 heads: pairs of tiles; 2: their keys shared out)
+    n = 2047 if heads > 2 else 32767
+    q, k, v = torch.zeros(1, heads, sq, d), torch.zeros(1, heads, n, d), torch.ones(1, heads, n, d)
+    q[..., 0], k[:, :, 5, 0], v[:, :, 5] = 1.0, gap, 0.0
+    q, k, v = q.to(dtype), k.to(dtype), v.to(dtype)
+    m = None if mask == "none" else torch.zeros(1, 1, 1 if mask == "keys" else sq, n, dtype=dtype)
+    out = b2a.sdpa(q.cuda(), k.cuda(), v.cuda(), None if m is None else m.cuda(), scale=1.0)
+    ref = osdpa.sdpa_ref(q[:, :2, :1], k[:, :2], v[:, :2], scale=1.0)
+    np.testing.assert_allclose(out.float().cpu().numpy(), np.broadcast_to(ref[:, :1], out.shape), atol=2.0 ** -24,
+                               rtol=2.0 ** -10 if dtype == torch.float16 else 2.0 ** -8)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("d,n,masked", [(64, 128, False), (64, 333, False), (64, 333, True), (128, 333, True)])
+def test_an_infinity_in_the_values_stays_one(b2a, dtype, d, n, masked):
+    q, k, v = _rand((1, 2, 150, d), 1, dtype), _rand((1, 2, n, d), 2, dtype), _rand((1, 2, n, d), 3, dtype)
+    v[0, 0, 7, 3], v[0, 1, n - 1, d - 1] = float("inf"), float("-inf")
+    m = torch.ones(1, 1, 1, n, dtype=torch.bool) if masked else None
+    out = b2a.sdpa(q.cuda(), k.cuda(), v.cuda(), None if m is None else m.cuda()).float().cpu()
+    assert (out[0, 0, :, 3] == float("inf")).all() and (out[0, 1, :, d - 1] == float("-inf")).all()
+    v[0, 0, 7, 3] = v[0, 1, n - 1, d - 1] = 0.0
+    out[0, 0, :, 3] = out[0, 1, :, d - 1] = 0.0
+    ref = osdpa.sdpa_ref(q, k, v)
+    ref[0, 0, :, 3] = ref[0, 1, :, d - 1] = 0.0
+    _check(out, ref, dtype)

@@ -1632,8 +1632,11 @@ int sdpa_tc_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t
                    cudaStream_t stream, const TcPeerOut* peer_out, const void* mask, bool split_p) {
     const bool bf16 = d.dtype == B2A_BF16;
     CUtensorMap mq, mk, mv;
-    if (!make_map(&mq, q, bf16, d.B, d.Hq, d.Sq, qs, 128, d.D) || !make_map(&mk, k, bf16, d.B, d.Hkv, d.Skv, ks, 128, d.D) ||
-        !make_map(&mv, v, bf16, d.B, d.Hkv, d.Skv, vs, 128, d.D))
+    // A causal row sees at most Sq keys: what lies behind (a cache's unfilled rows, which may hold NaN) comes in as zeros, like
+    // everything outside a map.
+    const int keys = d.causal ? std::min(d.Skv, d.Sq) : d.Skv;
+    if (!make_map(&mq, q, bf16, d.B, d.Hq, d.Sq, qs, 128, d.D) || !make_map(&mk, k, bf16, d.B, d.Hkv, keys, ks, 128, d.D) ||
+        !make_map(&mv, v, bf16, d.B, d.Hkv, keys, vs, 128, d.D))
         return B2A_ERR_CUDA;
     TcPeers peers{};
     if (peer_out != nullptr) {
@@ -1652,7 +1655,7 @@ int sdpa_tc_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t
         peers.light_first = peer_out->world >= 4 ? 1 : 0;
     }
     TcParams p{};
-    p.B = d.B; p.Hq = d.Hq; p.Hkv = d.Hkv; p.G = d.Hq / d.Hkv; p.Sq = d.Sq; p.Skv = d.Skv;
+    p.B = d.B; p.Hq = d.Hq; p.Hkv = d.Hkv; p.G = d.Hq / d.Hkv; p.Sq = d.Sq; p.Skv = keys;
     p.div_g = fast_div(p.G);
     p.div_hkv = fast_div(p.Hkv);
     p.div_streams = fast_div(p.B * p.Hkv);
@@ -1689,13 +1692,13 @@ int sdpa_tc_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t
     // (Sharded launches follow the same rule: their output is the unsharded kernel's, bit for bit.)
     bool key_split = false;
     const long long streams = static_cast<long long>(d.B) * d.Hkv, all_tiles = streams * nrb * p.G;
-    const int n = ((d.causal ? std::min(d.Skv, nrb * kBM) : d.Skv) + kBN - 1) / kBN, half = (n + 1) / 2;
+    const int n = (keys + kBN - 1) / kBN, half = (n + 1) / 2;
     if (items <= sms && (n <= 16 || 2 * all_tiles <= sms)) {
         const long long rounds = (all_tiles + sms - 1) / sms;
         double steps = static_cast<double>(rounds * half);
         if (d.causal) {
             long long halves = 0;
-            for (int rb = 0; rb < nrb; ++rb) halves += ((std::min(d.Skv, (rb + 1) * kBM) + kBN - 1) / kBN + 1) / 2;
+            for (int rb = 0; rb < nrb; ++rb) halves += ((std::min(keys, (rb + 1) * kBM) + kBN - 1) / kBN + 1) / 2;
             steps = std::max<double>(half, static_cast<double>(halves * p.G * streams) / sms);
         }
         key_split = steps + (rounds > 1 ? 1.5 : 0.0) < n;

@@ -141,3 +141,15 @@ def test_an_infinity_in_the_values_stays_one(b2a, dtype, d, n, masked):
     ref = osdpa.sdpa_ref(q, k, v)
     ref[0, 0, :, 3] = ref[0, 1, :, d - 1] = 0.0
     _check(out, ref, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("heads,sq,skv,d", [(2, 140, 300, 64), (100, 140, 300, 64), (2, 140, 300, 128), (100, 140, 300, 128),
+                                            (2, 129, 130, 64), (2, 4, 60, 128)])
+def test_causal_reads_no_key_beyond_the_queries(b2a, dtype, heads, sq, skv, d):
+    # the unfilled rows of a cache hold anything: causal attention stops at key Sq - 1
+    q, k, v = _rand((1, heads, sq, d), 1, dtype), _rand((1, heads, skv, d), 2, dtype), _rand((1, heads, skv, d), 3, dtype)
+    k[:, :, sq:] = float("nan")
+    v[:, :, sq:] = float("nan")
+    out = b2a.sdpa(q.cuda(), k.cuda(), v.cuda(), causal=True)
+    assert torch.equal(out, b2a.sdpa(q.cuda(), k[:, :, :sq].contiguous().cuda(), v[:, :, :sq].contiguous().cuda(), causal=True))

@@ -369,12 +369,14 @@ __device__ __forceinline__ void unpack2(uint32_t w, float& lo, float& hi) {
 // One value of an additive mask, in log2 units.  Finite values end at kMaskFloor (the lowest bf16 times log2(e) would
 // overflow): a row whose keys all carry the type's lowest value stays uniform over them, as in attn_generic_kernel.
 constexpr float kMaskFloor = -1.0e30f;
+__device__ __forceinline__ float mask_log2(float f) {
+    const float v = f * kLog2e;
+    return v < kMaskFloor && f != -INFINITY ? kMaskFloor : v;
+}
 template <bool kBf16>
 __device__ __forceinline__ float mask_log2(const uint8_t* row, int64_t at) {
     const uint16_t bits = reinterpret_cast<const uint16_t*>(row)[at];
-    const float f = kBf16 ? __uint_as_float(static_cast<uint32_t>(bits) << 16) : __half2float(__ushort_as_half(bits));
-    const float v = f * kLog2e;
-    return v < kMaskFloor && f != -INFINITY ? kMaskFloor : v;
+    return mask_log2(kBf16 ? __uint_as_float(static_cast<uint32_t>(bits) << 16) : __half2float(__ushort_as_half(bits)));
 }
 // time-bounded wait that ignores the abort flag: used only to drain work already in flight
 __device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
@@ -1217,8 +1219,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                                     float lo, hi;
                                     unpack2<kBf16>(w[i], lo, hi);
                                     const int e = 8 * h + 2 * i;
-                                    s[q][e] = __float_as_uint(fmaf(__uint_as_float(s[q][e]), c, lo * kLog2e));
-                                    s[q][e + 1] = __float_as_uint(fmaf(__uint_as_float(s[q][e + 1]), c, hi * kLog2e));
+                                    s[q][e] = __float_as_uint(fmaf(__uint_as_float(s[q][e]), c, mask_log2(lo)));
+                                    s[q][e + 1] = __float_as_uint(fmaf(__uint_as_float(s[q][e + 1]), c, mask_log2(hi)));
                                 }
                             }
                         }

@@ -153,3 +153,15 @@ def test_causal_reads_no_key_beyond_the_queries(b2a, dtype, heads, sq, skv, d):
     v[:, :, sq:] = float("nan")
     out = b2a.sdpa(q.cuda(), k.cuda(), v.cuda(), causal=True)
     assert torch.equal(out, b2a.sdpa(q.cuda(), k[:, :, :sq].contiguous().cuda(), v[:, :, :sq].contiguous().cuda(), causal=True))
+
+
+@pytest.mark.parametrize("skv", [200, 201, 1000])
+@pytest.mark.parametrize("rows", [1, 140])
+def test_the_lowest_value_in_every_place_is_an_average(b2a, skv, rows):
+    # bf16's lowest value times log2(e) is not finite; nothing of the scores is left, whatever form reads the mask
+    q, k, v = (_rand((2, 4, n, 128), s, torch.bfloat16) for n, s in ((140, 1), (skv, 2), (skv, 3)))
+    m = torch.full((2, 1, rows, skv), torch.finfo(torch.bfloat16).min, dtype=torch.bfloat16)
+    m[1, :, :, :150] = float("-inf")
+    out = b2a.sdpa(q.cuda(), k.cuda(), v.cuda(), m.cuda())
+    for i, lo in ((0, 0), (1, 150)):
+        _check(out[i], v[i, :, lo:].float().mean(1, keepdim=True).expand(4, 140, 128).numpy(), torch.bfloat16)

@@ -170,8 +170,8 @@ constexpr int smem_bytes() { return kWarps * stages<D>() * tile_bytes<D>() + par
 template <typename T>
 __device__ __forceinline__ float mask_value(const Dec16Params& p, int64_t at) {
     if (p.mask_kind == B2A_MASK_BOOL) return p.mask[at] != 0 ? 0.f : -INFINITY;
-    const float m = to_f32<T>(reinterpret_cast<const T*>(p.mask)[at]);
-    return m == -INFINITY ? m : fmaxf(m * kLog2e, kNegBig);
+    const float m = to_f32<T>(reinterpret_cast<const T*>(p.mask)[at]), v = m * kLog2e;
+    return v < kNegBig && m != -INFINITY ? kNegBig : v;  // (a NaN stays one)
 }
 
 // Grid (cluster size, KV heads, sequences); cluster (size, 1, 1).  NT: groups of eight query rows.

@@ -165,3 +165,15 @@ def test_the_lowest_value_in_every_place_is_an_average(b2a, skv, rows):
     out = b2a.sdpa(q.cuda(), k.cuda(), v.cuda(), m.cuda())
     for i, lo in ((0, 0), (1, 150)):
         _check(out[i], v[i, :, lo:].float().mean(1, keepdim=True).expand(4, 140, 128).numpy(), torch.bfloat16)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("sq,rows,skv,d", [(1, 1, 100, 128), (140, 1, 201, 64), (140, 140, 201, 64), (140, 140, 200, 128)])
+def test_a_nan_in_the_mask_stays_one(b2a, dtype, sq, rows, skv, d):
+    q, k, v = _rand((2, 2, sq, d), 1, dtype), _rand((2, 2, skv, d), 2, dtype), _rand((2, 2, skv, d), 3, dtype)
+    m = torch.zeros(2, 1, rows, skv, dtype=dtype)
+    m[1, :, rows // 2, 70] = float("nan")
+    out = b2a.sdpa(q.cuda(), k.cuda(), v.cuda(), m.cuda()).float().cpu()
+    hit = torch.zeros(sq, dtype=torch.bool)
+    hit[rows // 2 if rows > 1 else slice(None)] = True
+    assert torch.isnan(out[1][:, hit]).all() and torch.isfinite(out[1][:, ~hit]).all() and torch.isfinite(out[0]).all()

@@ -200,6 +200,36 @@ def test_absent_ranks_time_out_prefill_and_own_tiles_reach_every_rank(b2a, world
         lib.b2a_shard_group_destroy(g)
 
 
+@pytest.mark.parametrize("world", [2, 4, 8])
+@pytest.mark.parametrize("causal", [False, True])
+def test_a_prefill_shard_has_the_bits_of_the_launch_over_all_heads(b2a, world, causal):
+    # ... although its own few tiles alone would be computed with their keys shared out: 160 tiles of all ranks are not, 80, 40
+    # or 20 would be.  (As above: rank 0 alone runs the step, its wait for the others runs out.)
+    from openvino_contrib_b200 import _lib
+    from openvino_contrib_b200.sharding import _device_view
+    lib = _lib.load()
+    B, hq, hkv, S = 2, 16, 8, 640
+    gen = torch.Generator().manual_seed(4)
+    q, k, v = ((torch.randn(B, h, S, D, generator=gen) * 0.5).to(torch.float16).cuda() for h in (hq, hkv, hkv))
+    ql, kl, vl = (t[:, : t.shape[1] // world].contiguous() for t in (q, k, v))
+    groups = _ranks_in_one_process(lib, B * hq * S * D * 2, world)
+    assert lib.b2a_shard_group_set_wait_ms(groups[0], 20) == 0
+    d = _lib.SdpaDesc()
+    d.dtype = _lib.F16
+    d.B, d.Hq, d.Hkv, d.Sq, d.Skv, d.D, d.Dv = B, hq // world, hkv // world, S, S, D, D
+    d.causal = int(causal)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = C.c_void_p()
+    assert lib.b2a_sdpa_forward_sharded(groups[0], C.byref(d), ql.data_ptr(), kl.data_ptr(), vl.data_ptr(), C.byref(out),
+                                        status.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert int(status.item()) == _lib.DEV_TIMEOUT
+    full = _device_view(out.value, (B, hq, S, D), torch.float16, q.device)
+    assert torch.equal(full[:, : hq // world], b2a.sdpa(q, k, v, causal=causal)[:, : hq // world])
+    for g in groups:
+        lib.b2a_shard_group_destroy(g)
+
+
 def _base_of(lib, group) -> int:
     p = C.c_void_p()
     assert lib.b2a_shard_group_output(group, C.byref(p)) == 0

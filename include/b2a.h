@@ -88,6 +88,13 @@ int b2a_sdpa_workspace_bytes(const b2a_sdpa_desc* desc, int sm_count, size_t* ou
 int b2a_sdpa_forward(const b2a_sdpa_desc* desc, const void* q, const void* k, const void* v, const void* mask,
                      void* o, void* workspace, size_t workspace_bytes, int32_t* status, b2a_stream_t stream);
 
+/* The same for one of `parts` calls of equal extents that together are one problem over more batch entries or heads
+ * (each with its own tensors): the rows have the bits that one call over the whole problem would give them.  How small
+ * problems are spread over the GPU, and with it the order of the sums, follows from the number of (batch, head) pairs. */
+int b2a_sdpa_forward_part(const b2a_sdpa_desc* desc, int32_t parts, const void* q, const void* k, const void* v,
+                          const void* mask, void* o, void* workspace, size_t workspace_bytes, int32_t* status,
+                          b2a_stream_t stream);
+
 /* ---------------------------------------------------------------------------------------------
  * PagedAttentionExtension
  *

@@ -41,6 +41,8 @@ SIGNATURES = {
     "b2a_sdpa_workspace_bytes": (C.c_int, [C.POINTER(SdpaDesc), C.c_int, C.POINTER(C.c_size_t)]),
     "b2a_sdpa_forward": (C.c_int, [C.POINTER(SdpaDesc), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
                                    C.c_void_p, C.c_size_t, C.c_void_p, C.c_void_p]),
+    "b2a_sdpa_forward_part": (C.c_int, [C.POINTER(SdpaDesc), C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
+                                        C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p, C.c_void_p]),
     "b2a_paged_chunk_bytes": (C.c_size_t, [C.c_int32, C.c_int32, C.c_int32]),
     "b2a_paged_workspace_bytes": (C.c_int, [C.POINTER(PagedDesc), C.c_int, C.POINTER(C.c_size_t)]),
     "b2a_paged_kv_store": (C.c_int, [C.POINTER(PagedDesc), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,

@@ -139,14 +139,21 @@ int b2a_sdpa_workspace_bytes(const b2a_sdpa_desc* desc, int sm_count, size_t* ou
     SdpaResolved r;
     const int rc = resolve_sdpa(desc, r);
     if (rc != B2A_OK) return rc;
-    *out_bytes = 0;  // both SDPA kernels keep their state on chip
+    *out_bytes = 0;  // the SDPA kernels keep their state on chip
     return B2A_OK;
 }
 
 int b2a_sdpa_forward(const b2a_sdpa_desc* desc, const void* q, const void* k, const void* v, const void* mask,
                      void* o, void* workspace, size_t workspace_bytes, int32_t* status, b2a_stream_t stream) {
+    return b2a_sdpa_forward_part(desc, 1, q, k, v, mask, o, workspace, workspace_bytes, status, stream);
+}
+
+int b2a_sdpa_forward_part(const b2a_sdpa_desc* desc, int32_t parts, const void* q, const void* k, const void* v,
+                          const void* mask, void* o, void* workspace, size_t workspace_bytes, int32_t* status,
+                          b2a_stream_t stream) {
     (void)workspace;
     (void)workspace_bytes;
+    if (parts <= 0) return B2A_ERR_DIM;
     SdpaResolved r;
     const int rc = resolve_sdpa(desc, r);
     if (rc != B2A_OK) return rc;
@@ -158,15 +165,17 @@ int b2a_sdpa_forward(const b2a_sdpa_desc* desc, const void* q, const void* k, co
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     // a few query rows (token generation): no 128-row tile to fill, the keys and values are the work
     if (sdpa_decode16_supported(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, o))
-        return sdpa_decode16_launch(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, masked ? mask : nullptr, o, status, s);
+        return sdpa_decode16_launch(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, masked ? mask : nullptr, o, status, s, parts);
     if (sdpa_tc_supported(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, o) && (!masked || sdpa_tc_mask_supported(r.d, mask)))
-        return sdpa_tc_launch(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, o, status, s, nullptr, masked ? mask : nullptr);
+        return sdpa_tc_launch(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, o, status, s, nullptr, masked ? mask : nullptr, false,
+                              parts);
     // head size 64, and masks that cannot be read in 16-byte pieces.  From the smallest problems on: a launch of one item
     // takes about as long as one 32-key step of the general kernel
     if (sdpa_tc_split_supported(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, o))
-        return sdpa_tc_launch(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, o, status, s, nullptr, masked ? mask : nullptr, true);
+        return sdpa_tc_launch(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, o, status, s, nullptr, masked ? mask : nullptr, true,
+                              parts);
     if (sdpa_f32_supported(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, o))
-        return sdpa_f32_launch(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, masked ? mask : nullptr, o, s);
+        return sdpa_f32_launch(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, masked ? mask : nullptr, o, s, parts);
     return sdpa_generic_launch(r.d, r.qs, r.ks, r.vs, r.os, q, k, v, mask, o, status, s);
 }
 

@@ -534,7 +534,7 @@ int launch_d(const Dec16Params& p, int D, bool paged, int csize, int hkv, int ba
                     : launch_variant<T, NT, 64, false>(p, csize, hkv, batch, stream);
 }
 
-int launch_any(int dtype, const Dec16Params& p, int D, bool paged, int keys, int hkv, int batch, cudaStream_t stream) {
+int launch_any(int dtype, const Dec16Params& p, int D, bool paged, int keys, int hkv, int batch, cudaStream_t stream, int parts = 1) {
     // CTAs per (sequence, KV head), as long as every warp keeps two tiles or more.  Dense tensors: equal lengths, so at
     // least three quarters of one wave of two CTAs per SM and no second wave (8 x 3003 keys x 8 KV heads, with the
     // additive mask: two CTAs 32.3 us, four 20.9, eight 25.6).  A pool: lengths differ, and shorter pieces even them out
@@ -545,7 +545,7 @@ int launch_any(int dtype, const Dec16Params& p, int D, bool paged, int keys, int
     const int tiles = std::max(1, (keys + kTileKeys - 1) / kTileKeys);
     const long long want = paged ? 6LL * sms : 3LL * sms / 2;
     int csize = 1;
-    while (csize < kMaxCluster && static_cast<long long>(csize) * hkv * batch < want && tiles >= 4 * csize * kWarps) csize *= 2;
+    while (csize < kMaxCluster && static_cast<long long>(csize) * hkv * batch * parts < want && tiles >= 4 * csize * kWarps) csize *= 2;
     if (dtype == B2A_F16)
         return p.rows > 8 ? launch_d<__half, 2>(p, D, paged, csize, hkv, batch, stream)
                           : launch_d<__half, 1>(p, D, paged, csize, hkv, batch, stream);
@@ -575,7 +575,7 @@ bool sdpa_decode16_supported(const b2a_sdpa_desc& d, const int64_t (&qs)[4], con
 
 int sdpa_decode16_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t (&ks)[4], const int64_t (&vs)[4],
                          const int64_t (&os)[4], const void* q, const void* k, const void* v, const void* mask, void* o,
-                         int32_t* status, cudaStream_t stream) {
+                         int32_t* status, cudaStream_t stream, int parts) {
     Dec16Params p{};
     p.q = static_cast<const uint8_t*>(q);
     p.k = static_cast<const uint8_t*>(k);
@@ -596,7 +596,7 @@ int sdpa_decode16_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const i
     p.o_b = 2 * os[0]; p.o_h = 2 * os[1]; p.o_s = 2 * os[2];
     p.m_b = d.mask_strides[0]; p.m_h = d.mask_strides[1]; p.m_s = d.mask_strides[2]; p.m_k = d.mask_strides[3];
     p.status = status;
-    return launch_any(d.dtype, p, d.D, false, d.causal ? std::min(d.Sq, d.Skv) : d.Skv, d.Hkv, d.B, stream);
+    return launch_any(d.dtype, p, d.D, false, d.causal ? std::min(d.Sq, d.Skv) : d.Skv, d.Hkv, d.B, stream, parts);
 }
 
 bool paged_decode16_supported(const b2a_paged_desc& d) {

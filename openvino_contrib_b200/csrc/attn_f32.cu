@@ -331,7 +331,7 @@ bool sdpa_f32_supported(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const in
 
 int sdpa_f32_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t (&ks)[4], const int64_t (&vs)[4],
                     const int64_t (&os)[4], const void* q, const void* k, const void* v, const void* mask, void* o,
-                    cudaStream_t stream) {
+                    cudaStream_t stream, int parts) {
     F32Params p{};
     p.B = d.B; p.Hq = d.Hq; p.G = d.Hq / d.Hkv; p.Sq = d.Sq; p.Skv = d.Skv; p.D = d.D;
     p.causal = d.causal;
@@ -348,7 +348,7 @@ int sdpa_f32_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_
     for (int i = 0; i < 4; ++i) p.ms[i] = d.mask_strides[i];
     const int sms = device_sm_count();
     if (sms <= 0) return B2A_ERR_CUDA;
-    const long long heads = static_cast<long long>(d.B) * d.Hq;
+    const long long heads = static_cast<long long>(d.B) * d.Hq * parts;
     const int split = heads * ((d.Sq + 63) / 64) >= sms ? 1 : heads * ((d.Sq + 31) / 32) >= sms ? 2 : 4;
     if (d.D <= 64) return split == 1 ? launch<1, 1>(p, stream) : split == 2 ? launch<1, 2>(p, stream) : launch<1, 4>(p, stream);
     return split == 1 ? launch<2, 1>(p, stream) : split == 2 ? launch<2, 2>(p, stream) : launch<2, 4>(p, stream);

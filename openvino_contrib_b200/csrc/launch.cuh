@@ -20,7 +20,7 @@ bool sdpa_f32_supported(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const in
                         const int64_t (&os)[4], const void* q, const void* k, const void* v, const void* o);
 int sdpa_f32_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t (&ks)[4], const int64_t (&vs)[4],
                     const int64_t (&os)[4], const void* q, const void* k, const void* v, const void* mask, void* o,
-                    cudaStream_t stream);
+                    cudaStream_t stream, int parts = 1);
 
 // attn_decode16.cu — at most sixteen query rows per KV head over 16-bit keys and values (D = Dv = 64 or 128): a few query
 // rows on dense tensors, any mask; the one-token sequences of a paged step on a pool of the queries' own type
@@ -28,7 +28,7 @@ bool sdpa_decode16_supported(const b2a_sdpa_desc& d, const int64_t (&qs)[4], con
                              const int64_t (&os)[4], const void* q, const void* k, const void* v, const void* o);
 int sdpa_decode16_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t (&ks)[4], const int64_t (&vs)[4],
                          const int64_t (&os)[4], const void* q, const void* k, const void* v, const void* mask, void* o,
-                         int32_t* status, cudaStream_t stream);
+                         int32_t* status, cudaStream_t stream, int parts = 1);
 bool paged_decode16_supported(const b2a_paged_desc& d);
 int paged_decode16_launch(const b2a_paged_desc& d, const void* query, const void* k_cache, const void* v_cache,
                           const PagedTables& t, void* out, int32_t* status, cudaStream_t stream);
@@ -138,7 +138,8 @@ struct TcPeerOut {
 bool sdpa_tc_mask_supported(const b2a_sdpa_desc& d, const void* mask);
 int sdpa_tc_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t (&ks)[4], const int64_t (&vs)[4],
                    const int64_t (&os)[4], const void* q, const void* k, const void* v, void* o, int32_t* status,
-                   cudaStream_t stream, const TcPeerOut* peers = nullptr, const void* mask = nullptr, bool split_p = false);
+                   cudaStream_t stream, const TcPeerOut* peers = nullptr, const void* mask = nullptr, bool split_p = false,
+                   int parts = 1);
 // split_p: the form whose probabilities keep float32-like precision; head size 64 or 128 (128: with a mask), any mask
 bool sdpa_tc_split_supported(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t (&ks)[4],
                              const int64_t (&vs)[4], const int64_t (&os)[4], const void* q, const void* k, const void* v,

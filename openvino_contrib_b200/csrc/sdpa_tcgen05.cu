@@ -1631,7 +1631,7 @@ bool sdpa_tc_mask_supported(const b2a_sdpa_desc& d, const void* mask) {
 
 int sdpa_tc_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t (&ks)[4], const int64_t (&vs)[4],
                    const int64_t (&os)[4], const void* q, const void* k, const void* v, void* o, int32_t* status,
-                   cudaStream_t stream, const TcPeerOut* peer_out, const void* mask, bool split_p) {
+                   cudaStream_t stream, const TcPeerOut* peer_out, const void* mask, bool split_p, int parts) {
     const bool bf16 = d.dtype == B2A_BF16;
     CUtensorMap mq, mk, mv;
     // A causal row sees at most Sq keys: what lies behind (a cache's unfilled rows, which may hold NaN) comes in as zeros, like
@@ -1691,12 +1691,13 @@ int sdpa_tc_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t
     // It reads K and V twice as fast.  On more than half of the SMs that is more than the pairs ever ask of L2, and copies
     // running beside it starve: host tensors in pieces of 8 heads x 4096 tokens (256 tiles) took 5.05 ms a step instead of
     // 4.53, although the kernel itself went from 61 to 37 us.  So such grids share the keys out up to sixteen steps only.
-    // A sharded launch asks the rule for ALL ranks' heads: its output is that of one launch over them, bit for bit.
+    // A sharded launch, or one that is a part of a problem, asks the rule for ALL heads: its output is that of one launch over
+    // them, bit for bit.
     bool key_split = false;
-    const long long ranks = peer_out != nullptr ? peer_out->hq_total / d.Hq : 1;
-    const long long streams = static_cast<long long>(d.B) * d.Hkv * ranks, all_tiles = streams * nrb * p.G;
+    const long long shares = peer_out != nullptr ? peer_out->hq_total / d.Hq : parts;
+    const long long streams = static_cast<long long>(d.B) * d.Hkv * shares, all_tiles = streams * nrb * p.G;
     const int n = (keys + kBN - 1) / kBN, half = (n + 1) / 2;
-    if (items * ranks <= sms && (n <= 16 || 2 * all_tiles <= sms)) {
+    if (items * shares <= sms && (n <= 16 || 2 * all_tiles <= sms)) {
         const long long rounds = (all_tiles + sms - 1) / sms;
         double steps = static_cast<double>(rounds * half);
         if (d.causal) {
@@ -1706,7 +1707,7 @@ int sdpa_tc_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t
         }
         key_split = steps + (rounds > 1 ? 1.5 : 0.0) < n;
     }
-    const dim3 tile_grid(static_cast<unsigned>(key_split ? all_tiles / ranks : 0));
+    const dim3 tile_grid(static_cast<unsigned>(key_split ? all_tiles / shares : 0));
     if (split_p) {
         // a mask that is one row for all queries is read once per warp; anything else row by row
         const int form = mask_kind == B2A_MASK_NONE                    ? 0

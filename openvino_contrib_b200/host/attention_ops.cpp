@@ -73,6 +73,7 @@ SdpaOp::SdpaOp(const CreationContext& context, const NodeOp& node, IndexCollecti
     desc_.dtype = dt;
     desc_.B = bq; desc_.Hq = hq; desc_.Hkv = hk; desc_.Sq = sq; desc_.Skv = sk; desc_.D = e; desc_.Dv = ev;
     desc_.causal = node.get_causal() ? 1 : 0;
+    parts_ = static_cast<int32_t>(rt_info_int(node, "b2a.parts", 1));
     desc_.scale = 0.f;  // 1/sqrt(E)
     if (n_in == 5) {
         desc_.scale = *node.const_scale;
@@ -117,10 +118,10 @@ void SdpaOp::Execute(const InferenceRequestContext& context, Inputs in, Outputs 
     if (in.size() < (has_mask_ ? 4u : 3u) || out.size() != 1) ov::throw_ov_exception("ScaledDotProductAttention: operand count");
     const void* mask = has_mask_ ? in[3].get() : nullptr;
     void* ws = (workspace_bytes_ > 0 && !wb.mutable_buffers.empty()) ? wb.mutable_buffers[0].get() : nullptr;
-    throwIfError(b2a_sdpa_forward(&desc_, in[0].get(), in[1].get(), in[2].get(), mask, out[0].get(), ws,
-                                  workspace_bytes_, nullptr,
-                                  reinterpret_cast<b2a_stream_t>(context.getThreadContext().stream().get())),
-                 "b2a_sdpa_forward");
+    throwIfError(b2a_sdpa_forward_part(&desc_, parts_, in[0].get(), in[1].get(), in[2].get(), mask, out[0].get(), ws,
+                                       workspace_bytes_, nullptr,
+                                       reinterpret_cast<b2a_stream_t>(context.getThreadContext().stream().get())),
+                 "b2a_sdpa_forward_part");
 }
 
 PagedAttentionOp::PagedAttentionOp(const CreationContext& context, const NodeOp& node, IndexCollection&& inputIds,

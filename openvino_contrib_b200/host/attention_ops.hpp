@@ -31,6 +31,7 @@ private:
     b2a_sdpa_desc desc_{};
     size_t workspace_bytes_ = 0;
     bool has_mask_ = false;
+    int32_t parts_ = 1;  // run-time information "b2a.parts": the node is one of so many equal pieces of a problem
 };
 
 // PagedAttentionExtension.  The constructor depends only on what is static for a compiled model: head counts,

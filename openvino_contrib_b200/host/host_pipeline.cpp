@@ -48,6 +48,7 @@ HostSdpaRunner::HostSdpaRunner(int dtype, int B, int Hq, int Hkv, int Sq, int Sk
     node->add_input(et, {1, z(hpp_), z(Skv), z(D)});
     node->add_input(et, {1, z(hpp_), z(Skv), z(D)});
     node->add_output(et, {1, z(G_ * hpp_), z(Sq), z(D)});
+    node->get_rt_info()["b2a.parts"] = static_cast<int64_t>(pieces());
     CreationContext cc{device_, false};
     op_ = OperationRegistry::getInstance().createOperation(cc, node, tensor_ids(0, 3), tensor_ids(3, 1));
     const auto req = op_->GetWorkBufferRequest();

@@ -216,6 +216,21 @@ def test_host_pipeline_matches_device_call(b2a):
         pipe(q.cuda(), k, v, out)
 
 
+@pytest.mark.parametrize("dtype,b,hq,hkv,sq,skv,d,causal", [
+    (torch.float16, 2, 16, 8, 640, 640, 128, False),   # 160 tiles; a piece of ten would share its keys out
+    (torch.bfloat16, 4, 16, 16, 520, 520, 64, False),  # the same at head size 64
+    (torch.bfloat16, 8, 32, 8, 1, 3003, 128, False),   # few rows: clusters of four, a piece alone would take eight
+    (torch.float32, 8, 8, 8, 256, 256, 64, True),      # float32: 64-row tiles, a piece alone would take 16-row ones
+])
+def test_host_pipeline_pieces_have_the_bits_of_one_call(b2a, dtype, b, hq, hkv, sq, skv, d, causal):
+    gen = torch.Generator().manual_seed(11)
+    q, k, v = ((torch.randn(b, h, s, d, generator=gen) * 0.5).to(dtype).pin_memory() for h, s in ((hq, sq), (hkv, skv), (hkv, skv)))
+    out = torch.empty(b, hq, sq, d, dtype=dtype).pin_memory()
+    b2a.HostSdpaPipeline(b, hq, hkv, sq, skv, d, dtype, causal=causal, kv_heads_per_piece=1)(q, k, v, out)
+    torch.cuda.synchronize()
+    assert torch.equal(out.cuda(), b2a.sdpa(q.cuda(), k.cuda(), v.cuda(), causal=causal))
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("kind", ["bool", "add"])
 def test_masks_on_the_tensor_core_shape(b2a, dtype, kind):

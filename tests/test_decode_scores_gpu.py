@@ -26,7 +26,9 @@ def b2a():
     ([9, 250, 1500], 32, 8, 1), ([9, 250, 1500], 32, 8, 100), ([9, 250, 1500], 16, 8, 4096),
 ])
 def test_both_outputs(b2a, dtype, ctx, hq, hkv, window):
-    # the attention rows are the bits of paged_attention; the scores agree with the oracle like those of the call of their own
+    # the attention rows are the bits of paged_attention wherever both calls cut the sequences alike: in steps that leave the plan
+    # below 96 blocks a chunk, as these do (beyond, the scores halve the chunks: test_more_than_32_splits compares with the
+    # oracle).  The scores agree with the oracle like those of the call of their own
     w = PagedWorkload(ctx, [1] * len(ctx), hq, hkv, 128, seed=3 * hq + len(ctx))
     q = torch.from_numpy(w.query).to(dtype)
     cache, tables, status = w.device_cache(), w.device_tables(), torch.zeros(1, dtype=torch.int32, device="cuda")

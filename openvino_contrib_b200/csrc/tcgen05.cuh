@@ -68,8 +68,8 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t sm
                  "r"(smem_src), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
                  : "memory");
 }
-// The same two with an L2 cache policy (createpolicy): evict-first for data that is touched once (Q tiles, output
-// tiles), so that it does not push out the K/V tiles that every query head of a group comes back for.
+// The load with an L2 cache policy (createpolicy): evict-first for data that is touched once (Q tiles), so that it does
+// not push out the K/V tiles that every query head of a group comes back for.
 __device__ __forceinline__ uint64_t l2_evict_first_policy() {
     uint64_t pol;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
@@ -81,17 +81,6 @@ __device__ __forceinline__ void tma_load_4d_hint(uint32_t smem_dst, const CUtens
         "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5, %6}], [%2], %7;"
         ::"r"(smem_dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "l"(policy)
         : "memory");
-}
-__device__ __forceinline__ void tma_store_4d_hint(const CUtensorMap* map, uint32_t smem_src, int c0, int c1, int c2, int c3,
-                                                  uint64_t policy) {
-    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group.L2::cache_hint [%0, {%2, %3, %4, %5}], [%1], %6;"
-                 ::"l"(map), "r"(smem_src), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "l"(policy)
-                 : "memory");
-}
-// the box into L2 only
-__device__ __forceinline__ void tma_prefetch_4d(const CUtensorMap* map, int c0, int c1, int c2, int c3) {
-    asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];" ::"l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-                 : "memory");
 }
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }

@@ -154,6 +154,7 @@ int b2a_sdpa_forward_part(const b2a_sdpa_desc* desc, int32_t parts, const void* 
     (void)workspace;
     (void)workspace_bytes;
     if (parts <= 0) return B2A_ERR_DIM;
+    if (parts > 4096) parts = 4096;  // (every rule that looks at it is long past its last line by then, and no product overflows)
     SdpaResolved r;
     const int rc = resolve_sdpa(desc, r);
     if (rc != B2A_OK) return rc;

@@ -95,16 +95,8 @@ template <>
 struct ProbPieces<__nv_bfloat16> {
     static constexpr int kCount = 3, kAccs = 1;
     static __device__ __forceinline__ void split(float p0, float p1, uint32_t (&w)[3]) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            w[e] = __byte_perm(__float_as_uint(p0 * (1.f - 1.f / 1024.f)), __float_as_uint(p1 * (1.f - 1.f / 1024.f)), 0x7632);
-            p0 -= __uint_as_float(w[e] << 16);
-            p1 -= __uint_as_float(w[e] & 0xffff0000u);
-        }
-        const __nv_bfloat162 l = __floats2bfloat162_rn(p0, p1);
-        w[2] = *reinterpret_cast<const uint32_t*>(&l);
-    }
-};
+        uint64_t p;
+        asm("mov.b64 %0, {%1, %2};
 
 // Programmatic dependent launch: a kernel launched with launch_overlapped may be scheduled while the kernel before
 // it on the stream is still running (as soon as that one has executed grid_launch_dependents in every CTA, or has

@@ -16,11 +16,11 @@
 // f16 or three bf16 values (ProbPieces), which costs eight or sixteen more MMAs per tile where the tensor pipe idles anyway.
 //
 // Measured on a B200 (graph replay): bf16, 8 sequences x 3003 keys x 8 KV heads, additive mask (98 MB): 2049 us on
-// attn_generic_kernel before, 23.3 us now (4.2 TB/s; 15.1 us at the copy rate); 32 bf16 sequences of 256..4096 tokens in
-// a pool (293 MB, with the store of the step): 8149 us before, 56.5 us now (5.2 TB/s; 44.8 us at the copy rate).  Two bf16
-// pieces, which keep 2^-16 of a probability, took 22.8 and 55.3 us; two tf32 pieces beside V widened to tf32 24.0 and 59.5.
+// attn_generic_kernel before, 21.2 us now (4.6 TB/s; 15.1 us at the copy rate); 32 bf16 sequences of 256..4096 tokens in
+// a pool (293 MB, with the store of the step): 8149 us before, 57.3 us now (5.1 TB/s; 44.8 us at the copy rate).
+// On another box and before a cheaper floor for the mask: two bf16 pieces, which keep 2^-16 of a probability, 22.8 and 55.3 us,
+// three 23.3 and 56.5, two tf32 pieces beside V widened to tf32 24.0 and 59.5.
 #include <algorithm>
-#include <atomic>
 
 #include "launch.cuh"
 
@@ -113,17 +113,6 @@ __device__ __forceinline__ uint32_t pack_pair<__nv_bfloat16>(float lo, float hi)
     const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&h);
 }
-template <typename T>
-__device__ __forceinline__ float2 unpack_pair(uint32_t w);
-template <>
-__device__ __forceinline__ float2 unpack_pair<__half>(uint32_t w) {
-    return __half22float2(*reinterpret_cast<const __half2*>(&w));
-}
-template <>
-__device__ __forceinline__ float2 unpack_pair<__nv_bfloat16>(uint32_t w) {
-    return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
-}
-
 // Factor on the probabilities before they are cut into pieces (ProbPieces), carried by the row sum: f16's pieces reach down to
 // 2^-49 of the row's maximum with it.
 template <typename T>
@@ -514,13 +503,9 @@ template <typename T, int NT, int D, bool kPaged>
 int launch_variant(const Dec16Params& p, int csize, int hkv, int batch, cudaStream_t stream) {
     auto kern = attn_decode16_kernel<T, NT, D, kPaged>;
     constexpr int kSmem = smem_bytes<D, NT>();
-    static std::atomic<bool> configured[64];  // per device; setting the attribute twice is harmless
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return B2A_ERR_CUDA;
-    if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) return B2A_ERR_CUDA;
-        if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
-    }
+    static OncePerDevice configured;
+    const int rc = configure_once(kern, configured, kSmem);
+    if (rc != B2A_OK) return rc;
     return launch_overlapped_cluster(kern, dim3(csize, hkv, batch), dim3(kWarps * 32), csize, kSmem, stream, p) == cudaSuccess
                ? B2A_OK
                : B2A_ERR_CUDA;

@@ -304,15 +304,9 @@ int launch(const F32Params& p, cudaStream_t stream) {
     constexpr int BM = kRowsPerWarp * row_groups(kSplit);
     const size_t smem = smem_floats<NC, kSplit>(p.D) * sizeof(float);
     auto kern = attn_f32_kernel<NC, kSplit>;
-    static bool configured[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return B2A_ERR_CUDA;
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(smem_floats<NC, kSplit>(64 * NC) * sizeof(float))) != cudaSuccess)
-            return B2A_ERR_CUDA;
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
+    static OncePerDevice configured;
+    const int rc = configure_once(kern, configured, static_cast<int>(smem_floats<NC, kSplit>(64 * NC) * sizeof(float)));
+    if (rc != B2A_OK) return rc;
     kern<<<dim3((p.Sq + BM - 1) / BM, p.Hq, p.B), kThreads, smem, stream>>>(p);
     return cudaGetLastError() == cudaSuccess ? B2A_OK : B2A_ERR_CUDA;
 }

@@ -284,14 +284,10 @@ template <typename T>
 int launch_generic_t(const GenericParams& p, dim3 grid, cudaStream_t stream) {
     const size_t smem = generic_smem_bytes(p.D, p.Dv);
     auto kern = attn_generic_kernel<T>;
-    static bool configured[64] = {};  // per device, per element type (this function is a template)
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return B2A_ERR_CUDA;
-    if (smem > 48 * 1024 && (dev < 0 || dev >= 64 || !configured[dev])) {
-        // An attribute of the function, not a stream operation: legal while a stream is being captured.
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 120 * 1024) != cudaSuccess)
-            return B2A_ERR_CUDA;
-        if (dev >= 0 && dev < 64) configured[dev] = true;
+    static OncePerDevice configured;  // per element type (this function is a template)
+    if (smem > 48 * 1024) {
+        const int rc = configure_once(kern, configured, 120 * 1024);
+        if (rc != B2A_OK) return rc;
     }
     kern<<<grid, kThreads, smem, stream>>>(p);
     return cudaGetLastError() == cudaSuccess ? B2A_OK : B2A_ERR_CUDA;

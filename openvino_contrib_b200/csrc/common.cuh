@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "b2a.h"
 
 namespace b2a {
@@ -96,7 +98,22 @@ struct ProbPieces<__nv_bfloat16> {
     static constexpr int kCount = 3, kAccs = 1;
     static __device__ __forceinline__ void split(float p0, float p1, uint32_t (&w)[3]) {
         uint64_t p;
-        asm("mov.b64 %0, {%1, %2};
+        asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(p0), "f"(p1));
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {  // (two lanes an instruction; the subtraction is exact)
+            uint64_t below, cut;
+            uint32_t b0, b1;
+            asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(below) : "l"(p), "l"(0x3f7fc0003f7fc000ull));  // 1 - 2^-10
+            asm("mov.b64 {%0, %1}, %2;" : "=r"(b0), "=r"(b1) : "l"(below));
+            w[e] = __byte_perm(b0, b1, 0x7632);
+            asm("mov.b64 %0, {%1, %2};" : "=l"(cut) : "r"(b0 & 0xffff0000u), "r"(b1 & 0xffff0000u));
+            asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(p) : "l"(cut), "l"(0xbf800000bf800000ull), "l"(p));
+        }
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(p0), "=f"(p1) : "l"(p));
+        const __nv_bfloat162 l = __floats2bfloat162_rn(p0, p1);
+        w[2] = *reinterpret_cast<const uint32_t*>(&l);
+    }
+};
 
 // Programmatic dependent launch: a kernel launched with launch_overlapped may be scheduled while the kernel before
 // it on the stream is still running (as soon as that one has executed grid_launch_dependents in every CTA, or has
@@ -143,6 +160,20 @@ inline cudaError_t launch_overlapped_cluster(void (*kernel)(KernelArgs...), dim3
     cfg.attrs = attr;
     cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kernel, KernelArgs(args)...);
+}
+
+// Raises a kernel's limit of dynamic shared memory, once per device (an attribute of the function, not a stream operation: legal
+// while a stream is being captured).  Several host threads may get here at once; setting it twice is harmless.
+using OncePerDevice = std::atomic<bool>[64];
+template <typename Kern>
+inline int configure_once(Kern kern, OncePerDevice& done, int smem) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return B2A_ERR_CUDA;
+    if (dev < 0 || dev >= 64 || !done[dev].load(std::memory_order_acquire)) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return B2A_ERR_CUDA;
+        if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
+    }
+    return B2A_OK;
 }
 
 }  // namespace b2a

@@ -844,7 +844,7 @@ __global__ void __launch_bounds__(kD) paged_decode_merge_kernel(const DecodePara
 // tables while the decode kernel drains.
 // Against two passes of their own over K (paged_scores.cu) this trades 2 x 132 bytes read per key and KV head for 8 G
 // bytes written and read, mostly in L2, and four launches for none: 32 sequences of 512..4096 tokens, 32/8 heads, the
-// whole step 107 -> 46.6 us.
+// whole step 107 -> 39.6 us.
 constexpr int kScorePositions = 512;
 template <typename T>
 __global__ void __launch_bounds__(kD) paged_decode_merge_scores_kernel(const DecodeParams p) {
@@ -946,14 +946,9 @@ __global__ void __launch_bounds__(256) peer_ll_copy_kernel(const PeerPush push, 
 template <typename T, int NT, int kMode, int kWarps>
 int launch_kernel_w(const DecodeParams& p, int num_seqs, cudaStream_t stream) {
     auto kern = paged_decode_kernel<T, NT, kMode, kWarps>;
-    static std::atomic<bool> configured[64];  // per device; setting the attribute twice is harmless
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return B2A_ERR_CUDA;
-    if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(kWarps)) != cudaSuccess)
-            return B2A_ERR_CUDA;
-        if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
-    }
+    static OncePerDevice configured;
+    const int rc = configure_once(kern, configured, smem_bytes(kWarps));
+    if (rc != B2A_OK) return rc;
     // the split index is the slowest-varying one: every sequence's first chunks (always full) are dispatched before
     // anybody's last chunk (partial or empty), which shortens the tail of a step with uneven contexts
     dim3 grid(p.Hkv, num_seqs, p.max_splits);

@@ -496,8 +496,8 @@ __global__ void __launch_bounds__(128) paged_gather_kernel(const PagedTables t, 
 //   `kDim` columns behind O_X.  With a head size of 128 that is tile B's place: an item is then ONE tile.  It costs one or two
 //   times as many second products again (the tensor pipe idles behind the exponentials anyway) and six to eight instructions
 //   per pair of probabilities.  Bound: the special-function unit, 128 exponentials per row and step; the f16 encoder batch
-//   of 8 x 16 heads x 512 tokens, head size 64, boolean padding mask: 1167 us in attn_generic_kernel, 27.1 us here (5.1 us
-//   of memory traffic at the copy rate).
+//   of 8 x 16 heads x 512 tokens, head size 64, boolean padding mask: 1167 us in attn_generic_kernel, 27.0 us here (5.1 us
+//   of memory traffic at the copy rate).  With 509 keys: f16 27.2 us, bf16 33.7 us; head size 128 51.0 and 64.7 us.
 // kKeySplit (dense): a small problem - fewer pairs of tiles than SMs - is bound by its longest chain of key steps, one tile's
 //   softmax after the other's.  Then an item is ONE tile whose keys are shared out: "tile A" takes the first half of its key
 //   tiles, "tile B" the second, each with its own maximum, sum and accumulator, which are merged in the epilogue (the two
@@ -1565,7 +1565,7 @@ template <int kMask, int kDim, bool kSplitP, bool kKeySplit = false>
 int launch_dense(bool bf16, dim3 grid, cudaStream_t stream, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                  const TcParams& p, const TcPeers& peers) {
     constexpr int smem = smem_bytes(128 * kDim * 2);
-    static bool configured[2][64] = {};
+    static OncePerDevice configured[2];
     auto kern = bf16 ? attn_tc_kernel<true, 0, kMask, kDim, kSplitP, kKeySplit> : attn_tc_kernel<false, 0, kMask, kDim, kSplitP, kKeySplit>;
     const int rc = configure_once(kern, configured[bf16], smem);
     if (rc != B2A_OK) return rc;
@@ -1578,18 +1578,6 @@ bool strides_ok(const int64_t (&st)[4], int B, int H, int S) {
     for (int i = 0; i < 3; ++i)
         if (ext[i] > 1 && (st[i] <= 0 || st[i] % 8 != 0)) return false;  // 16-byte multiples
     return true;
-}
-
-template <typename Kern>
-int configure_once(Kern kern, bool (&done)[64], int smem) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return B2A_ERR_CUDA;
-    if (dev < 0 || dev >= 64 || !done[dev]) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-            return B2A_ERR_CUDA;
-        if (dev >= 0 && dev < 64) done[dev] = true;
-    }
-    return B2A_OK;
 }
 
 }  // namespace
@@ -1851,13 +1839,13 @@ int paged_tc_launch(const b2a_paged_desc& d, const void* query, const void* k_ca
     constexpr int kSmemPaged = smem_bytes(128 * kHeadDim * 2);
     if (gathered) {
         grid = dim3(static_cast<unsigned>(attention_ctas));
-        static bool configured[2][64] = {};
+        static OncePerDevice configured[2];
         auto kern = bf16 ? attn_tc_kernel<true, 2> : attn_tc_kernel<false, 2>;
         const int rc = configure_once(kern, configured[bf16], kSmemPaged);
         if (rc != B2A_OK) return rc;
         if (launch_overlapped(kern, grid, dim3(kThreadsDense), kSmemPaged, stream, mq, mk, mv, p, peers) != cudaSuccess) return B2A_ERR_CUDA;
     } else {
-        static bool configured[2][64] = {};
+        static OncePerDevice configured[2];
         auto kern = bf16 ? attn_tc_kernel<true, 1> : attn_tc_kernel<false, 1>;
         const int rc = configure_once(kern, configured[bf16], kSmemPaged);
         if (rc != B2A_OK) return rc;

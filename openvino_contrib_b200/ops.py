@@ -349,7 +349,8 @@ def paged_attention_scores(query: torch.Tensor, cache: PagedKvCache, past_lens, 
                            scores: Optional[torch.Tensor] = None, stream=None, status: Optional[torch.Tensor] = None,
                            cache_rows_settled: bool = False):
     """``paged_attention`` and ``paged_last_token_scores`` of a step of one-token sequences, from one walk over the
-    cache.  Returns ``(out, scores, score_begins)``, or None where the kernels do not take the step (more than one
+    cache.  The attention rows may differ from ``paged_attention``'s in the last bits: large steps are cut into shorter
+    chunks here.  Returns ``(out, scores, score_begins)``, or None where the kernels do not take the step (more than one
     token per sequence, another geometry, or more scratch than ``_SCORE_SCRATCH_LIMIT``): make the two calls then."""
     num_tokens, num_seqs = query.shape[0], past_lens.shape[0]
     if num_tokens != num_seqs or num_seqs == 0:
@@ -392,8 +393,11 @@ class PagedAttentionOp:
     static for a compiled model - head counts, head size, block size, the capacity maxima, and the scale and
     sliding window (Constants in an exported model) - so one instance serves every step of a continuous-batching
     loop whatever its token and sequence counts, and nothing about it changes afterwards: what a scheduler knows
-    about one step is passed to that ``Execute`` call.  ``Execute`` only enqueues: it allocates nothing (the work
-    buffer must be the one ``GetWorkBufferRequest`` asked for) and never waits for the device.
+    about one step is passed to that ``Execute`` call.  ``Execute`` only enqueues and never waits for the device; without
+    a score output it allocates nothing (the work buffer must be the one ``GetWorkBufferRequest`` asked for).  The score
+    output's offsets and scratch come from torch's allocator on each call.  For a step of one-token sequences the scratch
+    is 64 * hq bytes per entry of ``block_indices`` - of the tensor, so a padded table counts whole; above 1 GiB the step
+    takes the two-call form, which needs little (and which the C++ operator always takes).
     """
 
     type_name = "PagedAttentionExtension"

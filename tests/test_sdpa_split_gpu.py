@@ -17,8 +17,7 @@ def b2a():
 
 def _check(out, ref, dtype, what=""):
     # the result's own rounding (half a unit in the last place: 2^-11 of the value in f16, 2^-9 in bf16; twice that is
-    # allowed), and float32 sums of values up to about five.  bf16 probabilities are two bf16 values: 2^-17 each, of an
-    # average of values up to about five
+    # allowed), and float32 sums of values up to about five.  The probabilities keep 22 (f16) or 24 bits (bf16)
     rtol = 2.0 ** -10 if dtype == torch.float16 else 2.0 ** -8
     np.testing.assert_allclose(out.float().cpu().numpy().reshape(ref.shape), ref, rtol=rtol, atol=5e-5, err_msg=what)
 

@@ -19,22 +19,31 @@
 //
 // Work is cut into items: TWO 128-row query tiles of one KV head, walked over the keys 128 at a time.  CTAs are
 // persistent (one per SM; mode 1 keeps one item per CTA): the items, heaviest first, are dealt in snake order.
-//   warps 0-3   softmax of tile A: thread = query row = TMEM lane.  Reads S_A (tcgen05.ld), keeps the running max
-//               and sum, writes P_A = exp2(S*c - m) as 16-bit pairs over the first half of S_A's columns
-//               (tcgen05.st) and signals the MMA issuer after the first 64 keys and again after all 128; rescales
-//               O_A in TMEM when the maximum moved; finally normalises O_A and stores it, a thread its row (heads sharded
-//               over several ranks: through a staging slab per warp, [32 x 64] and one TMA tensor store per slab and rank).
+//   warps 0-3   softmax of tile A: thread = query row = TMEM lane.  Reads S (tcgen05.ld) and gives its place up, keeps the
+//               running max and sum, writes P_A = exp2(S*c - m) as 16-bit pairs into P_A's columns (tcgen05.st) and
+//               signals the PV issuer; rescales O_A in TMEM when the maximum moved; finally normalises O_A and stores
+//               it, a thread its row (heads sharded over several ranks: through a staging slab per warp, [32 x 64] and
+//               one TMA tensor store per slab and rank).
 //   warps 4-7   the same for tile B.
 //   warp  8     TMA producer (one lane): the Q tiles of an item as soon as the previous item's last QK^T has
-//               completed, and (modes 0, 2) K_j and V_j into two-stage rings that run on across items.
-//   warp  9     MMA issuer (one lane): S_X(j) = Q_X K_j^T (A and B from shared memory, K-major, 128-byte swizzle),
-//               O_X += P_X(j) V_j (A from TMEM, B from shared memory, MN-major).  Order per step:
-//               PV_A(j), QK_A(j+1), PV_B(j), QK_B(j+1) - while one tile's softmax runs, the tensor core works on
-//               the other tile.  Descriptors are put together at the point of issue (tcgen05.cuh) so the thread
-//               stays within its 56 registers.  The warp also owns the TMEM allocation (all 512 columns: S_A S_B
-//               O_A O_B).
-//   warps 10-11 complete the service warpgroup whose registers are handed to the softmax groups; in mode 2 with
-//               bf16 queries they convert the Q tiles to f16 in shared memory.
+//               completed, and (modes 0, 2) K_j and V_j into two-stage rings that run on across items, K a step ahead.
+//   warp  9     issues S = Q_X K_j^T (A and B from shared memory, K-major, 128-byte swizzle), in turn A(0) B(0) A(1) B(1)
+//               ..  S has ONE place of 128 columns: a turn's QK is issued as soon as the turn before has its scores in
+//               registers, which is long before its own softmax warps come for them.
+//   warp 10     issues O_X += P_X(j) V_j (A from TMEM, B from shared memory, MN-major) when P_X is ready.
+//   warp 11     completes the service warpgroup; in mode 2 with bf16 queries it and the producer's warp convert the Q
+//               tiles to f16 in shared memory, a tile each.
+// TMEM: S 128 columns, P_A and P_B 64 each, O_A and O_B 128 each: all 512 (allocated by warp 9).
+// Why S is shared and QK and PV have issuers of their own: with S and P of a tile in one place a step is the chain softmax ->
+// PV -> QK -> softmax (1750 + 256 + 512 cycles and three trips over barriers), and one issuer, which stands still while the
+// tensor core's short queue is full and pays about 130 cycles for every barrier it looks at, leaves the tensor core idle
+// for a third of a step.  Causal prefill of 4 x 4096 tokens, 32/8 heads, bf16: 785 thousand cycles a launch before, 692 now;
+// in time 542 us before and 516 now in a loop of passes, because the launch runs into the power limit (1.43 GHz there).
+// Three prompts of 400 to 1100 tokens behind caches of up to 3000: 92.2 -> 86.6 us a step.  (Issued by one warp on a shared S: 785.
+// P's first half sent ahead of the second, P kept in registers until PV(j-1) has read the columns, the maximum of half a
+// row while the other half is loaded, two PV issuers: no gain, the exponentials of the two tiles are what counts now.)
+// The calls that hold P in several pieces (kSplitP) have no columns for that: there S_X has a place per tile, the pieces of P
+// lie over it, and one lane of warp 9 issues PV_A(j), QK_A(j+1), PV_B(j), QK_B(j+1), PV in two halves as those of P arrive.
 //   warps 12-15 mode 1 only: the de-quantising K/V producers.
 // The two tiles are consecutive entries of the list (row block, query head of the group), query heads fastest, so
 // with an even group size both tiles cover the same rows of two heads that share K/V, and the causal structure of
@@ -61,16 +70,16 @@ constexpr int kBM = 128;             // query rows per tile = TMEM lanes
 constexpr int kBN = 128;             // keys per step
 constexpr int kHeadDim = 128;
 constexpr int kPanel = 128 * 128;    // bytes of one [128 rows x 64 elements] swizzled panel
-constexpr int kThreadsDense = 384;   // 3 warpgroups: softmax A, softmax B, {producer, MMA issuer, 2 idle warps}
+constexpr int kThreadsDense = 384;   // 3 warpgroups: softmax A, softmax B, {producer, QK issuer, PV issuer, one more}
 constexpr int kThreadsPaged = 512;   // plus the de-quantising producer warpgroup
-constexpr int kNumBars = 27;
+constexpr int kNumBars = 28;
 constexpr int kStageOut = 8 * 4096;  // epilogue staging: one [32 rows x 64 elements] slab per softmax warp
 constexpr int smem_bytes(int tile) { return 6 * tile + kStageOut + 1024 /* alignment slack */ + 256 /* barriers, TMEM slot, abort flag */; }
 constexpr float kLazyThreshold = 8.0f;  // log2 units
 constexpr int kCacheChunk = 16 * (kHeadDim + 4);  // bytes of one (block, KV head) chunk of the u8 pool
 
 enum Bar { Q_FULL = 0, K_FULL = 2, K_EMPTY = 4, V_FULL = 6, V_EMPTY = 8, S_FULL = 10, P_READY = 12, O_DONE = 14, DRAIN = 16, P_HALF = 17, Q_CONV = 19, Q_EMPTY = 21,
-           HALVES = 23 };
+           HALVES = 23, S_FREE = 27 };
 
 // n / d for 0 <= n < 2^31 by one multiplication: mul = ceil(2^(31 + shift) / d) with shift = ceil(log2 d) errs by less than
 // n / 2^(31 + shift) < 1 / d (Granlund and Montgomery's division by an invariant).  A role works out its place from the
@@ -514,6 +523,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     static_assert(!kSplitP || kMode == 0, "the paged modes hold P in 16 bits");
     constexpr bool kSingle = kSplitP && kDim == kHeadDim;  // an item is one tile: the pieces of P need tile B's columns
     static_assert(!(kSingle && kKeySplit), "no columns for the other half of the keys");
+    constexpr bool kSharedS = !kSplitP;  // one place for S, which the tiles take in turn; P has columns of its own
     constexpr int kTile = 128 * kDim * 2;  // bytes of a [128 x kDim] 16-bit tile: kDim / 64 panels
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -662,9 +672,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             if (i == P_READY || i == P_READY + 1 || i == P_HALF || i == P_HALF + 1) count = 128;
             if (i == Q_CONV || i == Q_CONV + 1) count = 128;
             if (i == Q_EMPTY || i == Q_EMPTY + 1) count = 1;
-            if (i >= HALVES) count = 64;  // the two warps of the same rows
+            if (i >= HALVES && i < HALVES + 4) count = 64;  // the two warps of the same rows
+            if (i == S_FREE) count = 128;
             if (kDequant && (i == K_FULL || i == K_FULL + 1 || i == V_FULL || i == V_FULL + 1)) count = 128;
-            if (kGathered && (i == Q_CONV || i == Q_CONV + 1)) count = 64;  // converted by warps 10 and 11
+            if (kGathered && (i == Q_CONV || i == Q_CONV + 1)) count = 32;  // a warp each
+            if (i == DRAIN && kSharedS) count = 2;
             mbar_init(BAR(i), count);
         }
         *abort_flag = 0;
@@ -677,7 +689,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = kSharedS ? 0u : *tmem_slot;  // (an allocation of all 512 columns starts at the first one)
 
     // Launched programmatically dependent: what is above overlaps the kernel before this one, everything that touches
     // memory comes after it.  Then a kernel that depends on this one (the decode kernel of a mixed step) may take the SMs
@@ -701,15 +713,43 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         total_items = pairs * p.B * p.Hkv;  // the launcher keeps this below 2^31
     }
 
-    // Registers follow the work: the service warpgroup keeps 56 per thread, the softmax groups take what is left
-    // (dense: 2*128*224 + 128*56 = 384*168; paged: 2*128*168 + 128*56 + 128*112 <= 512*128).
-    if (warp >= 8 && warp < 12) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
-    }
+    // Gathered K/V and bf16 queries: one warp turns Q tile X into f16 where it lies (the swizzle only permutes 16-byte chunks, so
+    // an element-wise pass keeps the layout).  `n`: Q tiles of this kind before it.
+    constexpr bool kConvertQ = kGathered && kBf16;
+    auto convert_q = [&](int X, int n) {
+        if (!__all_sync(0xffffffffu, mbar_wait(BAR(Q_FULL + X), n & 1, abort_flag))) return false;
+        uint4* tile = reinterpret_cast<uint4*>(gbase + X * kTile);
+        // (eight pieces in flight: the warp has nothing else to hide shared memory's latency behind)
+        for (int i = lane; i < kTile / 16; i += 32 * 8) {
+            uint4 v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = tile[i + 32 * u];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                uint32_t* w = reinterpret_cast<uint32_t*>(&v[u]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[e]));
+                    w[e] = pack_f16_finite(f.x, f.y);
+                }
+                tile[i + 32 * u] = v[u];
+            }
+        }
+        fence_proxy_async_smem();
+        mbar_arrive(BAR(Q_CONV + X));
+        return true;
+    };
+
+    // Registers follow the work: the service warpgroup keeps 88 (56) per thread, the softmax groups take what is left
+    // (2*128*208 + 128*88 = 384*168; in-kernel de-quantisation: 2*128*168 + 128*56 + 128*112 <= 512*128).  A sum above what the
+    // launch has would wait forever.
+    constexpr int kServiceRegs = kSharedS && !kDequant ? 88 : 56, kSoftmaxRegs = kDequant ? 168 : kSharedS ? 208 : 224, kDequantRegs = kDequant ? 112 : 0;
+    static_assert(256 * kSoftmaxRegs + 128 * kServiceRegs + 128 * kDequantRegs <= (kDequant ? 512 * 128 : 384 * 168), "register split");
+    if (warp >= 8 && warp < 12) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kServiceRegs));
     if (warp >= 12) {
         // =============================== de-quantising K/V producers (paged) ===============================
         if constexpr (kDequant) {
-            asm volatile("setmaxnreg.dec.sync.aligned.u32 112;");
+            asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kDequantRegs));
             Item item;
             get_item(0, item);  // paged mode: exactly one item per CTA
             const int nkvA = item.nkvA, nkvB = item.nkvB, nmax = item.nmax, hk = item.hk;
@@ -809,51 +849,25 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 mbar_arrive(BAR(V_FULL + st));
             }
         }
-    } else if (warp >= 10) {
-        // idle warps of the service warpgroup; with gathered K/V and bf16 queries they turn the Q tiles into f16 where
-        // they lie (the swizzle only permutes 16-byte chunks, so an element-wise pass keeps the layout)
-        if constexpr (kGathered && kBf16) {
+    } else if (warp >= (kSharedS ? 11 : 10)) {
+        // idle warps of the service warpgroup; with gathered K/V and bf16 queries warp 11 turns the Q tiles A into f16
+        if constexpr (kConvertQ) {
             Item item;
-            const int tp = static_cast<int>(threadIdx.x) - 320;  // 0..63
             bool ok = true;
-            int qn[2] = {0, 0};  // Q tiles of each kind seen so far
-            for (int kk = 0; ok && get_item(kk, item); ++kk)
-#pragma unroll
-            for (int X = 0; X < 2; ++X) {
-                if ((X ? item.nkvB : item.nkvA) > 0) {
-                    ok = ok && __all_sync(0xffffffffu, mbar_wait(BAR(Q_FULL + X), qn[X] & 1, abort_flag));
-                    ++qn[X];
-                    if (ok) {
-                        uint4* tile = reinterpret_cast<uint4*>(gbase + X * kTile);
-                        // (eight pieces in flight: two warps have nothing else to hide shared memory's latency behind)
-                        for (int i = tp; i < kTile / 16; i += 64 * 8) {
-                            uint4 v[8];
-#pragma unroll
-                            for (int u = 0; u < 8; ++u) v[u] = tile[i + 64 * u];
-#pragma unroll
-                            for (int u = 0; u < 8; ++u) {
-                                uint32_t* w = reinterpret_cast<uint32_t*>(&v[u]);
-#pragma unroll
-                                for (int k = 0; k < 4; ++k) {
-                                    const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[k]));
-                                    w[k] = pack_f16_finite(f.x, f.y);
-                                }
-                                tile[i + 64 * u] = v[u];
-                            }
-                        }
-                        fence_proxy_async_smem();
-                        mbar_arrive(BAR(Q_CONV + X));
-                    }
-                }
-            }
+            int qn = 0;
+            for (int k = 0; ok && get_item(k, item); ++k)
+                if (item.nkvA > 0) ok = convert_q(0, qn++);
         }
     } else if (warp == 8) {
         // =============================== TMA producer ===============================
-        if (lane == 0) {
-            prefetch_tensormap(&tmQ);
-            if constexpr (!kDequant) {
-                prefetch_tensormap(&tmK);
-                prefetch_tensormap(&tmV);
+        const bool lead = lane == 0;  // (with bf16 queries the whole warp goes along and converts the Q tiles B)
+        if (lead || kConvertQ) {
+            if (lead) {
+                prefetch_tensormap(&tmQ);
+                if constexpr (!kDequant) {
+                    prefetch_tensormap(&tmK);
+                    prefetch_tensormap(&tmV);
+                }
             }
             // running counts over the items of this CTA: K/V tiles issued (ring position) and Q tiles loaded
             int g = 0, issued_k = 0, issued_v = 0, qn[2] = {0, 0};
@@ -864,6 +878,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 auto load_q = [&](int X) {
                     const int nkvX = X ? it.nkvB : it.nkvA;
                     if (nkvX == 0) return;
+                    if (!lead) { ++qn[X]; return; }
                     // the tile's previous occupant is free once its last QK^T has completed
                     if (qn[X] > 0 && !mbar_wait(BAR(Q_EMPTY + X), (qn[X] - 1) & 1, abort_flag)) { ok = false; return; }
                     mbar_expect_tx(BAR(Q_FULL + X), kTile);
@@ -879,55 +894,163 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 }
                 if constexpr (kKeySplit) {
                     // tiles in the order A0 B0 A1 B1 ..: stage 0 of the rings is A's, stage 1 is B's; both use A's queries
-                    for (int n = 0; ok && n < it.nkvA + it.nkvB; ++n) {
+                    const int total = it.nkvA + it.nkvB;
+                    auto load = [&](int n, bool is_v) {
+                        if (!ok || n >= total) return;
                         const int st = n & 1, j = n >> 1, row = (st ? it.nkvA + j : j) * kBN;
-                        if (j > 0 && !mbar_wait(BAR(K_EMPTY + st), (j - 1) & 1, abort_flag)) { ok = false; break; }
-                        mbar_expect_tx(BAR(K_FULL + st), kTile);
-                        tma_load_4d(sK + st * kTile, &tmK, BAR(K_FULL + st), 0, row, it.hk, it.b);
-                        if constexpr (kDim > 64) tma_load_4d(sK + st * kTile + kPanel, &tmK, BAR(K_FULL + st), 64, row, it.hk, it.b);
-                        ++issued_k;
-                        if (n == 0) load_q(0);
-                        if (j > 0 && !mbar_wait(BAR(V_EMPTY + st), (j - 1) & 1, abort_flag)) { ok = false; break; }
-                        mbar_expect_tx(BAR(V_FULL + st), kTile);
-                        tma_load_4d(sV + st * kTile, &tmV, BAR(V_FULL + st), 0, row, it.hk, it.b);
-                        if constexpr (kDim > 64) tma_load_4d(sV + st * kTile + kPanel, &tmV, BAR(V_FULL + st), 64, row, it.hk, it.b);
-                        ++issued_v;
+                        const int full = (is_v ? V_FULL : K_FULL) + st, empty = (is_v ? V_EMPTY : K_EMPTY) + st;
+                        const uint32_t dst = (is_v ? sV : sK) + st * kTile;
+                        const CUtensorMap* map = is_v ? &tmV : &tmK;
+                        if (j > 0 && !mbar_wait(BAR(empty), (j - 1) & 1, abort_flag)) { ok = false; return; }
+                        mbar_expect_tx(BAR(full), kTile);
+                        tma_load_4d(dst, map, BAR(full), 0, row, it.hk, it.b);
+                        if constexpr (kDim > 64) tma_load_4d(dst + kPanel, map, BAR(full), 64, row, it.hk, it.b);
+                        ++(is_v ? issued_v : issued_k);
+                    };
+                    load(0, false);
+                    load_q(0);
+                    load(1, false);
+                    load(0, true);
+                    load(1, true);
+                    load(2, false);
+                    for (int n = 2; ok && n < total; ++n) {  // (QK runs ahead of PV)
+                        load(n + 1, false);
+                        load(n, true);
                     }
                 } else if constexpr (!kDequant) {
                     // gathered mode: the sequence's keys start at row kv_row0 of the scratch, which is one [1, Hkv, rows, 128] tensor
                     const int kv_row0 = kGathered ? kv_row_base + it.kv_tile0 * kBN : 0;
-                    for (int j = 0; ok && j < it.nmax; ++j, ++g) {
-                        const int st = g & 1, n = g >> 1;
-                        if (n > 0 && !mbar_wait(BAR(K_EMPTY + st), (n - 1) & 1, abort_flag)) { ok = false; break; }
+                    auto load_k = [&](int j) {
+                        if (!lead) return;
+                        const int st = (g + j) & 1, n = (g + j) >> 1;
+                        if (n > 0 && !mbar_wait(BAR(K_EMPTY + st), (n - 1) & 1, abort_flag)) { ok = false; return; }
                         mbar_expect_tx(BAR(K_FULL + st), kTile);
                         tma_load_4d(sK + st * kTile, &tmK, BAR(K_FULL + st), 0, kv_row0 + j * kBN, it.hk, it.b);
                         if constexpr (kDim > 64)
                             tma_load_4d(sK + st * kTile + kPanel, &tmK, BAR(K_FULL + st), 64, kv_row0 + j * kBN, it.hk, it.b);
                         ++issued_k;
+                    };
+                    if (it.nmax > 0) load_k(0);
+                    for (int j = 0; j < it.nmax; ++j) {
                         if (j == 0) {  // (the first K tile has room before the previous item's last QK^T gives up the Q tiles)
-                            load_q(0);
+                            if (ok) load_q(0);
                             if (ok) load_q(1);
-                            if (!ok) break;
                         }
-                        if (n > 0 && !mbar_wait(BAR(V_EMPTY + st), (n - 1) & 1, abort_flag)) { ok = false; break; }
-                        mbar_expect_tx(BAR(V_FULL + st), kTile);
-                        tma_load_4d(sV + st * kTile, &tmV, BAR(V_FULL + st), 0, kv_row0 + j * kBN, it.hk, it.b);
-                        if constexpr (kDim > 64)
-                            tma_load_4d(sV + st * kTile + kPanel, &tmV, BAR(V_FULL + st), 64, kv_row0 + j * kBN, it.hk, it.b);
-                        ++issued_v;
+                        if (kSharedS && ok && j + 1 < it.nmax) load_k(j + 1);  // (QK runs ahead of PV)
+                        const int st = (g + j) & 1, n = (g + j) >> 1;
+                        if (lead && ok && n > 0 && !mbar_wait(BAR(V_EMPTY + st), (n - 1) & 1, abort_flag)) ok = false;
+                        if (kConvertQ) ok = __shfl_sync(0xffffffffu, ok, 0);  // (the only place where the warp's lanes part)
+                        if (!ok) break;
+                        if (lead) {
+                            mbar_expect_tx(BAR(V_FULL + st), kTile);
+                            tma_load_4d(sV + st * kTile, &tmV, BAR(V_FULL + st), 0, kv_row0 + j * kBN, it.hk, it.b);
+                            if constexpr (kDim > 64)
+                                tma_load_4d(sV + st * kTile + kPanel, &tmV, BAR(V_FULL + st), 64, kv_row0 + j * kBN, it.hk, it.b);
+                            ++issued_v;
+                        }
+                        if (!kSharedS && j + 1 < it.nmax) load_k(j + 1);
+                        if constexpr (kConvertQ)
+                            if (j == 0 && it.nkvB > 0) ok = convert_q(1, qn[1] - 1);
                     }
+                    g += it.nmax;
                 }
             }
-            if (*abort_flag) {  // let copies already in flight land before the CTA goes away
+            if (lead && *abort_flag) {  // let copies already in flight land before the CTA goes away
                 for (int X = 0; X < 2; ++X)
                     if (qn[X] > 0) mbar_drain(BAR(Q_FULL + X), (qn[X] - 1) & 1);
                 for (int jj = max(0, issued_k - 2); jj < issued_k; ++jj) mbar_drain(BAR(K_FULL + (jj & 1)), (jj >> 1) & 1);
                 for (int jj = max(0, issued_v - 2); jj < issued_v; ++jj) mbar_drain(BAR(V_FULL + (jj & 1)), (jj >> 1) & 1);
             }
         }
+    } else if (kSharedS && (warp == 9 || warp == 10)) {
+        // =============================== MMA issuers: QK and PV ===============================
+        if constexpr (kSharedS) {  // whole warps, converged (tcgen05.cuh)
+            auto wait_for = [&](int bar, int parity) { return __all_sync(0xffffffffu, mbar_wait(BAR(bar), parity, abort_flag)) != 0; };
+            // operand formats (A and B of one MMA must agree): dense mode as given; paged mode f16 throughout - the
+            // de-quantised values keep 11 significant bits and bf16 queries are converted in shared memory first
+            constexpr uint32_t idesc_qk = instr_desc_f16(kKvBf16, false, kBM, kBN);
+            constexpr uint32_t idesc_pv = instr_desc_f16(kKvBf16, true, kBM, kDim);
+            const uint64_t q_desc = smem_desc_sw128(sQ, 16, 1024), k_desc = smem_desc_sw128(sK, 16, 1024);  // K-major: Q and K tiles
+            const uint64_t v_desc = smem_desc_sw128(sV, kPanel, 1024);                                      // MN-major: V tiles
+            auto issue_qk = [&](int X, int st) {  // S_X = Q_X K^T : steps of 16 along D
+                constexpr uint32_t d = 0;
+                const uint64_t qa = q_desc + static_cast<uint32_t>((kKeySplit ? 0 : X) * (kTile >> 4)), ka = k_desc + static_cast<uint32_t>(st * (kTile >> 4));
+                mma_ss_x4<2, 2, idesc_qk>(d, qa, ka, 0u);
+                if constexpr (kDim > 64) mma_ss_x4<2, 2, idesc_qk>(d, qa + kPanel / 16, ka + kPanel / 16, 1u);
+            };
+            // O_X += P_X V : 8 steps of 16 along the keys, in two halves
+            auto issue_pv = [&](int X, int st, bool acc, int half) {
+                const uint32_t d = static_cast<uint32_t>(256 + X * 128);
+                const uint32_t pa = static_cast<uint32_t>(128 + X * 64 + half * 32);
+                const uint64_t va = v_desc + static_cast<uint32_t>(st * (kTile >> 4) + half * (4 * 2048 / 16));
+                mma_ts_x4<8, 2048 / 16, idesc_pv>(d, pa, va, acc ? 1u : 0u);
+            };
+            bool ok = true;
+            constexpr int kQReady = (kPaged && kBf16) ? Q_CONV : Q_FULL;
+            // running counts over the items of this CTA: K/V ring position, steps of each tile, Q tiles consumed
+            int g0 = 0, sx[2] = {0, 0}, qn[2] = {0, 0};
+            Item it;
+            if (warp == 9) {
+                // S has one place, which the tiles' turns A(0) B(0) A(1) B(1) .. share: QK of a turn is issued as soon as the
+                // turn before has its scores in registers, long before its own softmax warps are there.
+                int turns = 0;
+                for (int k = 0; ok && get_item(k, it); ++k) {
+#pragma unroll 1
+                    for (int j = 0; ok && j < it.nmax; ++j) {
+                        const int g = g0 + j;
+#pragma unroll
+                        for (int X = 0; X < 2; ++X) {
+                            const int nkvX = X ? it.nkvB : it.nkvA, st = kKeySplit ? X : g & 1;
+                            if (ok && j < nkvX) {
+                                if (kKeySplit || X == 0 || it.nkvA <= j) ok = wait_for(K_FULL + st, (kKeySplit ? j : g >> 1) & 1);
+                                if (j == 0 && !(kKeySplit && X)) ok = ok && wait_for(kQReady + X, qn[X]++ & 1);
+                                if (turns > 0) ok = ok && wait_for(S_FREE, (turns - 1) & 1);
+                                if (!ok) break;
+                                ++turns;
+                                tc_fence_after();
+                                issue_qk(X, st);
+                                mma_commit<true>(BAR(S_FULL + X));
+                                if (j + 1 == nkvX) mma_commit<true>(BAR(Q_EMPTY + X));  // last use of this Q tile: the producer may refill it
+                                if (kKeySplit) mma_commit<true>(BAR(K_EMPTY + st));
+                            }
+                        }
+                        if (!kKeySplit) mma_commit<true>(BAR(K_EMPTY + (g & 1)));
+                    }
+                    g0 += it.nmax;
+                }
+            } else {
+                // warp 10: PV of every turn when its P is ready
+                for (int k = 0; ok && get_item(k, it); ++k) {
+#pragma unroll 1
+                    for (int j = 0; ok && j < it.nmax; ++j) {
+                        const int g = g0 + j;
+#pragma unroll
+                        for (int X = 0; X < 2; ++X) {
+                            const int st = kKeySplit ? X : g & 1;
+                            if (ok && j < (X ? it.nkvB : it.nkvA)) {
+                                if (kKeySplit || X == 0 || it.nkvA <= j) ok = wait_for(V_FULL + st, (kKeySplit ? j : g >> 1) & 1);
+                                ok = ok && wait_for(P_READY + X, sx[X]++ & 1);
+                                if (!ok) break;
+                                tc_fence_after();
+                                issue_pv(X, st, j > 0, 0);
+                                issue_pv(X, st, true, 1);
+                                mma_commit<true>(BAR(O_DONE + X));
+                                if (kKeySplit) mma_commit<true>(BAR(V_EMPTY + st));
+                            }
+                        }
+                        if (!kKeySplit) mma_commit<true>(BAR(V_EMPTY + (g & 1)));
+                    }
+                    g0 += it.nmax;
+                }
+            }
+            mma_commit<true>(BAR(DRAIN));  // everything issued has completed before TMEM and shared memory are given up
+            mbar_drain(BAR(DRAIN), 0);
+        }
     } else if (warp == 9) {
-        // =============================== MMA issuer ===============================
-        if (lane == 0) {
+        // =============================== MMA issuer, a place of S per tile ===============================
+        // One lane: a step is a chain of waits here, and a vote of the warp behind each costs more than the faster issue gives
+        // (encoder batch of 8 x 16 heads x 512 tokens 27.0 us, by the whole warp 27.6).
+        if (!kSharedS && lane == 0) {
             // operand formats (A and B of one MMA must agree): dense mode as given; paged mode f16 throughout - the
             // de-quantised values keep 11 significant bits and bf16 queries are converted in shared memory first
             constexpr uint32_t idesc_qk = instr_desc_f16(kKvBf16, false, kBM, kBN);
@@ -983,8 +1106,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                         if (!ok) break;
                         tc_fence_after();
                         issue_qk(X, X);
-                        mma_commit(BAR(S_FULL + X));
-                        mma_commit(BAR(K_EMPTY + X));
+                        mma_commit<false>(BAR(S_FULL + X));
+                        mma_commit<false>(BAR(K_EMPTY + X));
                     }
                     for (int i = 0; ok && i < n; ++i) {
                         const int X = i & 1, j = i >> 1;
@@ -996,15 +1119,15 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                         if (!ok) break;
                         tc_fence_after();
                         issue_pv(X, X, true, 1);
-                        mma_commit(BAR(O_DONE + X));
-                        mma_commit(BAR(V_EMPTY + X));
+                        mma_commit<false>(BAR(O_DONE + X));
+                        mma_commit<false>(BAR(V_EMPTY + X));
                         if (i + 2 < n) {
                             ok = mbar_wait(BAR(K_FULL + X), (j + 1) & 1, abort_flag);
                             if (!ok) break;
                             tc_fence_after();
                             issue_qk(X, X);
-                            mma_commit(BAR(S_FULL + X));
-                            mma_commit(BAR(K_EMPTY + X));
+                            mma_commit<false>(BAR(S_FULL + X));
+                            mma_commit<false>(BAR(K_EMPTY + X));
                         }
                     }
                     break;  // one item per CTA
@@ -1015,18 +1138,18 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 tc_fence_after();
                 if (nkvA > 0) {  // (tile A starts as soon as its own operands are there)
                     issue_qk(0, g0 & 1);
-                    mma_commit(BAR(S_FULL + 0));
-                    if (nkvA == 1) mma_commit(BAR(Q_EMPTY + 0));  // last use of this Q tile: the producer may refill it
+                    mma_commit<false>(BAR(S_FULL + 0));
+                    if (nkvA == 1) mma_commit<false>(BAR(Q_EMPTY + 0));  // last use of this Q tile: the producer may refill it
                 }
                 if (nkvB > 0) {
                     ok = mbar_wait(BAR(kQReady + 1), qn[1] & 1, abort_flag);
                     if (!ok) break;
                     tc_fence_after();
                     issue_qk(1, g0 & 1);
-                    mma_commit(BAR(S_FULL + 1));
-                    if (nkvB == 1) mma_commit(BAR(Q_EMPTY + 1));
+                    mma_commit<false>(BAR(S_FULL + 1));
+                    if (nkvB == 1) mma_commit<false>(BAR(Q_EMPTY + 1));
                 }
-                mma_commit(BAR(K_EMPTY + (g0 & 1)));
+                mma_commit<false>(BAR(K_EMPTY + (g0 & 1)));
                 for (int j = 0; ok && j < nmax; ++j) {
                     const int g = g0 + j, stv = g & 1;
                     if (!mbar_wait(BAR(V_FULL + stv), (g >> 1) & 1, abort_flag)) { ok = false; break; }
@@ -1042,7 +1165,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                             if (!mbar_wait(BAR(P_READY + X), par, abort_flag)) { ok = false; break; }
                             tc_fence_after();
                             issue_pv(X, stv, true, 1);
-                            mma_commit(BAR(O_DONE + X));
+                            mma_commit<false>(BAR(O_DONE + X));
                         }
                         if (ok && j + 1 < nkvX) {
                             if (!k_next_ready) {
@@ -1051,13 +1174,13 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                                 tc_fence_after();
                             }
                             issue_qk(X, (g + 1) & 1);
-                            mma_commit(BAR(S_FULL + X));
-                            if (j + 2 == nkvX) mma_commit(BAR(Q_EMPTY + X));
+                            mma_commit<false>(BAR(S_FULL + X));
+                            if (j + 2 == nkvX) mma_commit<false>(BAR(Q_EMPTY + X));
                         }
                     }
                     if (!ok) break;
-                    mma_commit(BAR(V_EMPTY + stv));
-                    if (j + 1 < nmax) mma_commit(BAR(K_EMPTY + ((g + 1) & 1)));
+                    mma_commit<false>(BAR(V_EMPTY + stv));
+                    if (j + 1 < nmax) mma_commit<false>(BAR(K_EMPTY + ((g + 1) & 1)));
                 }
                 g0 += nmax;
                 sx[0] += nkvA;
@@ -1065,20 +1188,17 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 qn[0] += nkvA > 0;
                 qn[1] += nkvB > 0;
             }
-            mma_commit(BAR(DRAIN));  // everything issued has completed before TMEM and shared memory are given up
+            mma_commit<false>(BAR(DRAIN));  // everything issued has completed before TMEM and shared memory are given up
             mbar_drain(BAR(DRAIN), 0);
         }
     } else {
         // =============================== softmax + epilogue of tile X ===============================
-        if constexpr (kDequant) {
-            asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
-        } else {
-            asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
-        }
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
         const int X = warp >> 2;
         const int r = static_cast<int>(threadIdx.x) - X * 128;
         const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-        const uint32_t tS = tmem + lane_base + static_cast<uint32_t>(X * 128);
+        const uint32_t tS = tmem + lane_base + static_cast<uint32_t>(kSharedS ? 0 : X * 128);
+        const uint32_t tP = tmem + lane_base + static_cast<uint32_t>(kSharedS ? 128 + X * 64 : X * 128);
         const uint32_t tO = tmem + lane_base + static_cast<uint32_t>(256 + X * 128);
         // 32 columns of an accumulator
         auto load_o = [&](uint32_t t, int q, uint32_t (&o)[32]) {
@@ -1153,6 +1273,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 #pragma unroll
                 for (int q = 0; q < 4; ++q) tmem_ld32(tS + 32 * q, s[q]);
                 tmem_wait_ld();
+                if constexpr (kSharedS) {  // the other tile's scores may come
+                    tc_fence_before();
+                    mbar_arrive(BAR(S_FREE));
+                }
                 const int key0 = (tile0 + j) * kBN;
                 if constexpr (kMask == 3) {
                     if ((mword[0] & mword[1] & mword[2] & mword[3]) != 0xffffffffu) {
@@ -1269,6 +1393,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                     m_used = m_new;
                     l *= alpha;
                 }
+                if (kSharedS && j > 0) {  // PV(j-1) has read P's columns.  (Waited for in the middle of the exponentials it cost 7 %.)
+                    ok = __all_sync(0xffffffffu, mbar_wait(BAR(O_DONE + X), (sxb + j - 1) & 1, abort_flag));
+                    tc_fence_after();
+                }
                 // P = exp2(S*c - m): the scale-and-shift and the row sum run two elements per instruction (f32x2).  (f16 in
                 // pieces: 2^7 P, at most 2^15, so that the pieces reach as far down as they can; the sum carries the factor too)
                 const float shift = kLowAcc ? 7.f - m_used : -m_used;
@@ -1294,11 +1422,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                             pk[i] = pack2<kKvBf16>(p0, p1);
                         }
                     }
-                    tmem_st16(tS + 16 * q, pk);  // P over the first 64 columns of S, behind what was already read
+                    tmem_st16(tP + 16 * q, pk);  // (pieces of P: over S's columns, all of which have been read)
                     if constexpr (kSplitP) tmem_st16(tS + 64 + 16 * q, pk_lo);  // (all of S is in registers by now)
                     if constexpr (kThirdPiece) tmem_st16(tO + kDim + 16 * q, pk_third);
                     // first 64 keys of P are in TMEM: PV can start on them, unless O still has to be rescaled
-                    if (q == 1 && !(need_any && j > 0)) {
+                    if (!kSharedS && q == 1 && !(need_any && j > 0)) {
                         tmem_wait_st();
                         tc_fence_before();
                         mbar_arrive(BAR(P_HALF + X));
@@ -1311,9 +1439,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 }
                 if (need_any && j > 0) {
                     // O_X still holds the old scale; PV_X(j-1) must have landed before it is touched
-                    ok = __all_sync(0xffffffffu, mbar_wait(BAR(O_DONE + X), (sxb + j - 1) & 1, abort_flag));
+                    if constexpr (!kSharedS) {
+                        ok = __all_sync(0xffffffffu, mbar_wait(BAR(O_DONE + X), (sxb + j - 1) & 1, abort_flag));
+                        tc_fence_after();
+                    }
                     if (!ok) break;
-                    tc_fence_after();
 #pragma unroll
                     for (int q = 0; q < (kLowAcc ? 2 : 1) * kDim / 32; ++q) {
                         uint32_t o[32];
@@ -1323,10 +1453,13 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                         for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
                         tmem_st32(tO + 32 * q, o);
                     }
-                    tmem_wait_st();
-                    tc_fence_before();
-                    mbar_arrive(BAR(P_HALF + X));
+                    if constexpr (!kSharedS) {
+                        tmem_wait_st();
+                        tc_fence_before();
+                        mbar_arrive(BAR(P_HALF + X));
+                    }
                 }
+                if (kSharedS && !ok) break;
                 tmem_wait_st();
                 tc_fence_before();
                 mbar_arrive(BAR(P_READY + X));

@@ -163,29 +163,7 @@ __host__ __device__ constexpr uint32_t instr_desc_f16(bool bf16, bool b_mn_major
     return instr_desc_f16_ab(bf16, bf16, b_mn_major, m, n);
 }
 
-// D[tmem] (+)= A[smem] . B[smem]; issued by ONE thread
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-        "}\n" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(static_cast<uint32_t>(accumulate))
-        : "memory");
-}
-// D[tmem] (+)= A[tmem] . B[smem]
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, bool accumulate) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
-        "}\n" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(static_cast<uint32_t>(accumulate))
-        : "memory");
-}
-// Register-lean forms for unrolled issue loops: the 64-bit descriptors are put together inside the asm block from a
+// D[tmem] (+)= A . B, issued by ONE thread, A in shared memory or in tensor memory.  The 64-bit descriptors are put together inside the asm block from a
 // 32-bit base (low word of the descriptor of the tile's first byte), a compile-time offset in 16-byte units and a
 // compile-time high word, so that the compiler has one live register per tile instead of one per MMA.
 __device__ __host__ constexpr uint32_t desc_lo_sw128(uint32_t lbo_bytes) { return ((lbo_bytes >> 4) & 0x3FFFu) << 16; }
@@ -227,9 +205,78 @@ __device__ __forceinline__ void mma_ts_c(uint32_t d_tmem, uint32_t a_tmem, uint3
         "r"(a_tmem), "r"(b_addr16), "r"(accumulate), "n"(kOffA), "n"(kOffB + kLoB), "n"(kHiB), "n"(kIdesc)
         : "memory");
 }
-// the mbarrier receives one arrival when every MMA issued so far by this thread has completed
+// Four instructions, the operands' descriptors a constant number of 16-byte units (TMEM columns) apart.  The WHOLE warp
+// executes this (and mma_commit<true>), converged; one elected lane - the same every time - issues.  Descriptors and predicates are
+// warp-uniform then, which is what the instruction wants: a single lane in a branch of its own moves every one of them over
+// first.  Cycles of the issuing warp for eight instructions of M = N = 128, K = 16 (the tensor core takes 512): a lane in
+// a branch 436, elected one by one 303, elected four a block 174; and four of them between a wait and a commit 450 and 266.
+template <uint32_t kStepA, uint32_t kStepB, uint32_t kIdesc>
+__device__ __forceinline__ void mma_ss_x4(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p, e, t;\n"
+        ".reg .b64 a1, a2, a3, b1, b2, b3;\n"
+        ".reg .b32 id;\n"
+        "setp.ne.b32 p, %3, 0;\n"
+        "setp.eq.b32 t, 0, 0;\n"
+        "mov.b32 id, %4;\n"
+        "elect.sync _|e, 0xffffffff;\n"
+        "add.s64 a1, %1, %5;\n"
+        "add.s64 a2, %1, %6;\n"
+        "add.s64 a3, %1, %7;\n"
+        "add.s64 b1, %2, %8;\n"
+        "add.s64 b2, %2, %9;\n"
+        "add.s64 b3, %2, %10;\n"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, id, p;\n"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, id, t;\n"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, id, t;\n"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, id, t;\n"
+        "}\n" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(accumulate), "n"(kIdesc), "n"(kStepA), "n"(2 * kStepA), "n"(3 * kStepA), "n"(kStepB),
+        "n"(2 * kStepB), "n"(3 * kStepB)
+        : "memory");
+}
+// the same with A in tensor memory
+template <uint32_t kStepA, uint32_t kStepB, uint32_t kIdesc>
+__device__ __forceinline__ void mma_ts_x4(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p, e, t;\n"
+        ".reg .b64 b1, b2, b3;\n"
+        ".reg .b32 id, a1, a2, a3;\n"
+        "setp.ne.b32 p, %3, 0;\n"
+        "setp.eq.b32 t, 0, 0;\n"
+        "mov.b32 id, %4;\n"
+        "elect.sync _|e, 0xffffffff;\n"
+        "add.u32 a1, %1, %5;\n"
+        "add.u32 a2, %1, %6;\n"
+        "add.u32 a3, %1, %7;\n"
+        "add.s64 b1, %2, %8;\n"
+        "add.s64 b2, %2, %9;\n"
+        "add.s64 b3, %2, %10;\n"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, id, p;\n"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, id, t;\n"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, id, t;\n"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, id, t;\n"
+        "}\n" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(b_desc), "r"(accumulate), "n"(kIdesc), "n"(kStepA), "n"(2 * kStepA), "n"(3 * kStepA), "n"(kStepB),
+        "n"(2 * kStepB), "n"(3 * kStepB)
+        : "memory");
+}
+// the mbarrier receives one arrival when every MMA issued so far by this thread, or the warp's elected lane, has completed
+template <bool kWarp>
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    if constexpr (kWarp) {
+        asm volatile(
+            "{\n"
+            ".reg .pred e;\n"
+            "elect.sync _|e, 0xffffffff;\n"
+            "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
+            "}\n" ::"r"(bar)
+            : "memory");
+    } else {
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    }
 }
 
 }  // namespace tc

@@ -17,7 +17,7 @@
 //
 // Measured on a B200 (graph replay): bf16, 8 sequences x 3003 keys x 8 KV heads, additive mask (98 MB): 2049 us on
 // attn_generic_kernel before, 21.2 us now (4.6 TB/s; 15.1 us at the copy rate); 32 bf16 sequences of 256..4096 tokens in
-// a pool (293 MB, with the store of the step): 8149 us before, 57.3 us now (5.1 TB/s; 44.8 us at the copy rate).
+// a pool (293 MB, with the store of the step): 8149 us before, 53.2 us now (5.5 TB/s; 44.8 us at the copy rate).
 // On another box and before a cheaper floor for the mask: two bf16 pieces, which keep 2^-16 of a probability, 22.8 and 55.3 us,
 // three 23.3 and 56.5, two tf32 pieces beside V widened to tf32 24.0 and 59.5.
 #include <algorithm>
@@ -47,6 +47,7 @@ struct Dec16Params {
     // paged pools: k_h / v_h are the chunk sizes, k_b / v_b the block sizes, k_s / v_s the rows
     PagedTables t;
     int sliding_window;
+    int cache_rows_settled;  // b2a_paged_desc: the kernel before this one writes no cache row but the new tokens'
     int32_t* status;
 };
 
@@ -177,7 +178,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attn_decode16_kernel(const Dec
 
     // ---- the keys of this (sequence, KV head), in 16-key tiles
     int kv_end = 0, first_pos = 0, tok = 0, bib0 = 0;
-    bool bad = false;
+    bool bad = false, decode_row = true;
     if constexpr (kPaged) {
         tok = __ldcg(p.t.subsequence_begins + seq);
         const int tok_end = __ldcg(p.t.subsequence_begins + seq + 1);
@@ -186,13 +187,9 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attn_decode16_kernel(const Dec
         const int bib1 = __ldcg(p.t.block_indices_begins + seq + 1);
         kv_end = past + 1;
         first_pos = p.sliding_window > 0 ? max(0, kv_end - p.sliding_window) : 0;
-        const bool decode_row = tok_end - tok == 1;  // the others belong to the multi-token kernel
+        decode_row = tok_end - tok == 1;  // the others belong to the multi-token kernel
         bad = decode_row && (past < 0 || tok < 0 || tok >= p.t.num_tokens ||
                              (kv_end + p.t.block_size - 1) / p.t.block_size > bib1 - bib0);
-        grid_dependency_wait();
-        grid_launch_dependents();
-        if (bad && split == 0 && tid == 0) report(p.status, B2A_DEV_BAD_LEN);
-        if (!decode_row || bad) return;  // the same decision in every CTA of the cluster
     } else {
         kv_end = p.causal ? min(p.Skv, p.Sq) : p.Skv;
         grid_dependency_wait();
@@ -202,7 +199,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attn_decode16_kernel(const Dec
     const int tiles = (kv_end + kTileKeys - 1) / kTileKeys - tile_lo;
     const int per_cta = (tiles + csize - 1) / csize;
     const int my_lo = tile_lo + min(tiles, split * per_cta), my_hi = tile_lo + min(tiles, (split + 1) * per_cta);
-    const int n_w = max(0, (my_hi - my_lo - warp + kWarps - 1) / kWarps);  // tiles my_lo + warp + kWarps * i
+    const int n_w = decode_row && !bad ? max(0, (my_hi - my_lo - warp + kWarps - 1) / kWarps) : 0;  // tiles my_lo + warp + kWarps * i
 
     const uint32_t smem_warp = static_cast<uint32_t>(__cvta_generic_to_shared(smem)) + warp * (kStages * tile_bytes<D>());
     const uint64_t policy = evict_first_policy();
@@ -210,13 +207,14 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attn_decode16_kernel(const Dec
     // follows the copies and a stage remembers in a bit whether its block was usable
     int window_ids = -1;
     uint32_t stage_ok = 0;
+    bool bad_block = false;
     auto load_window = [&](int i0) {
         window_ids = -1;
         if (i0 + lane < n_w) {
             const int key = (my_lo + warp + kWarps * (i0 + lane)) * kTileKeys;
             window_ids = __ldcg(p.t.block_indices + bib0 + key / p.t.block_size);
             if (window_ids < 0 || window_ids >= p.t.num_blocks_total) {
-                report(p.status, B2A_DEV_BAD_BLOCK);
+                bad_block = true;
                 window_ids = -1;
             }
         }
@@ -261,11 +259,32 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attn_decode16_kernel(const Dec
             cp_async16z(st + kHalfTile + off, in ? vs + at_v : vb, in ? 16 : 0, policy);
         }
     };
-    if constexpr (kPaged) load_window(0);
+    auto fill = [&]() {
 #pragma unroll
-    for (int s = 0; s < kStages - 1; ++s) {
-        if (s < n_w) issue(s);
-        cp_async_commit();
+        for (int s = 0; s < kStages - 1; ++s) {
+            if (s < n_w) issue(s);
+            cp_async_commit();
+        }
+    };
+    if constexpr (kPaged) {
+        // The step's tables exist before its kernels are launched, so the block ids are read while the kernel in front, the step's
+        // store, drains; and with the caller's promise that it writes no cache row but the new tokens', each in its
+        // sequence's last tile, so are the first tiles of a warp that does not reach that one.  (With the store's own kernel
+        // for such pools, 32 sequences of 256..4096 tokens x 8 KV heads, bf16: 56.3 -> 53.2 us a step.)
+        load_window(0);
+        const int last_tile = tile_lo + tiles - 1;
+        const bool early = p.cache_rows_settled && (my_hi - 1 < last_tile || my_lo + warp + kWarps * (kStages - 2) < last_tile);
+        if (early) fill();
+        grid_dependency_wait();
+        grid_launch_dependents();
+        if (bad && split == 0 && tid == 0) report(p.status, B2A_DEV_BAD_LEN);
+        if (!decode_row || bad) {  // the same decision in every CTA of the cluster
+            cp_async_wait<0>();
+            return;
+        }
+        if (!early) fill();
+    } else {
+        fill();
     }
 
     // ---- query rows as the B operand of S^T = K Q^T: row r = g * Sq + i is query position i of the group's head g
@@ -405,6 +424,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attn_decode16_kernel(const Dec
     }
     cp_async_wait<0>();
     __syncwarp();
+    if (bad_block) report(p.status, B2A_DEV_BAD_BLOCK);
 
     // ---- the warp's partial into its own stage memory
     constexpr int GP = NT * 8;
@@ -608,6 +628,7 @@ int paged_decode16_launch(const b2a_paged_desc& d, const void* query, const void
     p.k_b = p.v_b = d.Hkv * p.k_h;
     p.t = t;
     p.sliding_window = d.sliding_window;
+    p.cache_rows_settled = d.cache_rows_settled;
     p.status = status;
     const int keys = d.sliding_window > 0 ? std::min(d.sliding_window, d.max_context_len) : d.max_context_len;
     return launch_any(d.kv_dtype, p, d.D, true, keys, d.Hkv, d.num_seqs, stream);

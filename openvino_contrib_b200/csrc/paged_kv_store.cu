@@ -338,6 +338,58 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kRope ? 2 : 4) paged_kv_sto
     }
 }
 
+// A pool of the rows' own 16-bit type: the rows are copied, a thread per 16 bytes of a token's key or value rows, K first.  Bound by
+// its chain of loads: rows and tables in one trip (the entries on the guess that the token is its sequence's only one, as
+// above), the block id in a second, where a warp per row with the search in front took seven.  (Through float32 and back, as
+// every 16-bit row is stored: only a NaN's bits change.)
+template <typename T>
+__global__ void __launch_bounds__(256) paged_kv_copy_rows_kernel(const StoreParams p, const int pieces_per_token) {
+    const int lane = threadIdx.x & 31;
+    const long long piece = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+    const int tok = static_cast<int>(piece / pieces_per_token);  // (a multiple of 32 pieces a token: the same in all of a warp)
+    const int at = static_cast<int>(piece - static_cast<long long>(tok) * pieces_per_token);
+    grid_dependency_wait();  // the new key/value rows (and the pool's previous readers) belong to earlier kernels
+    grid_launch_dependents();
+    if (tok >= p.t.num_tokens) return;
+    const int half = pieces_per_token / 2, which = at >= half, e = at - which * half;  // 0 = key, 1 = value
+    uint4 row = reinterpret_cast<const uint4*>(which ? p.value : p.key)[static_cast<size_t>(tok) * half + e];
+    int seq = -1, past = 0, begin = 0, bib0 = 0, bib1 = 0;
+    if (tok < p.t.num_seqs) {
+        const int b0 = p.t.subsequence_begins[0], bn = p.t.subsequence_begins[p.t.num_seqs];
+        const int mine = p.t.subsequence_begins[tok], after = p.t.subsequence_begins[tok + 1];
+        past = p.t.past_lens[tok];
+        bib0 = p.t.block_indices_begins[tok];
+        bib1 = p.t.block_indices_begins[tok + 1];
+        begin = mine;
+        if (mine <= tok && tok < after && b0 <= tok && tok < bn) seq = tok;
+    }
+    if (seq < 0) {
+        seq = find_sequence(p.t, tok, lane);
+        if (seq < 0) return;  // not scheduled
+        past = p.t.past_lens[seq];
+        begin = p.t.subsequence_begins[seq];
+        bib0 = p.t.block_indices_begins[seq];
+        bib1 = p.t.block_indices_begins[seq + 1];
+    }
+    const int pos = past + (tok - begin), bs = p.t.block_size;
+    if (pos < 0 || pos / bs >= bib1 - bib0) {
+        if (lane == 0) report(p.status, B2A_DEV_BAD_LEN);
+        return;
+    }
+    const int blk = p.t.block_indices[bib0 + pos / bs];
+    if (blk < 0 || blk >= p.t.num_blocks_total) {
+        if (lane == 0) report(p.status, B2A_DEV_BAD_BLOCK);
+        return;
+    }
+    const int row_pieces = p.D / 8, hk = e / row_pieces;
+    uint4* dst = reinterpret_cast<uint4*>(which ? p.v_cache : p.k_cache) +
+                 ((static_cast<size_t>(blk) * p.Hkv + hk) * bs + pos % bs) * row_pieces + (e - hk * row_pieces);
+    T* h = reinterpret_cast<T*>(&row);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) h[i] = from_f32<T>(to_f32<T>(h[i]));
+    *dst = row;
+}
+
 }  // namespace
 
 int paged_kv_store_launch(const b2a_paged_desc& d, const void* key, const void* value, void* k_cache, void* v_cache,
@@ -368,6 +420,15 @@ int paged_kv_store_launch(const b2a_paged_desc& d, const void* key, const void* 
             e = rope_all ? launch_overlapped(paged_kv_store_rows128_kernel<__nv_bfloat16, true>, dim3(grid_t), block, 0, stream, p, per_warp)
                          : launch_overlapped(paged_kv_store_rows128_kernel<__nv_bfloat16, false>, dim3(grid_t), block, 0, stream, p, per_warp);
         return e == cudaSuccess ? B2A_OK : B2A_ERR_CUDA;
+    }
+    // (equal head sizes, and whole warps per token)
+    const long long pieces = 2LL * d.Hkv * d.D / 8;
+    if (d.kv_dtype != B2A_U8 && d.kv_dtype == d.q_dtype && d.D == d.Dv && d.D % 8 == 0 && pieces % 32 == 0 && pieces < (1 << 20) &&
+        p.rotary_dim == 0 && al8(key) && al8(value) && al8(k_cache) && al8(v_cache)) {
+        const unsigned grid_c = static_cast<unsigned>((pieces * d.num_tokens + 255) / 256);
+        return launch_overlapped(d.kv_dtype == B2A_F16 ? paged_kv_copy_rows_kernel<__half> : paged_kv_copy_rows_kernel<__nv_bfloat16>, dim3(grid_c), dim3(256), 0, stream, p, static_cast<int>(pieces)) == cudaSuccess
+                   ? B2A_OK
+                   : B2A_ERR_CUDA;
     }
     const long long total = 2LL * d.num_tokens * d.Hkv;
     const unsigned grid = static_cast<unsigned>((total + kWarpsPerCta - 1) / kWarpsPerCta);

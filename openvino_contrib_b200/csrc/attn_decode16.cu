@@ -17,7 +17,7 @@
 //
 // Measured on a B200 (graph replay): bf16, 8 sequences x 3003 keys x 8 KV heads, additive mask (98 MB): 2049 us on
 // attn_generic_kernel before, 21.2 us now (4.6 TB/s; 15.1 us at the copy rate); 32 bf16 sequences of 256..4096 tokens in
-// a pool (293 MB, with the store of the step): 8149 us before, 53.2 us now (5.5 TB/s; 44.8 us at the copy rate).
+// a pool (293 MB, with the store of the step): 8149 us before, 52.3 us now (5.6 TB/s; 44.8 us at the copy rate).
 // On another box and before a cheaper floor for the mask: two bf16 pieces, which keep 2^-16 of a probability, 22.8 and 55.3 us,
 // three 23.3 and 56.5, two tf32 pieces beside V widened to tf32 24.0 and 59.5.
 #include <algorithm>
@@ -47,7 +47,6 @@ struct Dec16Params {
     // paged pools: k_h / v_h are the chunk sizes, k_b / v_b the block sizes, k_s / v_s the rows
     PagedTables t;
     int sliding_window;
-    int cache_rows_settled;  // b2a_paged_desc: the kernel before this one writes no cache row but the new tokens'
     int32_t* status;
 };
 
@@ -267,25 +266,28 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attn_decode16_kernel(const Dec
         }
     };
     if constexpr (kPaged) {
-        // The step's tables exist before its kernels are launched, so the block ids are read while the kernel in front, the step's
-        // store, drains; and with the caller's promise that it writes no cache row but the new tokens', each in its
-        // sequence's last tile, so are the first tiles of a warp that does not reach that one.  (With the store's own kernel
-        // for such pools, 32 sequences of 256..4096 tokens x 8 KV heads, bf16: 56.3 -> 53.2 us a step.)
+        // The step's tables exist before its kernels are launched, so the block ids are read while the kernel in front, as a rule
+        // the step's store, drains, and the first tiles are asked into L2.  Not into shared memory: a block that this sequence
+        // holds as cached may be one that another sequence's new token goes into (prefixes shared within a step), and only
+        // what is read behind the wait is sure to show that row.  Cold pools, f16, 8 KV heads, us a step with the store, without
+        // the prefetch and with it: 2 sequences of 300..900 tokens 7.9 and 7.5, 8 of 2000 21.4 and 20.3, 32 of 256..4096 53.7
+        // and 51.7.  (Copies into shared memory here, of the tiles before a sequence's last: 7.2, 21.1 and 53.1.)
         load_window(0);
-        const int last_tile = tile_lo + tiles - 1;
-        const bool early = p.cache_rows_settled && (my_hi - 1 < last_tile || my_lo + warp + kWarps * (kStages - 2) < last_tile);
-        if (early) fill();
+#pragma unroll
+        for (int s = 0; s < kStages - 1; ++s) {
+            const int phys = __shfl_sync(0xffffffffu, window_ids, s);
+            if (s < n_w && phys >= 0 && lane < 2) {
+                const int key0 = (my_lo + warp + kWarps * s) * kTileKeys;
+                const int64_t at = static_cast<int64_t>(phys) * p.k_b + key0 % p.t.block_size * kRowBytes;
+                prefetch_l2((lane == 0 ? kb : vb) + at, kHalfTile);
+            }
+        }
         grid_dependency_wait();
         grid_launch_dependents();
         if (bad && split == 0 && tid == 0) report(p.status, B2A_DEV_BAD_LEN);
-        if (!decode_row || bad) {  // the same decision in every CTA of the cluster
-            cp_async_wait<0>();
-            return;
-        }
-        if (!early) fill();
-    } else {
-        fill();
+        if (!decode_row || bad) return;  // the same decision in every CTA of the cluster
     }
+    fill();
 
     // ---- query rows as the B operand of S^T = K Q^T: row r = g * Sq + i is query position i of the group's head g
     auto row_base = [&](const uint8_t* base, int64_t sb, int64_t sh, int64_t ss, int r) {
@@ -628,7 +630,6 @@ int paged_decode16_launch(const b2a_paged_desc& d, const void* query, const void
     p.k_b = p.v_b = d.Hkv * p.k_h;
     p.t = t;
     p.sliding_window = d.sliding_window;
-    p.cache_rows_settled = d.cache_rows_settled;
     p.status = status;
     const int keys = d.sliding_window > 0 ? std::min(d.sliding_window, d.max_context_len) : d.max_context_len;
     return launch_any(d.kv_dtype, p, d.D, true, keys, d.Hkv, d.num_seqs, stream);

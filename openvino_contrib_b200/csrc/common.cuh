@@ -125,6 +125,11 @@ struct ProbPieces<__nv_bfloat16> {
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// `bytes` from `src` (both in whole 16-byte pieces) on their way to L2
+__device__ __forceinline__ void prefetch_l2(const void* src, int bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(src), "r"(bytes) : "memory");
+}
+
 template <typename... KernelArgs, typename... Args>
 inline cudaError_t launch_overlapped(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                      Args&&... args) {

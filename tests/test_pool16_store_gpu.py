@@ -39,22 +39,73 @@ def test_rows_land_in_their_blocks(dtype, hkv, d, block_size, new):
         np.testing.assert_array_equal(pool.cpu().numpy().view(np.uint16).reshape(want.shape), want)
 
 
+def attention_rows(q, pools, past, t, hq, hkv, d, block_size, window):
+    """One new token per sequence over pools [blocks, hkv, block_size, d], in float64."""
+    out = np.zeros((len(q), hq, d))
+    for s, p in enumerate(past):
+        blocks = t[2][t[3][s]:t[3][s + 1]]
+        keys, values = (x[blocks].transpose(1, 0, 2, 3).reshape(hkv, -1, d)[:, :p + 1] for x in pools)
+        lo = max(0, p + 1 - window) if window else 0
+        for h in range(hq):
+            sc = keys[h * hkv // hq, lo:] @ q[s].reshape(hq, d)[h] / np.sqrt(d)
+            e = np.exp(sc - sc.max())
+            out[s, h] = e / e.sum() @ values[h * hkv // hq, lo:]
+    return out.reshape(len(q), hq * d)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("window", [0, 40])
-def test_settled_rows_give_the_same_bits(d, window):
+@pytest.mark.parametrize("captured", [False, True])
+def test_steps_through_the_operator_see_their_new_rows(dtype, d, window, captured):
+    # Store, attention, store, attention ..: the attention reads block ids, and asks for its first tiles, while the store in front
+    # of it drains.  The slots of all new tokens hold NaN in the beginning, so a row that was read too early shows; the new
+    # row is the first of a block, its last, and one inside, in contexts of one tile and of many.
     import openvino_contrib_b200 as b2a
-    past, hkv, hq = [0, 15, 16, 17, 300, 2047, 2048, 5000], 2, 8
-    t = tables(past, [1] * len(past), 16, 2)
-    dev = [torch.from_numpy(x).cuda() for x in t]
-    cache = b2a.PagedKvCache.allocate(int(t[2].max()) + 1, hkv, d, 16, torch.float16)
-    cache.k.view(torch.float16).normal_(), cache.v.view(torch.float16).normal_()
-    q, k, v = (torch.randn(len(past), h * d, device="cuda").half() for h in (hq, hkv, hkv))
-    outs = []
-    for settled in (False, True):
-        status = torch.zeros(1, dtype=torch.int32, device="cuda")
-        b2a.paged_kv_store(k, v, cache, *dev, status=status)
-        outs.append(b2a.paged_attention(q, cache, *dev, hq=hq, max_context_len=5001, max_q_len=1, sliding_window=window, status=status,
-                                        cache_rows_settled=settled))
+    past0, hkv, hq, steps = [0, 15, 16, 14, 300, 2047, 2048, 5000], 2, 8, 3
+    n = len(past0)
+    t = tables(past0, [steps] * n, 16, 2)
+    begins = np.arange(n + 1, dtype=np.int32)
+    g = torch.Generator().manual_seed(d + window)
+    filled = torch.randn(2, int(t[2].max()) + 1, hkv, 16, d, generator=g).to(dtype)
+    for s, p in enumerate(past0):
+        for pos in range(p, p + steps):
+            filled[:, t[2][t[3][s] + pos // 16], :, pos % 16] = float("nan")
+    rows = [[torch.randn(n, h * d, generator=g).to(dtype) for h in (hq, hkv, hkv)] for _ in range(steps)]
+    cache = b2a.PagedKvCache.allocate(filled.shape[1], hkv, d, 16, dtype)
+    op = b2a.PagedAttentionOp(hq, hkv, d, 16, dtype, max_seqs=n, max_context_len=5100, sliding_window=window, q_dtype=dtype)
+    work = {"mutable": [torch.empty(m, dtype=torch.uint8, device="cuda") for m in op.GetWorkBufferRequest()["mutable_sizes"]]}
+    pasts = [torch.tensor(past0, dtype=torch.int32, device="cuda") + i for i in range(steps)]
+    dev = [torch.from_numpy(x).cuda() for x in (begins, t[2], t[3])]
+    ins = [[x.cuda() for x in r] for r in rows]
+    outs = [torch.empty(n, hq * d, dtype=dtype, device="cuda") for _ in range(steps)]
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    fresh = filled.cuda()
+
+    def run():
+        for pool, x in zip((cache.k, cache.v), fresh):
+            pool.view(dtype).view(x.shape).copy_(x)
+        for i in range(steps):
+            op.Execute([*ins[i], cache.k, cache.v, pasts[i], *dev, None, window], [outs[i]], workbuffers=work, status=status)
+
+    if captured:
+        graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.graph(graph, stream=side):
+            run()
+        torch.cuda.synchronize()
+        run = graph.replay
+    for _ in range(2):  # (the second time from the pool with its NaNs again)
+        run()
         assert int(status.item()) == 0
-        k, v = k.clone(), v.clone()
-    assert torch.equal(*outs)
+        pools = [x.double().numpy() for x in filled]
+        u = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8
+        for i in range(steps):
+            q, k, v = (x.double().numpy() for x in rows[i])
+            for s, p in enumerate(past0):
+                at = t[2][t[3][s] + (p + i) // 16], slice(None), (p + i) % 16
+                pools[0][at], pools[1][at] = k[s].reshape(hkv, d), v[s].reshape(hkv, d)
+            ref = attention_rows(q, pools, [p + i for p in past0], t, hq, hkv, d, 16, window)
+            # the result is rounded to the type; sums and probabilities are float32's (5000 terms of order one)
+            err = np.abs(outs[i].double().cpu().numpy() - ref)
+            assert (err <= u * np.abs(ref) + 5e-5).all(), (i, float((err - u * np.abs(ref)).max()))

@@ -135,11 +135,9 @@ typedef struct b2a_paged_desc {
      * into an f16 scratch and the prefill kernel stages K/V tiles by TMA; without it (0) every prefill CTA
      * de-quantises its own tiles.  A bound that is too small makes the step report B2A_DEV_BAD_LEN. */
     int32_t prefill_kv_tokens;
-    /* Optional, decode rows only.  Non-zero: the caller promises that the kernel directly before this call on the stream
-     * writes no cache row other than the rows of this step's new tokens (true when that kernel is this step's
-     * b2a_paged_kv_store, or a kernel that does not touch the cache at all).  The decode kernel, which is launched
-     * while that kernel still drains, then starts copying cache blocks that hold no new token before it waits for
-     * it.  0 (the default): every cache read comes after the wait. */
+    /* Without effect, kept for callers that set it: the promise that the kernel directly before this call on the stream writes
+     * no cache row other than the rows of this step's new tokens.  The decode kernels, which are launched while that
+     * kernel still drains, need no promise: they ask for their first blocks ahead of time but read the cache after it. */
     int32_t cache_rows_settled;
 } b2a_paged_desc;
 

@@ -59,7 +59,6 @@ struct DecodeParams {
     float scale_log2;  // softmax scale * log2(e)
     int32_t* status;
     int beside_predecessor;      // see paged_decode_launch: no wait for the kernel before this one
-    int cache_rows_settled;      // b2a_paged_desc: the kernel before this one writes no cache row but the new tokens'
     cudaEvent_t predecessor_done;  // host side only: completes with that kernel
     // score output (kMode 3): the scaled scores of every cached key, base-2 units, [block of the table][Hkv][16 keys][G]
     float* raw_scores;
@@ -160,9 +159,8 @@ enum ChunkState {
 // sit on the SMs while that kernel drains.  The walk uses that time for the first two of its three dependent loads:
 // the step's tables and this warp's block ids are read BEFORE the wait (the tables of a step exist before its first
 // kernel is launched; nothing on this path writes them), through L2 so that no line cached by an earlier step is
-// met; so are the first cache blocks of a CTA that does not hold its sequence's last block.  Everything an earlier
-// kernel of the step produces - the query rows, the cache rows of the new tokens, the workspace, the status word, the
-// exchange's counters - is touched only after the wait.
+// met.  Everything an earlier kernel of the step produces - the query rows, the cache rows of the new tokens, the workspace, the
+// status word, the exchange's counters - is read and written only after the wait.
 //
 // With kScores the scaled scores also go to memory (raw_scores), for the kernel that turns them into probabilities.
 template <typename T, int NT, bool kRowIsSeq, int kWarps, bool kScores = false>
@@ -226,15 +224,16 @@ __device__ __forceinline__ ChunkState decode_chunk(const DecodeParams& p, uint8_
         }
     };
 
-    // With the caller's promise that the kernel before this one writes no cache row but the new tokens' (each in
-    // its sequence's last block), a CTA whose blocks end before that block reads nothing that kernel changes, so its
-    // first copy stages also go out before the wait.
-    const bool early = wait_for_predecessor && p.cache_rows_settled && state == kChunkWorked && my_hi < nblk;
-    if (early) {
+    // A warp's first blocks are asked into L2 meanwhile.  Not into shared memory: a block that this sequence holds as cached may
+    // be one that another sequence's new token goes into (prefixes shared within a step), and only what is read behind
+    // the wait is sure to show that row.  Cold pools, 8 KV heads, us a step with the store, without the prefetch and with it: 2
+    // sequences of 300..900 tokens 10.1 both, 4 of 8000 22.1 and 20.8, 64 of 512..4096 70.4 and 68.1.  (Copies into shared
+    // memory here, of blocks before a CTA's sequence's last: 10.0, 21.9 and 70.2.)
+    if (wait_for_predecessor) {
 #pragma unroll
         for (int s = 0; s < kStages - 1; ++s) {
-            if (s < n_w) issue(s);
-            cp_async_commit();
+            const int phys = __shfl_sync(0xffffffffu, my_phys, s);
+            if (s < n_w && phys >= 0 && lane < 2) prefetch_l2((lane == 0 ? p.k_cache : p.v_cache) + phys * block_stride + hk * head_stride, kChunk);
         }
     }
 
@@ -265,14 +264,11 @@ __device__ __forceinline__ ChunkState decode_chunk(const DecodeParams& p, uint8_
 
     if (bad_block) report(p.status, B2A_DEV_BAD_BLOCK);
 
-    // ---- pipeline prologue (unless it went out before the wait): the first stages are on their way before the
-    // query fragments are put together
-    if (!early) {
+    // ---- pipeline prologue: the first stages are on their way before the query fragments are put together
 #pragma unroll
-        for (int s = 0; s < kStages - 1; ++s) {
-            if (s < n_w) issue(s);
-            cp_async_commit();
-        }
+    for (int s = 0; s < kStages - 1; ++s) {
+        if (s < n_w) issue(s);
+        cp_async_commit();
     }
 
     // ---- query fragments (B operand of QK^T) and per-head sums of Q
@@ -1084,7 +1080,6 @@ int paged_decode_launch(const b2a_paged_desc& d, const DecodePlan& plan, const v
     p.blocks_per_cta = plan.blocks_per_cta;
     p.max_splits = plan.max_splits;
     p.sliding_window = d.sliding_window;
-    p.cache_rows_settled = d.cache_rows_settled;
     p.scale_log2 = d.scale * kLog2e;
     p.status = status;
     const bool two = p.G > 8;

@@ -280,8 +280,7 @@ def paged_attention(query: torch.Tensor, cache: PagedKvCache, past_lens, subsequ
 
     ``prefill_row_blocks`` and ``prefill_kv_tokens`` are the optional scheduler hints of ``b2a_paged_desc``
     (``KvBlockManager`` reports both); the second lets a mixed step de-quantise its prefill contexts once.
-    ``cache_rows_settled``: the caller's promise that the kernel directly before this call on the stream writes no
-    cache row other than this step's new tokens (see ``b2a_paged_desc``)."""
+    ``cache_rows_settled`` has no effect any more (see ``b2a_paged_desc``)."""
     _require_cuda(query, cache.k, cache.v, past_lens, subsequence_begins, block_indices, block_indices_begins, out)
     if not query.is_contiguous() or query.shape[1] != hq * cache.d:
         raise ValueError("query must be dense [tokens, Hq*D]")
@@ -483,7 +482,7 @@ class PagedAttentionOp:
             raise ValueError("query must be dense [tokens, Hq*D]")
         lib, scale_value = _lib.load(), self.scale if sc is None else float(sc)
         d = _paged_desc(key.dtype, cache, self.hq, num_seqs, key_tokens, self.max_context_len, max_q_len, scale_value,
-                        self.sliding_window, rb, kvt, True)  # (settled: the kernel before the attention is this step's store)
+                        self.sliding_window, rb, kvt)
         caches = (k_cache.data_ptr(), v_cache.data_ptr())
         tables = (_i32(past_lens).data_ptr(), _i32(subsequence_begins).data_ptr(), _i32(block_indices).data_ptr(),
                   _i32(block_indices_begins).data_ptr())
@@ -494,7 +493,7 @@ class PagedAttentionOp:
             done = paged_attention_scores(query, cache, past_lens, subsequence_begins, block_indices, block_indices_begins,
                                           self.hq, self.max_context_len, scale_value,
                                           self.sliding_window, out=outputs[0], scores=outputs[1], stream=stream,
-                                          status=status, cache_rows_settled=True)
+                                          status=status)
             if done is not None:
                 return done[2]
         d.q_dtype, d.num_tokens = _dtype_code(query.dtype), num_tokens

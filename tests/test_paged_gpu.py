@@ -226,9 +226,8 @@ def test_mixed_step_through_the_operator(b2a, dtype):
 
 
 def test_decode_steps_through_the_operator_see_their_new_tokens(b2a):
-    # Pure decode steps through the operator: its attention call promises that only the new tokens' rows changed
-    # (cache_rows_settled), so the decode kernel copies earlier blocks while the store kernel before it still runs.
-    # Three consecutive steps in one captured graph (store, attention, store, attention, ...: every attention kernel
+    # Pure decode steps through the operator: the decode kernel reads its block ids, and asks for its first blocks, while the
+    # store kernel before it still runs.  Three consecutive steps in one captured graph (store, attention, store, attention, ...: every attention kernel
     # is launched while a store kernel drains); every step's new row - first row of a fresh block, last row of a
     # block, somewhere inside - must be seen, and nothing else may differ from the oracle.
     hq, hkv, d, bs = 32, 4, 128, 16

@@ -33,7 +33,7 @@ def shared_step(writer_tokens, pairs, reader_ctx, seed):
     return [np.asarray(x, np.int32) for x in t], nb
 
 
-@pytest.mark.parametrize("kv", ["f16", "bf16"])
+@pytest.mark.parametrize("kv", ["f16", "bf16", "u8"])
 @pytest.mark.parametrize("writer_tokens,pairs", [(1, 3), (64, 2), (1, 40)])
 @pytest.mark.parametrize("reader_ctx", [33, 600, 4000])
 def test_new_rows_of_another_sequence_are_seen(kv, writer_tokens, pairs, reader_ctx):

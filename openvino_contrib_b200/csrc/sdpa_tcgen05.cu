@@ -42,8 +42,8 @@
 // Three prompts of 400 to 1100 tokens behind caches of up to 3000: 92.2 -> 86.6 us a step.  (Issued by one warp on a shared S: 785.
 // P's first half sent ahead of the second, P kept in registers until PV(j-1) has read the columns, the maximum of half a
 // row while the other half is loaded, two PV issuers: no gain, the exponentials of the two tiles are what counts now.)
-// The calls that hold P in several pieces (kSplitP) have no columns for that: there S_X has a place per tile, the pieces of P
-// lie over it, and one lane of warp 9 issues PV_A(j), QK_A(j+1), PV_B(j), QK_B(j+1), PV in two halves as those of P arrive.
+// The calls that hold P in several pieces (kSplitP) have no columns for that, and with in-kernel de-quantisation it does not pay:
+// there S_X has a place per tile, P lies over it, and one lane of warp 9 issues PV_A(j), QK_A(j+1), PV_B(j), QK_B(j+1), PV in two halves as those of P arrive.
 //   warps 12-15 mode 1 only: the de-quantising K/V producers.
 // The two tiles are consecutive entries of the list (row block, query head of the group), query heads fastest, so
 // with an even group size both tiles cover the same rows of two heads that share K/V, and the causal structure of
@@ -523,7 +523,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     static_assert(!kSplitP || kMode == 0, "the paged modes hold P in 16 bits");
     constexpr bool kSingle = kSplitP && kDim == kHeadDim;  // an item is one tile: the pieces of P need tile B's columns
     static_assert(!(kSingle && kKeySplit), "no columns for the other half of the keys");
-    constexpr bool kSharedS = !kSplitP;  // one place for S, which the tiles take in turn; P has columns of its own
+    // One place for S, which the tiles take in turn; P has columns of its own.  (Not with in-kernel de-quantisation, which is bound
+    // by its producers: a step of three prompts behind caches takes 209 us in f16 and 216 in bf16 that way, 202 and 208 with a
+    // place per tile - two more warps that issue and wait beside them.)
+    constexpr bool kSharedS = !kSplitP && kMode != 1;
     constexpr int kTile = 128 * kDim * 2;  // bytes of a [128 x kDim] 16-bit tile: kDim / 64 panels
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -741,9 +744,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     };
 
     // Registers follow the work: the service warpgroup keeps 88 (56) per thread, the softmax groups take what is left
-    // (2*128*208 + 128*88 = 384*168; in-kernel de-quantisation: 2*128*168 + 128*56 + 128*112 <= 512*128).  A sum above what the
+    // (2*128*208 + 128*88 = 384*168; a place of S per tile: 224 and 56; in-kernel de-quantisation: 2*128*168 + 128*56 + 128*112 <= 512*128).  A sum above what the
     // launch has would wait forever.
-    constexpr int kServiceRegs = kSharedS && !kDequant ? 88 : 56, kSoftmaxRegs = kDequant ? 168 : kSharedS ? 208 : 224, kDequantRegs = kDequant ? 112 : 0;
+    constexpr int kServiceRegs = kSharedS ? 88 : 56, kSoftmaxRegs = kDequant ? 168 : kSharedS ? 208 : 224, kDequantRegs = kDequant ? 112 : 0;
     static_assert(256 * kSoftmaxRegs + 128 * kServiceRegs + 128 * kDequantRegs <= (kDequant ? 512 * 128 : 384 * 168), "register split");
     if (warp >= 8 && warp < 12) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kServiceRegs));
     if (warp >= 12) {

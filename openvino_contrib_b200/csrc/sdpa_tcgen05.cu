@@ -42,7 +42,7 @@
 // Three prompts of 400 to 1100 tokens behind caches of up to 3000: 92.2 -> 86.6 us a step.  (Issued by one warp on a shared S: 785.
 // P's first half sent ahead of the second, P kept in registers until PV(j-1) has read the columns, the maximum of half a
 // row while the other half is loaded, two PV issuers: no gain, the exponentials of the two tiles are what counts now.)
-// The calls that hold P in several pieces (kSplitP) have no columns for that, and with in-kernel de-quantisation it does not pay:
+// The calls that hold P in several pieces (kSplitP) have no columns for that, and with in-kernel de-quantisation or items of one key step (kOwnS) it does not pay:
 // there S_X has a place per tile, P lies over it, and one lane of warp 9 issues PV_A(j), QK_A(j+1), PV_B(j), QK_B(j+1), PV in two halves as those of P arrive.
 //   warps 12-15 mode 1 only: the de-quantising K/V producers.
 // The two tiles are consecutive entries of the list (row block, query head of the group), query heads fastest, so
@@ -514,7 +514,8 @@ __global__ void __launch_bounds__(128) paged_gather_kernel(const PagedTables t, 
 //   the tensor-memory lanes of its number modulo four).  One item per CTA; the launcher's rule compares the two chains.
 //   Causal prompts, 32/8 heads, D = 128, graph replay: 512 tokens 12.9 -> 9.4 us, 777 tokens 17.6 -> 15.7 us; 8 heads x 2048
 //   tokens, D = 64, no mask: 36.9 -> 22.2 us.
-template <bool kBf16, int kMode, int kMask = 0, int kDim = kHeadDim, bool kSplitP = false, bool kKeySplit = false>
+// kOwnS (dense, no mask, at most 128 keys): a place of S per tile although P is not in pieces.
+template <bool kBf16, int kMode, int kMask = 0, int kDim = kHeadDim, bool kSplitP = false, bool kKeySplit = false, bool kOwnS = false>
 __global__ void __launch_bounds__(kMode == 1 ? kThreadsPaged : kThreadsDense, 1)
 attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                const __grid_constant__ CUtensorMap tmV, const TcParams p, const __grid_constant__ TcPeers peers) {
@@ -526,7 +527,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     // One place for S, which the tiles take in turn; P has columns of its own.  (Not with in-kernel de-quantisation, which is bound
     // by its producers: a step of three prompts behind caches takes 209 us in f16 and 216 in bf16 that way, 202 and 208 with a
     // place per tile - two more warps that issue and wait beside them.)
-    constexpr bool kSharedS = !kSplitP && kMode != 1;
+    constexpr bool kSharedS = !kSplitP && kMode != 1 && !kOwnS;
     constexpr int kTile = 128 * kDim * 2;  // bytes of a [128 x kDim] 16-bit tile: kDim / 64 panels
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -1700,12 +1701,12 @@ bool make_map(CUtensorMap* map, const void* ptr, bool bf16, int B, int H, int S,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int kMask, int kDim, bool kSplitP, bool kKeySplit = false>
+template <int kMask, int kDim, bool kSplitP, bool kKeySplit = false, bool kOwnS = false>
 int launch_dense(bool bf16, dim3 grid, cudaStream_t stream, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                  const TcParams& p, const TcPeers& peers) {
     constexpr int smem = smem_bytes(128 * kDim * 2);
     static OncePerDevice configured[2];
-    auto kern = bf16 ? attn_tc_kernel<true, 0, kMask, kDim, kSplitP, kKeySplit> : attn_tc_kernel<false, 0, kMask, kDim, kSplitP, kKeySplit>;
+    auto kern = bf16 ? attn_tc_kernel<true, 0, kMask, kDim, kSplitP, kKeySplit, kOwnS> : attn_tc_kernel<false, 0, kMask, kDim, kSplitP, kKeySplit, kOwnS>;
     const int rc = configure_once(kern, configured[bf16], smem);
     if (rc != B2A_OK) return rc;
     return launch_overlapped(kern, grid, dim3(kThreadsDense), smem, stream, mq, mk, mv, p, peers) == cudaSuccess ? B2A_OK : B2A_ERR_CUDA;
@@ -1859,6 +1860,11 @@ int sdpa_tc_launch(const b2a_sdpa_desc& d, const int64_t (&qs)[4], const int64_t
     if (mask_kind == B2A_MASK_BOOL) return launch_dense<1, kHeadDim, false>(bf16, grid, stream, mq, mk, mv, p, peers);
     if (mask_kind == B2A_MASK_ADD) return launch_dense<2, kHeadDim, false>(bf16, grid, stream, mq, mk, mv, p, peers);
     if (key_split) return launch_dense<0, kHeadDim, false, true>(bf16, tile_grid, stream, mq, mk, mv, p, peers);
+    // One key step an item: there is no next step whose QK^T could run beside the softmax, and PV starts on the first half of P where
+    // S has a place per tile (us, shared and per tile: 4 x 200 heads x 100 tokens 23.6 and 21.2, 32 heads x 128 6.15 and
+    // 5.8, 8 x 32/8 heads x 128 without the causal mask 8.2 and 7.6).  From two steps on it is even (4 x 32/8 heads x 256: 9.8
+    // both) or the other way round (16 x 32/8 heads x 129: 21.7 and 22.8).
+    if (n == 1) return launch_dense<0, kHeadDim, false, false, true>(bf16, grid, stream, mq, mk, mv, p, peers);
     return launch_dense<0, kHeadDim, false>(bf16, grid, stream, mq, mk, mv, p, peers);
 }
 

@@ -747,8 +747,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     // Registers follow the work: the service warpgroup keeps 72 (56) per thread, the softmax groups take what is left
     // (2*128*216 + 128*72 = 384*168; a place of S per tile: 224 and 56; in-kernel de-quantisation: 2*128*168 + 128*56 + 128*112
     // <= 512*128).  A sum above what the launch has would wait forever.  (88 and 208: the masked and the bf16 gathered forms spill
-    // 8 bytes more, three steps of 384 keys without a mask take 33.6 us instead of 32.8.)
-    constexpr int kServiceRegs = kSharedS ? 72 : 56, kSoftmaxRegs = kDequant ? 168 : kSharedS ? 216 : 224, kDequantRegs = kDequant ? 112 : 0;
+    // 8 bytes more, three steps of 384 keys without a mask take 33.6 us instead of 32.8.)  With P in three pieces the issuing lane
+    // wants 72 as well (us, 56 and 72 registers: 8 x 16 heads x 512 tokens, D = 64, bf16, causal 28.7 and 27.3, unmasked 33.1
+    // and 31.5; two pieces 21.9 and 23.2, 23.6 and 24.9), but for the forms that have the most to keep in the softmax warps.
+    constexpr bool kWideService = kSharedS || (kSplitP && kBf16 && kMask != 5 && !kKeySplit);
+    constexpr int kServiceRegs = kWideService ? 72 : 56, kSoftmaxRegs = kDequant ? 168 : kWideService ? 216 : 224, kDequantRegs = kDequant ? 112 : 0;
     static_assert(256 * kSoftmaxRegs + 128 * kServiceRegs + 128 * kDequantRegs <= (kDequant ? 512 * 128 : 384 * 168), "register split");
     if (warp >= 8 && warp < 12) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kServiceRegs));
     if (warp >= 12) {
@@ -1474,10 +1477,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             if (ok) {
                 tc_fence_after();
                 const float inv = l > 0.f ? 1.f / l : 0.f;
-                // Where the tile goes: with P in pieces worked out again here rather than kept in registers across the key loop.
-                // (Otherwise that is the dearer way: 192 bytes of spill loads instead of 24 in the unmasked form of head size 128,
-                // and 300 cycles an item; 8 x 32 heads x 300 tokens 27.3 us instead of 25.1, 2048 tokens 33.6 instead of 32.4.)
-                if constexpr (kSplitP && !kKeySplit) {
+                // Where the tile goes is kept across the key loop.  (Worked out again here it is 192 bytes of spill loads instead of
+                // 24 in the unmasked form of head size 128, and 300 cycles an item: 8 x 32 heads x 300 tokens 27.3 us instead of 25.1,
+                // 2048 tokens 33.6 instead of 32.4.)  Only three pieces of P beside a mask read element by element leave no
+                // room for it (4 x 16 heads x 509 tokens, a boolean mask row per query: 99 us kept, 90 this way).
+                if constexpr (kSplitP && kBf16 && kMask == 5) {
                     int k_again = k;
                     asm volatile("" : "+r"(k_again));
                     get_item(k_again, item);

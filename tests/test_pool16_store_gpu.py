@@ -15,8 +15,9 @@ def tables(past, new, block_size, seed):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("hkv,d,block_size", [(1, 128, 16), (2, 64, 16), (3, 128, 16), (8, 128, 32), (2, 8, 8), (16, 8, 5),
-                                              (1, 64, 16), (4, 12, 16)])  # (the last two: the general kernel)
+@pytest.mark.parametrize("hkv,d,block_size", [(1, 128, 16), (2, 64, 16), (3, 128, 16), (8, 128, 32), (16, 8, 5), (16, 16, 8),
+                                              # no whole warps a token: the general kernel
+                                              (2, 8, 8), (1, 64, 16), (4, 12, 16)])
 @pytest.mark.parametrize("new", [[1] * 5, [1, 7, 1, 40], [33]])
 def test_rows_land_in_their_blocks(dtype, hkv, d, block_size, new):
     import openvino_contrib_b200 as b2a
@@ -36,6 +37,48 @@ def test_rows_land_in_their_blocks(dtype, hkv, d, block_size, new):
             for i in range(new[s]):
                 pos = past[s] + i
                 want[t[2][t[3][s] + pos // block_size], :, pos % block_size] = bits[t[1][s] + i]
+        np.testing.assert_array_equal(pool.cpu().numpy().view(np.uint16).reshape(want.shape), want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("hkv,d", [(2, 64), (16, 8), (2, 8)])  # (the last: the general kernel)
+@pytest.mark.parametrize("what", ["block id too large", "block id negative", "no block for the position", "negative past",
+                                  "tokens that no sequence has"])
+def test_bad_tables_are_reported_and_write_nothing(dtype, hkv, d, what):
+    import openvino_contrib_b200 as b2a
+    from openvino_contrib_b200._lib import DEV_BAD_BLOCK, DEV_BAD_LEN
+    past, new = [20, 3, 40], [1, 30, 1]
+    t = tables(past, new, 16, 4)
+    cache = b2a.PagedKvCache.allocate(int(t[2].max()) + 4, hkv, d, 16, dtype, poison=0x5A)
+    tokens, lost, status_bit = sum(new), set(), 0
+    if what.startswith("block id"):
+        t[2][t[3][1]] = cache.num_blocks if "large" in what else -1  # the second sequence's first block: its positions 3 to 15
+        lost, status_bit = set(range(1, 14)), DEV_BAD_BLOCK
+    elif what == "no block for the position":
+        t[0][1] = 10  # positions 10 to 39, and two blocks instead of three
+        t[3][2:] -= 1
+        t[2] = np.delete(t[2], t[3][2])
+        lost, status_bit = {1 + i for i in range(30) if 10 + i >= 32}, DEV_BAD_LEN
+    elif what == "negative past":
+        t[0][2] = -5
+        lost, status_bit = {31}, DEV_BAD_LEN
+    else:
+        tokens += 9  # rows behind the last sequence's
+        lost = set(range(32, 41))
+    rows = [torch.randn(tokens, hkv * d, generator=torch.Generator().manual_seed(i)).to(dtype) for i in range(2)]
+    before = [c.cpu().numpy().copy() for c in (cache.k, cache.v)]
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    b2a.paged_kv_store(rows[0].cuda(), rows[1].cuda(), cache, *[torch.from_numpy(x).cuda() for x in t], status=status)
+    assert int(status.item()) == status_bit
+    for pool, was, r in zip((cache.k, cache.v), before, rows):
+        want = was.view(np.uint16).reshape(-1, hkv, 16, d)
+        bits = r.view(torch.int16).numpy().view(np.uint16).reshape(-1, hkv, d)
+        for s in range(len(new)):
+            for i in range(new[s]):
+                if t[1][s] + i in lost:
+                    continue
+                pos = t[0][s] + i
+                want[t[2][t[3][s] + pos // 16], :, pos % 16] = bits[t[1][s] + i]
         np.testing.assert_array_equal(pool.cpu().numpy().view(np.uint16).reshape(want.shape), want)
 
 

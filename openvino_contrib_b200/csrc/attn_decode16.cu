@@ -30,6 +30,7 @@ namespace {
 constexpr int kWarps = 4;
 constexpr int kTileKeys = 16;
 constexpr int kMaxCluster = 8;          // the portable limit
+constexpr unsigned kSeats = 148 * 2;    // CTAs that the GPU holds at once
 constexpr float kNegBig = -1.0e30f;     // finite "minus infinity": start of the running maximum, floor of finite masks
 
 struct Dec16Params {
@@ -267,19 +268,21 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attn_decode16_kernel(const Dec
     };
     if constexpr (kPaged) {
         // The step's tables exist before its kernels are launched, so the block ids are read while the kernel in front, as a rule
-        // the step's store, drains, and the first tiles are asked into L2.  Not into shared memory: a block that this sequence
+        // the step's store, drains, and the first wave's CTAs ask their first tiles into L2.  Not into shared memory: a block that this sequence
         // holds as cached may be one that another sequence's new token goes into (prefixes shared within a step), and only
         // what is read behind the wait is sure to show that row.  Cold pools, f16, 8 KV heads, us a step with the store, without
         // the prefetch and with it: 2 sequences of 300..900 tokens 7.9 and 7.5, 8 of 2000 21.4 and 20.3, 32 of 256..4096 53.7
         // and 51.7.  (Copies into shared memory here, of the tiles before a sequence's last: 7.2, 21.1 and 53.1.)
         load_window(0);
+        if (blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z) < kSeats) {
 #pragma unroll
-        for (int s = 0; s < kStages - 1; ++s) {
-            const int phys = __shfl_sync(0xffffffffu, window_ids, s);
-            if (s < n_w && phys >= 0 && lane < 2) {
-                const int key0 = (my_lo + warp + kWarps * s) * kTileKeys;
-                const int64_t at = static_cast<int64_t>(phys) * p.k_b + key0 % p.t.block_size * kRowBytes;
-                prefetch_l2((lane == 0 ? kb : vb) + at, kHalfTile);
+            for (int s = 0; s < kStages - 1; ++s) {
+                const int phys = __shfl_sync(0xffffffffu, window_ids, s);
+                if (s < n_w && phys >= 0 && lane < 2) {
+                    const int key0 = (my_lo + warp + kWarps * s) * kTileKeys;
+                    const int64_t at = static_cast<int64_t>(phys) * p.k_b + key0 % p.t.block_size * kRowBytes;
+                    prefetch_l2((lane == 0 ? kb : vb) + at, kHalfTile);
+                }
             }
         }
         grid_dependency_wait();

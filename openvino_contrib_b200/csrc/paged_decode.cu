@@ -37,6 +37,7 @@ constexpr int kD = 128;
 constexpr int kBS = 16;
 constexpr int kChunk = kBS * (kD + 4);   // 2112 bytes: 2048 codes, 16 f16 scales, 16 f16 zero-points
 constexpr int kStage = 2 * kChunk;       // K chunk then V chunk
+constexpr unsigned kSeats = 148 * 16;    // warps that the GPU holds at once
 constexpr int kStages = 3;                // copy stages per warp
 // Warps per CTA: 4 when the grid fills every SM four CTAs deep (16 warps per SM hide one another's latencies).  A grid
 // of at most two CTAs per SM - a head shard of a step - would leave each warp alone with its chain of dependent
@@ -224,12 +225,13 @@ __device__ __forceinline__ ChunkState decode_chunk(const DecodeParams& p, uint8_
         }
     };
 
-    // A warp's first blocks are asked into L2 meanwhile.  Not into shared memory: a block that this sequence holds as cached may
+    // A warp's first blocks are asked into L2 meanwhile, in the CTAs of the first wave (later ones find nothing to wait for, and
+    // asking twice costs: 16 sequences of 32768 tokens 194.9 us a step with it in all CTAs, 192.0 so).  Not into shared memory: a block that this sequence holds as cached may
     // be one that another sequence's new token goes into (prefixes shared within a step), and only what is read behind
     // the wait is sure to show that row.  Cold pools, 8 KV heads, us a step with the store, without the prefetch and with it: 2
     // sequences of 300..900 tokens 10.1 both, 4 of 8000 22.1 and 20.8, 64 of 512..4096 70.4 and 68.1.  (Copies into shared
     // memory here, of blocks before a CTA's sequence's last: 10.0, 21.9 and 70.2.)
-    if (wait_for_predecessor) {
+    if (wait_for_predecessor && blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z) < kSeats / kWarps) {
 #pragma unroll
         for (int s = 0; s < kStages - 1; ++s) {
             const int phys = __shfl_sync(0xffffffffu, my_phys, s);

@@ -68,14 +68,15 @@ HostSdpaRunner::HostSdpaRunner(int dtype, int B, int Hq, int Hkv, int Sq, int Sk
         cuda_ok(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "cudaEventCreate");
     uploaded_.resize(z(pieces()));
     computed_.resize(z(pieces()));
-    for (auto& e : uploaded_) cuda_ok(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
-    for (auto& e : computed_) cuda_ok(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+    kv_uploaded_.resize(z(pieces()));
+    for (auto* events : {&kv_uploaded_, &uploaded_, &computed_})
+        for (auto& e : *events) cuda_ok(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
 }
 
 HostSdpaRunner::~HostSdpaRunner() {
     cudaDeviceSynchronize();
-    for (auto e : uploaded_) cudaEventDestroy(e);
-    for (auto e : computed_) cudaEventDestroy(e);
+    for (const auto* events : {&kv_uploaded_, &uploaded_, &computed_})
+        for (auto e : *events) cudaEventDestroy(e);
     if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
     for (cudaEvent_t e : {begin_, end_, caller_in_, caller_out_})
         if (e) cudaEventDestroy(e);
@@ -144,22 +145,32 @@ void HostSdpaRunner::Enqueue(const void* q, const void* k, const void* v, void* 
     const size_t kv_piece = static_cast<size_t>(hpp_) * Skv_ * D_ * esize_;
     auto at = [](const void* p, size_t off) { return static_cast<const char*>(p) + off; };
     auto at_m = [](void* p, size_t off) { return static_cast<char*>(p) + off; };
-    for (int i = 0; i < pieces(); ++i) {
-        const size_t qo = static_cast<size_t>(i) * q_piece, kvo = static_cast<size_t>(i) * kv_piece;
-        // ParameterOp's part: host -> device, K and V first (the kernel's first loads), then the queries
+    auto upload = [&](int i) {  // ParameterOp's part: host -> device, K and V first (the kernel's first loads), then the queries
+        const size_t n = static_cast<size_t>(i), qo = n * q_piece, kvo = n * kv_piece;
         cuda_ok(cudaMemcpyAsync(at_m(dk_, kvo), at(k, kvo), kv_piece, cudaMemcpyHostToDevice, up_), "cudaMemcpyAsync");
         cuda_ok(cudaMemcpyAsync(at_m(dv_, kvo), at(v, kvo), kv_piece, cudaMemcpyHostToDevice, up_), "cudaMemcpyAsync");
+        cuda_ok(cudaEventRecord(kv_uploaded_[n], up_), "cudaEventRecord");
         cuda_ok(cudaMemcpyAsync(at_m(dq_, qo), at(q, qo), q_piece, cudaMemcpyHostToDevice, up_), "cudaMemcpyAsync");
-        cuda_ok(cudaEventRecord(uploaded_[static_cast<size_t>(i)], up_), "cudaEventRecord");
-        cuda_ok(cudaStreamWaitEvent(main, uploaded_[static_cast<size_t>(i)], 0), "cudaStreamWaitEvent");
+        cuda_ok(cudaEventRecord(uploaded_[n], up_), "cudaEventRecord");
+    };
+    upload(0);
+    for (int i = 0; i < pieces(); ++i) {
+        const size_t n = static_cast<size_t>(i), qo = n * q_piece, kvo = n * kv_piece;
+        const bool more = i + 1 < pieces();
+        if (more) upload(i + 1);
+        cuda_ok(cudaStreamWaitEvent(main, uploaded_[n], 0), "cudaStreamWaitEvent");
         const std::vector<CUDA::DevicePointer<const void*>> in{CUDA::DevicePointer<const void*>{at(dq_, qo)},
                                                                CUDA::DevicePointer<const void*>{at(dk_, kvo)},
                                                                CUDA::DevicePointer<const void*>{at(dv_, kvo)}};
         const std::vector<CUDA::DevicePointer<void*>> outs{CUDA::DevicePointer<void*>{at_m(do_, qo)}};
         op_->Execute(request_, {in.data(), in.size()}, {outs.data(), outs.size()}, workbuffers_);
-        cuda_ok(cudaEventRecord(computed_[static_cast<size_t>(i)], main), "cudaEventRecord");
-        // ResultOp's part: device -> host
-        cuda_ok(cudaStreamWaitEvent(down_, computed_[static_cast<size_t>(i)], 0), "cudaStreamWaitEvent");
+        cuda_ok(cudaEventRecord(computed_[n], main), "cudaEventRecord");
+        // ResultOp's part: device -> host, beside the upload of the next piece's queries.  Started as soon as its piece is computed it
+        // runs beside the short uploads of K and V as well, and both directions lose: whether it did depended on the
+        // kernel's time, so a faster kernel made slower steps (bf16, 4 x 4096 tokens, 32/8 heads: 4.50 ms with a kernel of 61 us
+        // a piece, 4.68 with one of 56, 4.36 this way; 2048 tokens 2.62, 2.64, 2.28; 8192 tokens 4.93, 4.83, 4.78).
+        cuda_ok(cudaStreamWaitEvent(down_, computed_[n], 0), "cudaStreamWaitEvent");
+        if (more) cuda_ok(cudaStreamWaitEvent(down_, kv_uploaded_[n + 1], 0), "cudaStreamWaitEvent");
         cuda_ok(cudaMemcpyAsync(at_m(out, qo), at(do_, qo), q_piece, cudaMemcpyDeviceToHost, down_), "cudaMemcpyAsync");
     }
     cuda_ok(cudaEventRecord(end_, down_), "cudaEventRecord");

@@ -30,7 +30,7 @@ namespace nvidia_gpu {
 class HostSdpaRunner {
 public:
     // dtype: b2a_dtype of q, k, v, o (B2A_F32 / B2A_F16 / B2A_BF16).  Allocates the device tensors, three streams
-    // and two events per piece; throws through ov::throw_ov_exception.
+    // and three events per piece; throws through ov::throw_ov_exception.
     // kv_heads_per_piece: KV heads (with their query heads) per piece; must divide Hkv; 0 = the default (pieces of
     // at least 8 MB of upload: copies much smaller than that do not reach the bus's bandwidth).
     HostSdpaRunner(int dtype, int B, int Hq, int Hkv, int Sq, int Skv, int D, bool causal, int device = 0,
@@ -66,7 +66,7 @@ private:
     const void* last_[4] = {nullptr, nullptr, nullptr, nullptr};  // host tensors of the previous Run
     cudaGraphExec_t graph_exec_ = nullptr;                        // the step over last_, once captured
     bool capture_failed_ = false;
-    std::vector<cudaEvent_t> uploaded_, computed_;
+    std::vector<cudaEvent_t> kv_uploaded_, uploaded_, computed_;
 };
 
 }  // namespace nvidia_gpu

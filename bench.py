@@ -36,8 +36,8 @@ PREFILL = dict(B=4, Hq=32, Hkv=8, S=4096, D=128)
 # They are constants of this file, not measurements of the run that prints them (a profiler cannot run inside a
 # timed benchmark); the line says so next to each figure.
 NCU_TRAFFIC = {
-    "prefill": 436.1e6,   # attn_tc_kernel<bf16, dense> on the full prefill workload
-    "cfg3": 627.5e6,      # paged_decode_kernel<f16, 1> on the 64-sequence decode
+    "prefill": 418.9e6,   # attn_tc_kernel<bf16, dense> on the full prefill workload
+    "cfg3": 627.4e6,      # paged_decode_kernel<f16, 1> on the 64-sequence decode
 }
 TRAFFIC_SOURCE = "profiler capture of this kernel on this workload (a constant, not measured in this run)"
 L2_BYTES = 126 * (1 << 20)

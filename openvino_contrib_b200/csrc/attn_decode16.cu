@@ -548,8 +548,10 @@ int launch_any(int dtype, const Dec16Params& p, int D, bool paged, int keys, int
     // CTAs per (sequence, KV head), as long as every warp keeps two tiles or more.  Dense tensors: equal lengths, so at
     // least three quarters of one wave of two CTAs per SM and no second wave (8 x 3003 keys x 8 KV heads, with the
     // additive mask: two CTAs 32.3 us, four 20.9, eight 25.6).  A pool: lengths differ, and shorter pieces even them out
-    // (32 sequences of 256..4096 tokens x 8 KV heads, with the store kernel: one CTA 59.8 us, two 57.2, four 54.8,
-    // eight 72.4 - then the start and the merge of a CTA outweigh its tiles), so about three waves.
+    // (32 sequences of 256..4096 tokens x 8 KV heads, bf16, cold, with the store kernel: one CTA 61.5 us, two 57.5, four 52.7,
+    // eight 71.5 - then the start and the merge of a CTA outweigh its tiles), so about three waves.  The line is the ragged
+    // step's: equal lengths would have fewer (8 sequences of 2000 tokens: four CTAs 14.9 us, the rule's eight 20.7), and
+    // so would contexts far below the capacity that the rule goes by (8 of 64 tokens, built for 8192: two 6.3, eight 12.0).
     const int sms = device_sm_count();
     if (sms <= 0) return B2A_ERR_CUDA;
     const int tiles = std::max(1, (keys + kTileKeys - 1) / kTileKeys);

@@ -37,13 +37,15 @@
 // Why S is shared and QK and PV have issuers of their own: with S and P of a tile in one place a step is the chain softmax ->
 // PV -> QK -> softmax (1750 + 256 + 512 cycles and three trips over barriers), and one issuer, which stands still while the
 // tensor core's short queue is full and pays about 130 cycles for every barrier it looks at, leaves the tensor core idle
-// for a third of a step.  Causal prefill of 4 x 4096 tokens, 32/8 heads, bf16: 785 thousand cycles a launch before, 692 now;
-// in time 542 us before and 516 now in a loop of passes, because the launch runs into the power limit (1.43 GHz there).
-// Three prompts of 400 to 1100 tokens behind caches of up to 3000: 92.2 -> 86.6 us a step.  (Issued by one warp on a shared S: 785.
-// P's first half sent ahead of the second, P kept in registers until PV(j-1) has read the columns, the maximum of half a
-// row while the other half is loaded, two PV issuers: no gain, the exponentials of the two tiles are what counts now.)
-// The calls that hold P in several pieces (kSplitP) have no columns for that, and with in-kernel de-quantisation or items of one key step (kOwnS) it does not pay:
-// there S_X has a place per tile, P lies over it, and one lane of warp 9 issues PV_A(j), QK_A(j+1), PV_B(j), QK_B(j+1), PV in two halves as those of P arrive.
+// for a third of a step.  Causal prefill of 4 x 4096 tokens, 32/8 heads, bf16: 785 thousand cycles a launch before, 695 now; in
+// a loop of passes, where the power limit lowers the clock, 542 us before and 509 now.  Three prompts of 400 to 1100 tokens
+// behind caches of up to 3000: 92.2 -> 86.9 us a step.  (Issued by one warp on a shared S: 785 thousand cycles.  P's first half
+// sent ahead of the second, P kept in registers until PV(j-1) has read the columns, the maximum of half a row while the
+// other half is loaded, two PV issuers: no gain.  The special-function unit, where the exponentials of both tiles go,
+// is busy 70 % of the launch's cycles now, the tensor pipe 67 %.)
+// Where that does not pay, S_X has a place per tile, P lies over it, and one lane of warp 9 issues PV_A(j), QK_A(j+1), PV_B(j),
+// QK_B(j+1), PV in two halves as those of P arrive: calls that hold P in several pieces (kSplitP: no columns left for a P of its
+// own), in-kernel de-quantisation (mode 1, bound by its producers) and items of one key step (kOwnS).
 //   warps 12-15 mode 1 only: the de-quantising K/V producers.
 // The two tiles are consecutive entries of the list (row block, query head of the group), query heads fastest, so
 // with an even group size both tiles cover the same rows of two heads that share K/V, and the causal structure of
@@ -505,8 +507,8 @@ __global__ void __launch_bounds__(128) paged_gather_kernel(const PagedTables t, 
 //   `kDim` columns behind O_X.  With a head size of 128 that is tile B's place: an item is then ONE tile.  It costs one or two
 //   times as many second products again (the tensor pipe idles behind the exponentials anyway) and six to eight instructions
 //   per pair of probabilities.  Bound: the special-function unit, 128 exponentials per row and step; the f16 encoder batch
-//   of 8 x 16 heads x 512 tokens, head size 64, boolean padding mask: 1167 us in attn_generic_kernel, 27.0 us here (5.1 us
-//   of memory traffic at the copy rate).  With 509 keys: f16 27.2 us, bf16 33.7 us; head size 128 51.0 and 64.7 us.
+//   of 8 x 16 heads x 512 tokens, head size 64, boolean padding mask: 1167 us in attn_generic_kernel, 26.3 us here (5.1 us
+//   of memory traffic at the copy rate).  With 509 keys: f16 26.2 us, bf16 33.9 us; head size 128 46.9 and 60.8 us.
 // kKeySplit (dense): a small problem - fewer pairs of tiles than SMs - is bound by its longest chain of key steps, one tile's
 //   softmax after the other's.  Then an item is ONE tile whose keys are shared out: "tile A" takes the first half of its key
 //   tiles, "tile B" the second, each with its own maximum, sum and accumulator, which are merged in the epilogue (the two
@@ -1057,7 +1059,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     } else if (warp == 9) {
         // =============================== MMA issuer, a place of S per tile ===============================
         // One lane: a step is a chain of waits here, and a vote of the warp behind each costs more than the faster issue gives
-        // (encoder batch of 8 x 16 heads x 512 tokens 27.0 us, by the whole warp 27.6).
+        // (encoder batch of 8 x 16 heads x 512 tokens: by the whole warp 2 % slower).
         if (!kSharedS && lane == 0) {
             // operand formats (A and B of one MMA must agree): dense mode as given; paged mode f16 throughout - the
             // de-quantised values keep 11 significant bits and bf16 queries are converted in shared memory first

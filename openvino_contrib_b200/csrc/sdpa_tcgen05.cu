@@ -33,6 +33,7 @@
 //   warp 10     issues O_X += P_X(j) V_j (A from TMEM, B from shared memory, MN-major) when P_X is ready.
 //   warp 11     completes the service warpgroup; in mode 2 with bf16 queries it and the producer's warp convert the Q
 //               tiles to f16 in shared memory, a tile each.
+//   warps 12-15 mode 1 only: the de-quantising K/V producers, which convert the Q tiles there.
 // TMEM: S 128 columns, P_A and P_B 64 each, O_A and O_B 128 each: all 512 (allocated by warp 9).
 // Why S is shared and QK and PV have issuers of their own: with S and P of a tile in one place a step is the chain softmax ->
 // PV -> QK -> softmax (1750 + 256 + 512 cycles and three trips over barriers), and one issuer, which stands still while the
@@ -46,7 +47,6 @@
 // Where that does not pay, S_X has a place per tile, P lies over it, and one lane of warp 9 issues PV_A(j), QK_A(j+1), PV_B(j),
 // QK_B(j+1), PV in two halves as those of P arrive: calls that hold P in several pieces (kSplitP: no columns left for a P of its
 // own), in-kernel de-quantisation (mode 1, bound by its producers) and items of one key step (kOwnS).
-//   warps 12-15 mode 1 only: the de-quantising K/V producers.
 // The two tiles are consecutive entries of the list (row block, query head of the group), query heads fastest, so
 // with an even group size both tiles cover the same rows of two heads that share K/V, and the causal structure of
 // the pair is identical.

@@ -26,13 +26,16 @@ def test_rows_land_in_their_blocks(dtype, hkv, d, block_size, new):
     cache = b2a.PagedKvCache.allocate(int(t[2].max()) + 4, hkv, d, block_size, dtype)
     rows = [torch.randn(sum(new), hkv * d, generator=torch.Generator().manual_seed(i)).to(dtype) for i in range(2)]
     rows[0][0, 0], rows[1][-1, -1] = float("inf"), 1e-7
+    quiet = 0x7E01 if dtype == torch.float16 else 0x7FC1  # NaNs with a payload and a sign, which become the canonical one
+    rows[0].view(torch.int16)[-1, 2], rows[1].view(torch.int16)[0, 3] = quiet, quiet - 0x8000
     before = [c.cpu().numpy().copy() for c in (cache.k, cache.v)]
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
     b2a.paged_kv_store(rows[0].cuda(), rows[1].cuda(), cache, *[torch.from_numpy(x).cuda() for x in t], status=status)
     assert int(status.item()) == 0
     for pool, was, r in zip((cache.k, cache.v), before, rows):
         want = was.view(np.uint16).reshape(-1, hkv, block_size, d)
-        bits = r.view(torch.int16).numpy().view(np.uint16).reshape(-1, hkv, d)
+        bits = r.view(torch.int16).numpy().view(np.uint16).reshape(-1, hkv, d).copy()
+        bits[torch.isnan(r).numpy().reshape(bits.shape)] = 0x7FFF
         for s in range(len(new)):
             for i in range(new[s]):
                 pos = past[s] + i

@@ -59,3 +59,20 @@ def test_one_key_step(dtype, b, hq, hkv, sq, skv, causal):
         # rows 0..126 see the same keys in the same step whichever kernel takes the call
         shorter = b2a.sdpa(*(t[:, :, :127].contiguous() for t in (q, k, v)), causal=True)
         assert torch.equal(shorter, out[:, :, :127])
+
+
+@pytest.mark.parametrize("s", [100, 128])
+def test_one_key_step_of_a_head_shard(s):
+    # the sharded epilogue (slabs and tensor stores) in the form for one key step, several items a CTA
+    import openvino_contrib_b200 as b2a
+    from openvino_contrib_b200.sharding import HeadShard, ShardGroup
+    b, hq, hkv = 4, 120, 40
+    g = torch.Generator(device="cuda").manual_seed(s)
+    q, k, v = (torch.randn(b, h, s, 128, generator=g, device="cuda").half() for h in (hq, hkv, hkv))
+    group = ShardGroup(HeadShard(0, 1, hq, hkv), staging_bytes=2 * q.numel() * 2)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for causal in (True, False):
+        full = group.sdpa(q, k, v, causal=causal, status=status).clone()
+        assert int(status.item()) == 0
+        assert torch.equal(full, b2a.sdpa(q, k, v, causal=causal))
+    group.close()
